@@ -100,13 +100,15 @@ struct ag_ctx {
   std::vector<int> mapHbond, mapIsHB, mapCov;
   std::vector<float> solparProbe, volProbe;
   int emapMode = agk::kEmapKahan;
-  float rNear = 11.0f;
+  float rNear = 11.25f;
+  float rNode = 27.0f;              // AG_TUNE_EMAP_NODE_RADIUS (0: no node sums)
+  bool smoothTail = false;          // the staged dielectric table is AutoGrid's function
   float delta = 2.0e-3f;
   int packedTable = 1;              // AG_TUNE_EMAP_PACKED_TABLE
   agc::DevBuf<uint4> epsPacked;     // 16- and 8-bit copies of the staged table's saturating tail
   int pkVecs = 0, pkVec8 = 0, pkB16 = 8192, pkB8 = 8192;  // pkVecs == 0: no packed table
   float pkScale = 0;
-  int ctasPerSm = agk::kEmapCtasPerSm;
+  int ctasPerSm = 8;                // AG_TUNE_EMAP_CTAS_PER_SM
   agc::DevBuf<double> checksum;
   int checksumSplits = 0;
   int testIdleWait = 0;             // test hook AG_TUNE_TEST_IDLE_WAIT
@@ -146,7 +148,7 @@ namespace agc {
 
 int checkGrid(const ag_grid* g);
 // E-map work items and CTA boxes of a grid for a CTA tile shape.
-void makeItems(const ag_grid& g, const int tile[3], int warpCompact, std::vector<int>& items,
+void makeItems(const ag_grid& g, const int tile[3], int warpCompact, bool dense, std::vector<int>& items,
                std::vector<agk::EmapBlock>& blocks);
 // Stage the e-map inputs of a job (atoms, dielectric table, CTA boxes).
 int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const double* inv_eps, bool deviceInputs);

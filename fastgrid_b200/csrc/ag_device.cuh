@@ -80,4 +80,10 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   return y;
 }
 
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 }  // namespace agd

@@ -179,6 +179,10 @@ extern "C" int ag_ctx_tune(ag_ctx* c, int knob, double v) {
       if (!(v >= 8.0 && v <= 40.0)) return fail(AG_E_INVALID, "rNear must be in [8, 40] A");
       c->rNear = (float)v;
       return AG_OK;
+    case AG_TUNE_EMAP_NODE_RADIUS:
+      if (!(v == 0.0 || (v >= 24.0 && v <= 1.0e6))) return fail(AG_E_INVALID, "node radius must be 0 or at least 24 A");
+      c->rNode = (float)v;
+      return AG_OK;
     case AG_TUNE_EMAP_PACKED_TABLE:
       if (!(v == 0.0 || v == 1.0)) return fail(AG_E_INVALID, "packed-table switch must be 0 or 1");
       c->packedTable = (int)v;
@@ -241,8 +245,72 @@ int checkGrid(const ag_grid* g) {
   return AG_OK;
 }
 
-// Work items of the e-map (NX points of one row each), grouped into CTAs of
-// 256 items walking tiles of TX x TY x TZ items, with each CTA's box.
+// The box of the items [b.item0, b.item0 + b.nitems).
+static void emapBox(const ag_grid& g, const std::vector<int>& items, agk::EmapBlock& b) {
+  const double h = g.spacing;
+  int i0[3] = {1 << 30, 1 << 30, 1 << 30}, i1[3] = {-1, -1, -1};  // grid points
+  for (int k = b.item0; k < b.item0 + b.nitems; k++) {
+    const int v = items[k];
+    const int xa = (v & 0xFF) * agk::kNX;  // (an interleaved pair's union is the same box)
+    const int p0[3] = {xa, (v >> 8) & 0x7FF, (v >> 19) & 0x7FF};
+    const int p1[3] = {std::min(g.nx, xa + agk::kNX) - 1, p0[1], p0[2]};
+    for (int d = 0; d < 3; d++) {
+      i0[d] = std::min(i0[d], p0[d]);
+      i1[d] = std::max(i1[d], p1[d]);
+    }
+  }
+  const int n2[3] = {g.nx / 2, g.ny / 2, g.nz / 2};
+  double o[3];
+  float half[3];
+  for (int d = 0; d < 3; d++) {
+    const double lo = (i0[d] - n2[d]) * h, hi = (i1[d] - n2[d]) * h;
+    o[d] = 0.5 * (lo + hi);
+    half[d] = (float)(50.0 * (hi - lo) + 1.0);
+  }
+  b.ox = o[0];
+  b.oy = o[1];
+  b.oz = o[2];
+  b.hx = half[0];
+  b.hy = half[1];
+  b.hz = half[2];
+  // Atoms at least rFar (50-55 A) from the box use the saturated dielectric
+  // (table entries past 55 A differ from entry 8191 by < 2.6e-7 relative, past
+  // 50 A by < 1.3e-6); nearer ones read the table, whose index then stays
+  // below 8191 without clamping.
+  const double diag = 2.0 * std::sqrt((double)b.hx * b.hx + (double)b.hy * b.hy + (double)b.hz * b.hz) / 100.0;
+  const double rFar = std::max(50.0, std::min(55.0, 81.0 - diag));
+  b.rfar2 = (float)((100.0 * rFar) * (100.0 * rFar));
+  b.clampMid = rFar + diag >= 81.0 ? 1 : 0;  // mid-list bins may then exceed the table
+  // Interpolation from the box's nodes: with five nodes per axis the error of
+  // an atom's term is below 1.3e-6 of it (rms 3e-7) from 9.5 half-widths on,
+  // and falls with the fifth power of the distance.
+  b.rnode = 9.5f * std::max(b.hx, std::max(b.hy, b.hz));
+}
+
+// Tiles along y and z for tiles of `w` items along x and at most T[1] x T[2]
+// rows: the counts from the least ones up that need the fewest warps (a partly
+// filled warp costs as much as a full one) plus one per CTA for its share of
+// the atom handling.  ntz > 0 fixes the second count.
+static std::pair<int, int> bestSplit(int ny, int nz, const int T[3], int w, int ntz = 0) {
+  const int by = (ny + T[1] - 1) / T[1], bz = ntz > 0 ? ntz : (nz + T[2] - 1) / T[2];
+  std::pair<int, int> best(by, bz);
+  int64_t bestCost = -1;
+  for (int y = by; y <= std::min(ny, by + 3); y++)
+    for (int z = bz; z <= (ntz > 0 ? ntz : std::min(nz, bz + 3)); z++) {
+      const int sy = ny / y, sz = nz / z, my = ny % y, mz = nz % z;  // my tiles of sy + 1 rows, y - my of sy
+      auto cost = [&](int a, int b) { return (int64_t)(w * a * b + 31) / 32 + 1; };
+      const int64_t c = (y - my) * ((z - mz) * cost(sy, sz) + mz * cost(sy, sz + 1)) +
+                        my * ((z - mz) * cost(sy + 1, sz) + mz * cost(sy + 1, sz + 1));
+      if (bestCost < 0 || c < bestCost) {
+        bestCost = c;
+        best = {y, z};
+      }
+    }
+  return best;
+}
+
+// Work items of the e-map (NX points of one row each), grouped into CTAs of at
+// most 256 items in tiles of TX x TY x TZ items, with each CTA's box.
 // warpCompact >= 1: inside a tile, items go in blocks of TX x 4 x 4 (x fastest),
 // so each warp's 32 items form a compact box (for kernels that skip atoms
 // per warp); otherwise x, then y, then z.
@@ -254,74 +322,81 @@ int checkGrid(const ag_grid* g) {
 // fewer table bins, and the table reads of a warp hit fewer distinct words in
 // one shared-memory bank.  A column whose partner is past the grid edge keeps
 // its own NX consecutive points.
-void makeItems(const ag_grid& g, const int tile[3], int warpCompact, std::vector<int>& items,
+// dense: the tiles' items, in boustrophedon tile order, are cut into CTAs of
+// 256 whatever the tiles, so that every CTA but the last is full and a box may
+// span two tiles (the surrogate's near field, whose cost is per CTA and whose
+// warps skip atoms: 4.49 ms per surrogate e-map on 161^3 against 4.60 ms with
+// a CTA per tile).  Otherwise a CTA is a tile and its box stays compact, which
+// the direct e-map's node sums need: they begin 9.5 half-widths from the box.
+void makeItems(const ag_grid& g, const int tile[3], int warpCompact, bool dense, std::vector<int>& items,
                std::vector<agk::EmapBlock>& blocks) {
   const int nxc = (g.nx + agk::kNX - 1) / agk::kNX;
-  const int TX = tile[0], TY = tile[1], TZ = tile[2];
   items.clear();
-  // Tiles in boustrophedon order (y rows and x columns reverse direction on
-  // alternate passes), so a CTA that continues from one tile into the next
-  // stays within neighbouring tiles and its box stays compact.
-  const int ntx = (nxc + TX - 1) / TX, nty = (g.ny + TY - 1) / TY, ntz = (g.nz + TZ - 1) / TZ;
-  const bool compact = warpCompact && TY % 4 == 0 && TZ % 4 == 0;
-  int serp = 0;
-  for (int kz = 0; kz < ntz; kz++)
-    for (int ky0 = 0; ky0 < nty; ky0++) {
-      const int ky = (kz & 1) ? nty - 1 - ky0 : ky0;
-      for (int kx0 = 0; kx0 < ntx; kx0++, serp++) {
-        const int kx = (serp / ntx) & 1 ? ntx - 1 - kx0 : kx0;
-        const int tx = kx * TX, ty = ky * TY, tz = kz * TZ;
-        if (compact) {
-          for (int zb = tz; zb < tz + TZ; zb += 4)
-            for (int yb = ty; yb < ty + TY; yb += 4)
-              for (int z = zb; z < std::min(g.nz, zb + 4); z++)
-                for (int y = yb; y < std::min(g.ny, yb + 4); y++)
-                  for (int x = tx; x < std::min(nxc, tx + TX); x++) {
-                    const bool il = warpCompact == 2 && TX % 2 == 0 && (x ^ 1) < nxc;
-                    items.push_back(x | (y << 8) | (z << 19) | (il ? agk::kItemInterleaved : 0));
-                  }
-        } else {
-          for (int z = tz; z < std::min(g.nz, tz + TZ); z++)
-            for (int y = ty; y < std::min(g.ny, ty + TY); y++)
-              for (int x = tx; x < std::min(nxc, tx + TX); x++) items.push_back(x | (y << 8) | (z << 19));
+  blocks.clear();
+  const int n[3] = {nxc, g.ny, g.nz}, pts[3] = {agk::kNX, 1, 1};
+  int T[3] = {tile[0], tile[1], tile[2]};
+  if (!dense) {
+    // A tile that is larger than the grid along an axis grows along the
+    // others, the shortest (in points) first.
+    for (int d = 0; d < 3; d++) T[d] = std::min(tile[d], n[d]);
+    for (;;) {
+      int best = -1;
+      for (int d = 0; d < 3; d++)
+        if (T[d] < n[d] && 2 * T[0] * T[1] * T[2] <= 256 && (best < 0 || T[d] * pts[d] < T[best] * pts[best])) best = d;
+      if (best < 0) break;
+      T[best] = std::min(2 * T[best], n[best]);
+    }
+  }
+  const bool compact = warpCompact && tile[1] % 4 == 0 && tile[2] % 4 == 0;
+  auto addTile = [&](int x0, int x1, int y0, int y1, int z0, int z1) {
+    const int step = compact ? 4 : std::max(y1 - y0, z1 - z0);
+    for (int zb = z0; zb < z1; zb += step)
+      for (int yb = y0; yb < y1; yb += step)
+        for (int z = zb; z < std::min(z1, zb + step); z++)
+          for (int y = yb; y < std::min(y1, yb + step); y++)
+            for (int x = x0; x < x1; x++) {
+              const bool il = compact && warpCompact == 2 && x0 % 2 == 0 && (x ^ 1) < x1;
+              items.push_back(x | (y << 8) | (z << 19) | (il ? agk::kItemInterleaved : 0));
+            }
+  };
+  auto addBlock = [&](int i0, int i1) {
+    agk::EmapBlock b{};
+    b.item0 = i0;
+    b.nitems = i1 - i0;
+    emapBox(g, items, b);
+    blocks.push_back(b);
+  };
+  const int ntx = (nxc + T[0] - 1) / T[0];
+  if (dense) {
+    const int nty = (g.ny + T[1] - 1) / T[1], ntz = (g.nz + T[2] - 1) / T[2];
+    int serp = 0;
+    for (int kz = 0; kz < ntz; kz++)
+      for (int ky0 = 0; ky0 < nty; ky0++) {
+        const int ky = (kz & 1) ? nty - 1 - ky0 : ky0;
+        for (int kx0 = 0; kx0 < ntx; kx0++, serp++) {
+          const int kx = (serp / ntx) & 1 ? ntx - 1 - kx0 : kx0;
+          addTile(kx * T[0], std::min(nxc, kx * T[0] + T[0]), ky * T[1], std::min(g.ny, ky * T[1] + T[1]), kz * T[2],
+                  std::min(g.nz, kz * T[2] + T[2]));
         }
       }
-    }
-  blocks.clear();
-  const double h = g.spacing;
-  const int n2x = g.nx / 2, n2y = g.ny / 2, n2z = g.nz / 2;
-  for (size_t i0 = 0; i0 < items.size(); i0 += 256) {
-    agk::EmapBlock b{};
-    b.item0 = (int)i0;
-    b.nitems = (int)std::min<size_t>(256, items.size() - i0);
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-    for (int k = 0; k < b.nitems; k++) {
-      int v = items[i0 + k];
-      int xc = v & 0xFF, y = (v >> 8) & 0x7FF, z = (v >> 19) & 0x7FF;  // the pair's union is the same box
-      int xa = xc * agk::kNX, xb = std::min(g.nx - 1, xa + agk::kNX - 1);
-      double p[2][3] = {{(xa - n2x) * h, (y - n2y) * h, (z - n2z) * h}, {(xb - n2x) * h, (y - n2y) * h, (z - n2z) * h}};
-      for (int q = 0; q < 2; q++)
-        for (int d = 0; d < 3; d++) {
-          lo[d] = std::min(lo[d], p[q][d]);
-          hi[d] = std::max(hi[d], p[q][d]);
-        }
-    }
-    b.ox = 0.5 * (lo[0] + hi[0]);
-    b.oy = 0.5 * (lo[1] + hi[1]);
-    b.oz = 0.5 * (lo[2] + hi[2]);
-    b.hx = (float)(50.0 * (hi[0] - lo[0]) + 1.0);
-    b.hy = (float)(50.0 * (hi[1] - lo[1]) + 1.0);
-    b.hz = (float)(50.0 * (hi[2] - lo[2]) + 1.0);
-    // Atoms at least rFar (50-55 A) from the box use the saturated dielectric
-    // (table entries past 55 A differ from entry 8191 by < 2.6e-7 relative, past
-    // 50 A by < 1.3e-6); nearer ones read the table, whose index then stays
-    // below 8191 without clamping.
-    const double diag = 2.0 * std::sqrt((double)b.hx * b.hx + (double)b.hy * b.hy + (double)b.hz * b.hz) / 100.0;
-    const double rFar = std::max(50.0, std::min(55.0, 81.0 - diag));
-    b.rfar2 = (float)((100.0 * rFar) * (100.0 * rFar));
-    b.clampMid = rFar + diag >= 81.0 ? 1 : 0;  // mid-list bins may then exceed the table
-    blocks.push_back(b);
+    const int total = (int)items.size();
+    for (int i0 = 0; i0 < total; i0 += 256) addBlock(i0, std::min(total, i0 + 256));
+    return;
   }
+  // Rows and planes are divided evenly among the tiles; a last, narrower
+  // column of tiles takes correspondingly more rows.
+  const int ntz = bestSplit(g.ny, g.nz, T, T[0]).second;
+  for (int kz = 0; kz < ntz; kz++)
+    for (int kx = 0; kx < ntx; kx++) {
+      const int x0 = kx * T[0], x1 = std::min(nxc, x0 + T[0]);
+      const int tall[3] = {x1 - x0, std::min(g.ny, T[1] * (T[0] / (x1 - x0))), T[2]};
+      const int nty = bestSplit(g.ny, g.nz, tall, x1 - x0, ntz).first;
+      for (int ky = 0; ky < nty; ky++) {
+        const int i0 = (int)items.size();
+        addTile(x0, x1, g.ny * ky / nty, g.ny * (ky + 1) / nty, g.nz * kz / ntz, g.nz * (kz + 1) / ntz);
+        addBlock(i0, (int)items.size());
+      }
+    }
 }
 
 void buildItems(ag_ctx* c) {
@@ -329,7 +404,7 @@ void buildItems(ag_ctx* c) {
   if (c->itemsFor[0] == g.nx && c->itemsFor[1] == g.ny && c->itemsFor[2] == g.nz && c->itemsH == g.spacing &&
       c->itemsTile == c->tile[0] * 10000 + c->tile[1] * 100 + c->tile[2] && c->itemsCompact == c->warpCompact)
     return;
-  makeItems(g, c->tile, c->warpCompact, c->hItems, c->hBlocks);
+  makeItems(g, c->tile, c->warpCompact, false, c->hItems, c->hBlocks);
   c->itemsOnDevice = false;
   c->itemsCompact = c->warpCompact;
   c->itemsFor[0] = g.nx;
@@ -395,6 +470,23 @@ int packTableTailInto(const float* t, int n, unsigned char* raw, int cap, int& b
   return total;
 }
 
+// Whether the table is AutoGrid's 332 / eps (InputDataLoader.cpp:715-742) from
+// 20 A on, to FP32 rounding: the node sums of the e-map use that function.
+bool tableIsSmooth(const float* t, int n) {
+  static float ref[8192];
+  static std::once_flag once;
+  std::call_once(once, [] {
+    for (int i = 0; i < 8192; i++) {
+      const double E = std::exp(-0.3153767175 * (i / 100.0));
+      ref[i] = (float)((332.0 + 332.0 * 7.7839 * E) / (78.4 - 66.57180475 * E));
+    }
+  });
+  if (n != 8192) return false;
+  for (int i = 2000; i < 8192; i++)
+    if (!(std::fabs(t[i] - ref[i]) <= 1.2e-7f * ref[i])) return false;
+  return true;
+}
+
 // The same, into 16-byte vectors (empty: no usable tail).
 std::vector<uint4> packTableTail(const std::vector<float>& t, int& b16, int& b8, int& vec8, float& kScale) {
   std::vector<uint4> out(agk::kEmapPackedBytes / 16);
@@ -431,6 +523,7 @@ int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const doub
     for (int i = 0; i < 8192; i++) t[i] = (float)inv_eps[i];
     CK(c->epsTab.ensure(8192));
     CK(cudaMemcpyAsync(c->epsTab.p, t.data(), sizeof(float) * 8192, cudaMemcpyHostToDevice, c->stream));
+    c->smoothTail = tableIsSmooth(t.data(), 8192);
     const std::vector<uint4> pk = packTableTail(t, c->pkB16, c->pkB8, c->pkVec8, c->pkScale);
     c->pkVecs = (int)pk.size();
     if (!pk.empty()) {
@@ -453,6 +546,20 @@ int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const doub
   return AG_OK;
 }
 
+// Atoms per CTA when the grid alone does not give every SM enough waves of
+// resident CTAs to even out their unequal costs: whole 256-atom tiles (a tile
+// costs its barriers and its latency however few atoms it holds), half tiles
+// only where whole ones would not give every SM three CTAs.  With CTAs for 16 per SM 8,000
+// atoms on 101^3 points took 2.45 ms and with 6 per SM 2.63 ms.
+int emapChunk(int nAtoms, int nblocks, int sms, int ctasPerSm) {
+  const int want = 2 * sms * ctasPerSm;
+  if (nblocks >= want) return std::max(nAtoms, 1);
+  const int ns = (want + nblocks - 1) / nblocks;
+  const int chunk = std::max(256, nAtoms / ns / 256 * 256);
+  if (chunk == 256 && (int64_t)nblocks * ((nAtoms + 255) / 256) < 3 * sms) return 128;
+  return chunk;
+}
+
 // Launch parameters of the e-map of the staged job; allowSplit = false keeps
 // every CTA on all atoms (the batch kernel's mode).
 int buildEmapParams(ag_ctx* c, float* dOut, bool allowSplit, agk::EmapParams& P) {
@@ -471,6 +578,11 @@ int buildEmapParams(ag_ctx* c, float* dOut, bool allowSplit, agk::EmapParams& P)
   P.thr = c->thr.p;
   P.rnear2 = (100.f * c->rNear) * (100.f * c->rNear);
   P.delta = c->delta;
+  // Node sums: the smooth dielectric leaves out the 0.01 A steps of the table,
+  // which matter up to rNode; the constant dielectric has none.  Near atoms
+  // (the cap of 1/r, compensated terms) are never summed at the nodes.
+  P.rnodeMin = (c->rNode > 0.f && (!c->ddd || c->smoothTail)) ? 100.f * std::max(c->rNear, c->ddd ? c->rNode : 0.f)
+                                                              : INFINITY;
   if (c->ddd && c->packedTable && c->pkVecs > 0) {
     P.packed = c->epsPacked.p;
     P.packedVecs = c->pkVecs;
@@ -487,14 +599,8 @@ int buildEmapParams(ag_ctx* c, float* dOut, bool allowSplit, agk::EmapParams& P)
   // Split atoms across CTAs when the grid alone cannot fill the GPU.
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-  const int want = 2 * sms * c->ctasPerSm;  // two waves of resident CTAs
-  int nsplit = 1;
-  if (allowSplit && P.nblocks < want && c->nAtoms > 512)
-    nsplit = std::min((want + P.nblocks - 1) / P.nblocks, (c->nAtoms + 255) / 256);
-  int chunk = (c->nAtoms + nsplit - 1) / nsplit;
-  chunk = ((chunk + 255) / 256) * 256;
-  if (chunk == 0) chunk = 256;
-  nsplit = std::max(1, (c->nAtoms + chunk - 1) / chunk);
+  const int chunk = allowSplit ? emapChunk(c->nAtoms, P.nblocks, sms, c->ctasPerSm) : std::max(c->nAtoms, 1);
+  const int nsplit = std::max(1, (c->nAtoms + chunk - 1) / chunk);
   P.chunk = chunk;
   P.nsplit = nsplit;
   if (nsplit > 1) {

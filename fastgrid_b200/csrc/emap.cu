@@ -38,6 +38,10 @@
 //    100 w 2^-16 (g + k_b ulp(g)) = 100 w 2^-16 invEps[b] from it.
 //    Mid and far terms are summed in plain FP32 over chunks of kChunk atoms
 //    and the chunk sums are Kahan-compensated.
+//  * Atoms at least R from the box (27 A; more for boxes wider than 5.7 A) do
+//    not enter point by point: their sum is a smooth function over the box,
+//    so it is formed at 5 x 5 x 5 Chebyshev nodes of the box and interpolated
+//    to the box's 2,048 points at the end (node_atoms, node_field).
 //  * When the grid is too small to fill the GPU, atoms are split across CTAs
 //    and the per-CTA results are reduced in FP64, in a fixed order, by a
 //    second kernel.
@@ -58,19 +62,25 @@ constexpr int kTabLen = 8192;     // invEps entries
 constexpr int kChunk = 32;        // atoms per plain-FP32 chunk sum
 
 // Atom classes of a tile, in their order in EmapSmem::list.
-enum { kClsNear = 0, kClsMid = 1, kClsMid16 = 2, kClsMid8 = 3, kClsFar = 4, kNumCls = 5 };
+enum { kClsNode = 0, kClsNear = 1, kClsMid = 2, kClsMid16 = 3, kClsMid8 = 4, kClsFar = 5, kNumCls = 6 };
+
+constexpr int kNodes1 = 5;                             // interpolation nodes per axis
+constexpr int kNodes = kNodes1 * kNodes1 * kNodes1;    // per CTA box
+constexpr int kNodeGroups = 4;                         // thread groups that share a tile's node atoms
 
 struct EmapSmem {
   float tab[kTabLen];             // 32 KB
   double4 ring[2][kTile];         // 16 KB, TMA destination
   __align__(16) unsigned char packed[kEmapPackedBytes];
   // This tile's atoms grouped by class: local scaled x, y, z and 100*w
-  // (near, mid), 100*w*g*2^-16 (packed mid) or 100*w*g (far).
-  float4 list[kTile];
-  short nearIdx[kTile];           // tile slot of each near atom (for FP64 lookups)
+  // (near, mid), 100*w*g*2^-16 (packed mid) or 100*w*g (far).  The node atoms
+  // come first, two atoms in two entries: (x0, x1, y0, y1), (z0, z1, w0, w1).
+  float4 list[kTile + 2];
+  float4 nodeAcc[kThreads];       // per thread: Kahan sum and compensation of its two nodes
+  short nearIdx[kTile + 2];       // tile slot of each near atom (for FP64 lookups)
   // Near atom: bit w set if it lies within rNear of warp w's points, bit 8 + w
   // if within 0.51 A of them (the 1/r cap can apply).
-  unsigned short nearMask[kTile];
+  unsigned short nearMask[kTile + 2];
   float4 wlo[kThreads / 32], whi[kThreads / 32];  // each warp's box (local, scaled), widened by 0.01 A
   int cnt[kNumCls][kThreads / 32];
   double wpart[kThreads / 32];
@@ -226,6 +236,110 @@ __device__ __forceinline__ void mid_packed_atoms(const float4* __restrict__ list
   }
 }
 
+// Chebyshev node k of [-1, 1]: cos((2 k + 1) pi / 10).
+__device__ __forceinline__ float cheb_node(int k) {
+  const float v = (k == 0 || k == 4) ? 0.95105652f : (k == 2 ? 0.f : 0.58778525f);
+  return k > 2 ? -v : v;
+}
+
+// Lagrange weights of the five nodes at t.  1 / prod_{m != j} (c_j - c_m) is
+// 16 (-1)^j sin((2 j + 1) pi / 10) / 5.
+__device__ __forceinline__ void node_weights(float t, float (&w)[kNodes1]) {
+  const float inv[kNodes1] = {0.98885438f, -2.58885438f, 3.2f, -2.58885438f, 0.98885438f};
+  float d[kNodes1];
+#pragma unroll
+  for (int k = 0; k < kNodes1; k++) d[k] = t - cheb_node(k);
+#pragma unroll
+  for (int j = 0; j < kNodes1; j++) {
+    float p = inv[j];
+#pragma unroll
+    for (int m = 0; m < kNodes1; m++)
+      if (m != j) p *= d[m];
+    w[j] = p;
+  }
+}
+
+// Sum of a tile's node atoms at this thread's two nodes of the box (half
+// extents hx, hy, hz).  64 threads cover the nodes, and the kNodeGroups groups
+// of 64 take the atom pairs in turn; packed FP32 over the two atoms of a pair,
+// whose record keeps equal components side by side (no register moves).  The
+// kernel is the dielectric's smooth form, 332 / eps = g (1 + E (c1 + c2 E)),
+// E = exp(-lambda (r - 0.005)) (half a bin in: the left-edge bins are met on
+// average); the next term of the series is below 1e-9 from 24 A on.
+template <bool DDD>
+__device__ __forceinline__ void node_atoms(EmapSmem& S, const int npairs, const float hx, const float hy,
+                                           const float hz) {
+  const int q = threadIdx.x & 63, grp = threadIdx.x >> 6;
+  float2 nx[2], ny[2], nz[2], s[2];
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int n = min(2 * q + u, kNodes - 1);
+    nx[u] = dup2(-cheb_node(n % kNodes1) * hx);
+    ny[u] = dup2(-cheb_node((n / kNodes1) % kNodes1) * hy);
+    nz[u] = dup2(-cheb_node(n / (kNodes1 * kNodes1)) * hz);
+    s[u] = make_float2(0.f, 0.f);
+  }
+  const float2 nl = dup2(-4.5499247e-3f);    // -lambda / (100 ln 2), lambda = 0.3153767175 per A
+  const float2 sh = dup2(2.2749621e-3f);     // 0.005 lambda / ln 2
+  const float2 c1 = dup2(8.6330307f);        // a + c, a = 7.7839, c = 66.57180475 / 78.4
+  const float2 c2 = dup2(7.3305663f);        // c (a + c)
+  const float2 one = dup2(1.f);
+#pragma unroll 2
+  for (int p = grp; p < npairs; p += kNodeGroups) {
+    const float4 xy = S.list[2 * p], zw = S.list[2 * p + 1];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const float2 dx = __fadd2_rn(make_float2(xy.x, xy.y), nx[u]);
+      const float2 dy = __fadd2_rn(make_float2(xy.z, xy.w), ny[u]);
+      const float2 dz = __fadd2_rn(make_float2(zw.x, zw.y), nz[u]);
+      const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+      const float2 rs = rsqrt2(r2);
+      float2 term = __fmul2_rn(make_float2(zw.z, zw.w), rs);
+      if (DDD) {
+        const float2 arg = __ffma2_rn(__fmul2_rn(r2, rs), nl, sh);
+        const float2 E = make_float2(ex2_approx(arg.x), ex2_approx(arg.y));
+        term = __fmul2_rn(term, __ffma2_rn(E, __ffma2_rn(E, c2, c1), one));
+      }
+      s[u] = __fadd2_rn(s[u], term);
+    }
+  }
+  float4 a = S.nodeAcc[threadIdx.x];
+  const float y0 = (s[0].x + s[0].y) - a.y, t0 = a.x + y0;
+  const float y1 = (s[1].x + s[1].y) - a.w, t1 = a.z + y1;
+  a.y = (t0 - a.x) - y0;
+  a.x = t0;
+  a.w = (t1 - a.z) - y1;
+  a.z = t1;
+  S.nodeAcc[threadIdx.x] = a;
+}
+
+// The node atoms' field at this thread's points, from the node sums F (in
+// shared memory, x fastest): the y and z weights first, then x per point.
+__device__ __forceinline__ void node_field(const float* F, const float2 (&gxn)[kNX / 2], float gy, float gz, float hx,
+                                           float hy, float hz, float (&out)[kNX]) {
+  float wy[kNodes1], wz[kNodes1], c[kNodes1] = {0.f, 0.f, 0.f, 0.f, 0.f};
+  node_weights(gy / hy, wy);
+  node_weights(gz / hz, wz);
+#pragma unroll
+  for (int kz = 0; kz < kNodes1; kz++)
+#pragma unroll
+    for (int ky = 0; ky < kNodes1; ky++) {
+      const float w = wz[kz] * wy[ky];
+#pragma unroll
+      for (int kx = 0; kx < kNodes1; kx++) c[kx] = fmaf(w, F[(kz * kNodes1 + ky) * kNodes1 + kx], c[kx]);
+    }
+  const float inv = 1.f / hx;
+#pragma unroll
+  for (int k = 0; k < kNX; k++) {
+    float wx[kNodes1];
+    node_weights(-lo_hi(gxn[k >> 1], k) * inv, wx);
+    float v = 0.f;
+#pragma unroll
+    for (int kx = 0; kx < kNodes1; kx++) v = fmaf(wx[kx], c[kx], v);
+    out[k] = v;
+  }
+}
+
 // One near atom against this thread's points, bins decided exactly near an
 // edge.  GUARD: cap 1/r at 2 and clamp the bin at the table's end; without it
 // the caller has shown that no point of the warp lies within 0.51 A of the
@@ -331,8 +445,15 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
 #pragma unroll
   for (int k = 0; k < kNX / 2; k++) gxn[k] = make_float2(-gx[2 * k], -gx[2 * k + 1]);
 
+  // Atoms this far (0.01 A) from the box are summed at its nodes.
+  const float rnode = MODE == kEmapKahan ? fmaxf(B.rnode, P.rnodeMin) : __int_as_float(0x7F800000);
+  // Mid-list bins may pass the table's end (not if the node atoms begin before).
+  const bool clampMid = B.clampMid && !(rnode + 2.f * sqrtf(B.hx * B.hx + B.hy * B.hy + B.hz * B.hz) < 8100.f);
+  int nodeTotal = 0;  // node atoms seen so far (uniform)
+  S.nodeAcc[tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+
   // Packed tail tables for this box: only when no bin can pass the table's end.
-  const bool pk = DDD && P.packed != nullptr && !B.clampMid;
+  const bool pk = DDD && P.packed != nullptr && !clampMid;
   if (DDD) {
     const float4* src = reinterpret_cast<const float4*>(P.table);
     float4* dst = reinterpret_cast<float4*>(S.tab);
@@ -426,7 +547,10 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
       const float dx = fmaxf(fabsf(loc.x) - B.hx, 0.f), dy = fmaxf(fabsf(loc.y) - B.hy, 0.f),
                   dz = fmaxf(fabsf(loc.z) - B.hz, 0.f);
       const float d2 = dx * dx + dy * dy + dz * dz;
-      if (d2 < P.rnear2) {
+      if (d2 >= rnode * rnode) {
+        cls = kClsNode;
+        loc.w *= gFar;
+      } else if (d2 < P.rnear2) {
         cls = kClsNear;
         // The warps whose own points it is near: the others evaluate it as a mid atom.
         unsigned m = 0;
@@ -462,7 +586,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
     __syncthreads();
     // Start of each class in the list, and of this warp's atoms within it.
     int base[kNumCls];
-    int run = 0, myPos = 0;
+    int run = 0, myPos = 0, nodeCnt = 0;
 #pragma unroll
     for (int c = 0; c < kNumCls; c++) {
       base[c] = run;
@@ -474,22 +598,44 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
         run += v;
       }
       if (cls == c) myPos = base[c] + off + __popc(myBallot & lt);
+      if (c == kClsNode) {  // whole pairs
+        nodeCnt = run;
+        run = (run + 1) & ~1;
+      }
     }
-    if (cls >= 0) {
+    const int nNode = base[kClsNear];
+    if (cls == kClsNode) {
+      float* pr = reinterpret_cast<float*>(S.list) + 8 * (myPos >> 1) + (myPos & 1);
+      pr[0] = loc.x;
+      pr[2] = loc.y;
+      pr[4] = loc.z;
+      pr[6] = loc.w;
+    } else if (cls >= 0) {
       S.list[myPos] = loc;
       if (cls == kClsNear) {
         S.nearIdx[myPos] = (short)tid;
         S.nearMask[myPos] = (unsigned short)nearBits;
       }
     }
+    if (tid == 0 && (nodeCnt & 1)) {
+      // An odd last pair is completed by an atom of no weight far away.
+      float* pr = reinterpret_cast<float*>(S.list) + 8 * (nodeCnt >> 1) + 1;
+      pr[0] = 1.0e7f;
+      pr[2] = 0.f;
+      pr[4] = 0.f;
+      pr[6] = 0.f;
+    }
     __syncthreads();
-    const int nNear = base[kClsMid];
+    if (nNode > 0) {
+      node_atoms<DDD>(S, nNode >> 1, B.hx, B.hy, B.hz);
+      nodeTotal += nNode;
+    }
 
     // Mid atoms: table read, or a packed tail table.
     if (DDD) {
       const uint32_t tabBiased = smem_u32(S.tab) - 0x2C000000u;
       const int nMid = base[kClsMid16] - base[kClsMid];
-      if (B.clampMid)
+      if (clampMid)
         mid_atoms<MODE, true>(S.list + base[kClsMid], tabBiased, nMid, gxn, gy, gz, sum, cmp);
       else
         mid_atoms<MODE, false>(S.list + base[kClsMid], tabBiased, nMid, gxn, gy, gz, sum, cmp);
@@ -530,7 +676,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
 
     // Near atoms: clamp 1/r at 2 and decide bins near an edge exactly.
 #pragma unroll 1
-    for (int j = 0; j < nNear; j++) {
+    for (int j = base[kClsNear]; j < base[kClsMid]; j++) {
       const float4 a = S.list[j];
       const float dy = a.y - gy, dz = a.z - gz;
       // The 1e-30 keeps r2 > 0 (an atom on a grid point) without a per-point max.
@@ -559,7 +705,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
         }
         continue;
       }
-      if (!B.clampMid && !((S.nearMask[j] >> (8 + warp)) & 1u))  // uniform
+      if (!clampMid && !((S.nearMask[j] >> (8 + warp)) & 1u))  // uniform
         near_exact<DDD, MODE, false>(S, P, slot, j, dyz2, ax, aw, gxn, iy, iz, xb, xs, sum, cmp);
       else
         near_exact<DDD, MODE, true>(S, P, slot, j, dyz2, ax, aw, gxn, iy, iz, xb, xs, sum, cmp);
@@ -581,14 +727,32 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
     }
   }
 
+  // The node atoms' part: their sums at the nodes, interpolated to the points.
+  float fld[kNX] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (nodeTotal > 0) {
+    float* F = reinterpret_cast<float*>(S.list);
+    if (tid < kNodes) {
+      double f = 0.0;
+#pragma unroll
+      for (int grp = 0; grp < kNodeGroups; grp++) {
+        const float4 a = S.nodeAcc[64 * grp + (tid >> 1)];
+        f += (tid & 1) ? (double)a.z - (double)a.w : (double)a.x - (double)a.y;
+      }
+      F[tid] = (float)f;
+    }
+    __syncthreads();
+    node_field(F, gxn, gy, gz, B.hx, B.hy, B.hz, fld);
+  }
+
   if (!active) return;
   const int64_t row = ((int64_t)iz * P.ny + iy) * P.nx;
 #pragma unroll
   for (int k = 0; k < kNX; k++) {
     const int x = xb + k * xs;
     if (x >= P.nx) break;
-    const double v = (MODE == kEmapKahan) ? (double)lo_hi(sum[k >> 1], k) - (double)lo_hi(cmp[k >> 1], k)
-                                          : (double)lo_hi(sum[k >> 1], k);
+    const double v = ((MODE == kEmapKahan) ? (double)lo_hi(sum[k >> 1], k) - (double)lo_hi(cmp[k >> 1], k)
+                                           : (double)lo_hi(sum[k >> 1], k)) +
+                     (double)fld[k];
     if (P.nsplit == 1)
       P.out[row + x] = (float)v;
     else

@@ -330,6 +330,7 @@ extern "C" int ag_emap_noalloc(const ag_grid* grid, int n_atoms, const double* d
   P.thr = D.thr;
   P.rnear2 = (100.f * 14.0f) * (100.f * 14.0f);
   P.delta = 2.0e-3f;
+  P.rnodeMin = INFINITY;
   P.out = d_out;
   P.status = D.status;
   P.checksum = D.checksum;

@@ -238,7 +238,7 @@ int surrPrepare(ag_ctx* c, SurrState& S) {
   static const int kTile[3] = {1, 16, 16};
   const int key[4] = {g.nx, g.ny, g.nz, kTile[0] * 10000 + kTile[1] * 100 + kTile[2]};
   if (memcmp(key, S.itemsKey, sizeof key) != 0 || S.itemsH != g.spacing) {
-    makeItems(g, kTile, 1, S.hItems, S.hBlocks);
+    makeItems(g, kTile, 1, true, S.hItems, S.hBlocks);
     CK(S.dItems.ensure(S.hItems.size()));
     CK(S.dBlocks.ensure(S.hBlocks.size()));
     CK(cudaMemcpyAsync(S.dItems.p, S.hItems.data(), sizeof(int) * S.hItems.size(), cudaMemcpyHostToDevice,
@@ -314,12 +314,24 @@ int surrBase(ag_ctx* c, SurrState& S, float* dBase, uint4* dFeat, float sIn) {
     CK(cudaMemsetAsync(dBase, 0, sizeof(float) * np, c->stream));
   } else {
     agk::EmapParams P;
-    if (int e = buildEmapParams(c, dBase, true, P)) return e;
+    if (int e = buildEmapParams(c, dBase, false, P)) return e;
     P.checksum = nullptr;
     P.atoms = S.atomsSorted.p;
     P.items = S.dItems.p;
     P.blocks = S.dBlocks.p;
     P.nblocks = (int)S.hBlocks.size();
+    // Whole 256-atom tiles are split across CTAs on grids too small for two
+    // waves of three CTAs per SM.
+    const int want = 6 * sms(c);
+    if (P.nblocks < want && c->nAtoms > 512) {
+      const int ns = std::min((want + P.nblocks - 1) / P.nblocks, (c->nAtoms + 255) / 256);
+      P.chunk = ((c->nAtoms + ns - 1) / ns + 255) / 256 * 256;
+      P.nsplit = (c->nAtoms + P.chunk - 1) / P.chunk;
+      if (P.nsplit > 1) {
+        CK(c->partial.ensure((size_t)P.nsplit * np));
+        P.partial = c->partial.p;
+      }
+    }
     P.tileLo = S.tileLo.p;
     P.tileHi = S.tileHi.p;
     P.rnear2 = (float)((100.0 * a) * (100.0 * a));
