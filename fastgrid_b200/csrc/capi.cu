@@ -246,7 +246,7 @@ int checkGrid(const ag_grid* g) {
 }
 
 // The box of the items [b.item0, b.item0 + b.nitems).
-static void emapBox(const ag_grid& g, const std::vector<int>& items, agk::EmapBlock& b) {
+static void emapBox(const ag_grid& g, const int* items, agk::EmapBlock& b) {
   const double h = g.spacing;
   int i0[3] = {1 << 30, 1 << 30, 1 << 30}, i1[3] = {-1, -1, -1};  // grid points
   for (int k = b.item0; k < b.item0 + b.nitems; k++) {
@@ -328,11 +328,12 @@ static std::pair<int, int> bestSplit(int ny, int nz, const int T[3], int w, int 
 // warps skip atoms: 4.49 ms per surrogate e-map on 161^3 against 4.60 ms with
 // a CTA per tile).  Otherwise a CTA is a tile and its box stays compact, which
 // the direct e-map's node sums need: they begin 9.5 half-widths from the box.
-void makeItems(const ag_grid& g, const int tile[3], int warpCompact, bool dense, std::vector<int>& items,
-               std::vector<agk::EmapBlock>& blocks) {
+// Writes the items (one per 8 points of a row) and at most blockCap boxes;
+// returns the number of boxes, or -1 if there are more.  Allocates nothing.
+int makeItemsInto(const ag_grid& g, const int tile[3], int warpCompact, bool dense, int* items,
+                  agk::EmapBlock* blocks, int blockCap) {
   const int nxc = (g.nx + agk::kNX - 1) / agk::kNX;
-  items.clear();
-  blocks.clear();
+  int nitems = 0, nblocks = 0;
   const int n[3] = {nxc, g.ny, g.nz}, pts[3] = {agk::kNX, 1, 1};
   int T[3] = {tile[0], tile[1], tile[2]};
   if (!dense) {
@@ -356,15 +357,18 @@ void makeItems(const ag_grid& g, const int tile[3], int warpCompact, bool dense,
           for (int y = yb; y < std::min(y1, yb + step); y++)
             for (int x = x0; x < x1; x++) {
               const bool il = compact && warpCompact == 2 && x0 % 2 == 0 && (x ^ 1) < x1;
-              items.push_back(x | (y << 8) | (z << 19) | (il ? agk::kItemInterleaved : 0));
+              items[nitems++] = x | (y << 8) | (z << 19) | (il ? agk::kItemInterleaved : 0);
             }
   };
   auto addBlock = [&](int i0, int i1) {
-    agk::EmapBlock b{};
-    b.item0 = i0;
-    b.nitems = i1 - i0;
-    emapBox(g, items, b);
-    blocks.push_back(b);
+    if (nblocks < blockCap) {
+      agk::EmapBlock b{};
+      b.item0 = i0;
+      b.nitems = i1 - i0;
+      emapBox(g, items, b);
+      blocks[nblocks] = b;
+    }
+    nblocks++;
   };
   const int ntx = (nxc + T[0] - 1) / T[0];
   if (dense) {
@@ -379,9 +383,8 @@ void makeItems(const ag_grid& g, const int tile[3], int warpCompact, bool dense,
                   std::min(g.nz, kz * T[2] + T[2]));
         }
       }
-    const int total = (int)items.size();
-    for (int i0 = 0; i0 < total; i0 += 256) addBlock(i0, std::min(total, i0 + 256));
-    return;
+    for (int i0 = 0; i0 < nitems; i0 += 256) addBlock(i0, std::min(nitems, i0 + 256));
+    return nblocks <= blockCap ? nblocks : -1;
   }
   // Rows and planes are divided evenly among the tiles; a last, narrower
   // column of tiles takes correspondingly more rows.
@@ -392,11 +395,24 @@ void makeItems(const ag_grid& g, const int tile[3], int warpCompact, bool dense,
       const int tall[3] = {x1 - x0, std::min(g.ny, T[1] * (T[0] / (x1 - x0))), T[2]};
       const int nty = bestSplit(g.ny, g.nz, tall, x1 - x0, ntz).first;
       for (int ky = 0; ky < nty; ky++) {
-        const int i0 = (int)items.size();
+        const int i0 = nitems;
         addTile(x0, x1, g.ny * ky / nty, g.ny * (ky + 1) / nty, g.nz * kz / ntz, g.nz * (kz + 1) / ntz);
-        addBlock(i0, (int)items.size());
+        addBlock(i0, nitems);
       }
     }
+  return nblocks <= blockCap ? nblocks : -1;
+}
+
+void makeItems(const ag_grid& g, const int tile[3], int warpCompact, bool dense, std::vector<int>& items,
+               std::vector<agk::EmapBlock>& blocks) {
+  items.resize((size_t)((g.nx + agk::kNX - 1) / agk::kNX) * g.ny * g.nz);
+  blocks.resize(items.size() / 32 + 64);
+  int nb = makeItemsInto(g, tile, warpCompact, dense, items.data(), blocks.data(), (int)blocks.size());
+  if (nb < 0) {  // many small tiles
+    blocks.resize(items.size());
+    nb = makeItemsInto(g, tile, warpCompact, dense, items.data(), blocks.data(), (int)blocks.size());
+  }
+  blocks.resize(nb);
 }
 
 void buildItems(ag_ctx* c) {

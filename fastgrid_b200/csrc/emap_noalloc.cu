@@ -14,7 +14,7 @@
 // fit).  Larger grids are rejected with AG_E_INVALID before any CUDA call, and
 // so are input pointers that are not 16-byte aligned (the kernel reads atoms
 // by 16-byte bulk copies and the table as float4).  The arrays take about
-// 21 MiB on every device that loads the library, until the process exits.
+// 22 MiB on every device that loads the library, until the process exits.
 //
 // Sharing: every call, from any thread or stream, uses the same device arrays,
 // and they keep the previous call's contents.  Calls whose GPU work overlaps
@@ -47,19 +47,28 @@
 namespace ag {
 void setLastError(const char* msg);  // capi.cu
 }
+// capi.cu; none of these allocates
 namespace agc {
-void emapBinThresholdsInto(double* thr);  // capi.cu: fills thr[0 .. 8192], no allocation
+void emapBinThresholdsInto(double* thr);  // fills thr[0 .. 8192]
+bool tableIsSmooth(const float* t, int n);
+int emapChunk(int nAtoms, int nblocks, int sms, int ctasPerSm);
+int makeItemsInto(const ag_grid& g, const int tile[3], int warpCompact, bool dense, int* items,
+                  agk::EmapBlock* blocks, int blockCap);
 int packTableTailInto(const float* t, int n, unsigned char* raw, int cap, int& b16, int& b8, int& vec8,
-                      float& kScale);  // capi.cu: packed tail tables of the dielectric table, no allocation
+                      float& kScale);  // packed tail tables of the dielectric table
 }
 
 namespace {
 
 constexpr int kNaMaxItems = 1 << 20;             // 4 MiB of work items
-constexpr int kNaMaxBlocks = (kNaMaxItems + 255) / 256;
+constexpr int kNaMaxBlocks = 16384;             // CTA boxes (at least kNaMaxItems / 256)
 constexpr int64_t kNaMaxPartial = 1 << 21;       // 16 MiB of FP64 partial sums
 constexpr int kNaThr = 8193;
+// A: exact-bin and node radii.  This entry point has always decided bins exactly
+// out to 14 A; with these two its error against FP64 stays what it was.
+constexpr float kNaNear = 14.5f, kNaNode = 28.0f;
 constexpr int kNaMaxSplit = 1024;                // atom splits (checksum slots)
+constexpr int kNaCtasPerSm = 8;                  // as AG_TUNE_EMAP_CTAS_PER_SM's default
 
 static __device__ __align__(256) double g_naPartial[kNaMaxPartial];
 static __device__ __align__(256) int g_naItems[kNaMaxItems];
@@ -182,60 +191,13 @@ int naSetup(NaDevice& d) {
   return AG_OK;
 }
 
-// Work items (8 x points of one row) in 2 x 16 x 8 tiles, boustrophedon order,
-// 256 per CTA, with each CTA's box; returns the number of CTAs or -1 if the
-// grid needs more than kNaMaxItems items.
-int naItems(const ag_grid& g, int& nitems) {
-  const int nxc = (g.nx + agk::kNX - 1) / agk::kNX;
-  const int64_t need = (int64_t)nxc * g.ny * g.nz;
-  if (need > kNaMaxItems) return -1;
-  const int TX = 2, TY = 16, TZ = 8;
-  const int ntx = (nxc + TX - 1) / TX, nty = (g.ny + TY - 1) / TY, ntz = (g.nz + TZ - 1) / TZ;
-  int n = 0, serp = 0;
-  for (int kz = 0; kz < ntz; kz++)
-    for (int ky0 = 0; ky0 < nty; ky0++) {
-      const int ky = (kz & 1) ? nty - 1 - ky0 : ky0;
-      for (int kx0 = 0; kx0 < ntx; kx0++, serp++) {
-        const int kx = (serp / ntx) & 1 ? ntx - 1 - kx0 : kx0;
-        for (int z = kz * TZ; z < std::min(g.nz, kz * TZ + TZ); z++)
-          for (int y = ky * TY; y < std::min(g.ny, ky * TY + TY); y++)
-            for (int x = kx * TX; x < std::min(nxc, kx * TX + TX); x++) g_hItems[n++] = x | (y << 8) | (z << 19);
-      }
-    }
-  nitems = n;
-  const double h = g.spacing;
-  const int n2x = g.nx / 2, n2y = g.ny / 2, n2z = g.nz / 2;
-  int nb = 0;
-  for (int i0 = 0; i0 < n; i0 += 256, nb++) {
-    agk::EmapBlock b{};
-    b.item0 = i0;
-    b.nitems = std::min(256, n - i0);
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-    for (int k = 0; k < b.nitems; k++) {
-      const int v = g_hItems[i0 + k];
-      const int xc = v & 0xFF, y = (v >> 8) & 0x7FF, z = (v >> 19) & 0x7FF;
-      const int xa = xc * agk::kNX, xb = std::min(g.nx - 1, xa + agk::kNX - 1);
-      const double p[2][3] = {{(xa - n2x) * h, (y - n2y) * h, (z - n2z) * h},
-                              {(xb - n2x) * h, (y - n2y) * h, (z - n2z) * h}};
-      for (int q = 0; q < 2; q++)
-        for (int d = 0; d < 3; d++) {
-          lo[d] = std::min(lo[d], p[q][d]);
-          hi[d] = std::max(hi[d], p[q][d]);
-        }
-    }
-    b.ox = 0.5 * (lo[0] + hi[0]);
-    b.oy = 0.5 * (lo[1] + hi[1]);
-    b.oz = 0.5 * (lo[2] + hi[2]);
-    b.hx = (float)(50.0 * (hi[0] - lo[0]) + 1.0);
-    b.hy = (float)(50.0 * (hi[1] - lo[1]) + 1.0);
-    b.hz = (float)(50.0 * (hi[2] - lo[2]) + 1.0);
-    const double diag = 2.0 * std::sqrt((double)b.hx * b.hx + (double)b.hy * b.hy + (double)b.hz * b.hz) / 100.0;
-    const double rFar = std::max(50.0, std::min(60.0, 81.0 - diag));
-    b.rfar2 = (float)((100.0 * rFar) * (100.0 * rFar));
-    b.clampMid = rFar + diag >= 81.0 ? 1 : 0;
-    g_hBlocks[nb] = b;
-  }
-  return nb;
+// Work items and CTA boxes of a grid, as for the ordinary entry points (a CTA
+// per 2 x 8 x 16 tile); grids that need more boxes than there is room for are
+// cut into full CTAs instead.
+int naItems(const ag_grid& g) {
+  static const int kTile[3] = {2, 8, 16};
+  const int nb = agc::makeItemsInto(g, kTile, 2, false, g_hItems, g_hBlocks, kNaMaxBlocks);
+  return nb >= 0 ? nb : agc::makeItemsInto(g, kTile, 2, true, g_hItems, g_hBlocks, kNaMaxBlocks);
 }
 
 }  // namespace
@@ -261,10 +223,8 @@ extern "C" int ag_emap_noalloc(const ag_grid* grid, int n_atoms, const double* d
   NaDevice& D = g_dev[dev];
   if (int e = naSetup(D)) return e;
   cudaStream_t st = (cudaStream_t)stream;
-  int nitems = 0;
-  const int nblocks = naItems(*grid, nitems);
-  if (nblocks < 0)
-    return naFail(AG_E_INVALID, "grid too large for ag_emap_noalloc (more than 1048576 work items of 8 points)");
+  const int64_t nitems = (int64_t)((grid->nx + agk::kNX - 1) / agk::kNX) * grid->ny * grid->nz;
+  const int nblocks = naItems(*grid);
   const int64_t np = (int64_t)grid->nx * grid->ny * grid->nz;
   if (n_atoms == 0) {
     if (cudaMemsetAsync(d_out, 0, sizeof(float) * np, st) != cudaSuccess ||
@@ -276,12 +236,10 @@ extern "C" int ag_emap_noalloc(const ag_grid* grid, int n_atoms, const double* d
   // partial-sum array's and the checksum array's capacity.
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int want = 2 * agk::kEmapCtasPerSm * sms;
-  int nsplit = 1;
-  if (nblocks < want && n_atoms > 512) nsplit = std::min((want + nblocks - 1) / nblocks, (n_atoms + 255) / 256);
-  nsplit = std::min(nsplit, kNaMaxSplit);
+  int chunk = agc::emapChunk(n_atoms, nblocks, sms, kNaCtasPerSm);
+  int nsplit = std::min((n_atoms + chunk - 1) / chunk, kNaMaxSplit);
   while (nsplit > 1 && (int64_t)nsplit * np > kNaMaxPartial) nsplit--;
-  const int chunk = ((n_atoms + nsplit - 1) / nsplit + 255) / 256 * 256;
+  chunk = std::max(chunk, ((n_atoms + nsplit - 1) / nsplit + 127) / 128 * 128);
   nsplit = std::max(1, (n_atoms + chunk - 1) / chunk);
 
   if (cudaMemcpyAsync(D.items, g_hItems, sizeof(int) * nitems, cudaMemcpyHostToDevice, st) != cudaSuccess ||
@@ -294,10 +252,12 @@ extern "C" int ag_emap_noalloc(const ag_grid* grid, int n_atoms, const double* d
   // (32 KB) and packed on the host, as for the ordinary entry points.
   int pkBytes = 0, b16 = 8192, b8 = 8192, vec8 = 0;
   float kScale = 0.f;
+  bool smooth = true;  // the constant dielectric
   if (d_inv_eps) {
     if (cudaMemcpyAsync(g_hTab, d_inv_eps, sizeof g_hTab, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
       return naFail(AG_E_CUDA, "cannot read the dielectric table");
+    smooth = agc::tableIsSmooth(g_hTab, 8192);
     pkBytes = agc::packTableTailInto(g_hTab, 8192, g_hPacked, agk::kEmapPackedBytes, b16, b8, vec8, kScale);
     if (pkBytes > 0 &&
         cudaMemcpyAsync(D.packed, g_hPacked, (size_t)pkBytes, cudaMemcpyHostToDevice, st) != cudaSuccess)
@@ -328,9 +288,9 @@ extern "C" int ag_emap_noalloc(const ag_grid* grid, int n_atoms, const double* d
     P.kScale = kScale;
   }
   P.thr = D.thr;
-  P.rnear2 = (100.f * 14.0f) * (100.f * 14.0f);
+  P.rnear2 = (100.f * kNaNear) * (100.f * kNaNear);
   P.delta = 2.0e-3f;
-  P.rnodeMin = INFINITY;
+  P.rnodeMin = smooth ? 100.f * (d_inv_eps ? kNaNode : kNaNear) : INFINITY;
   P.out = d_out;
   P.status = D.status;
   P.checksum = D.checksum;

@@ -231,7 +231,7 @@ int ag_main(int argc, char** argv);
  * cudaStream_t, NULL for the default stream) and the call is synchronous: it
  * returns when that work is done, so it cannot be recorded into a stream
  * capture (a call on a capturing stream fails with AG_E_CUDA).  Scratch
- * lives in fixed device arrays of the library (about 21 MiB on each device
+ * lives in fixed device arrays of the library (about 22 MiB on each device
  * that loads it, kept until exit): grids above about 8.4 million points
  * (1,048,576 rows of 8 points) are rejected with AG_E_INVALID, also before
  * any CUDA call.  All calls share those arrays and they keep the last call's

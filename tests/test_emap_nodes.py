@@ -109,6 +109,31 @@ def test_node_sums_match_point_sums_and_oracle(nx, ny, nz, h, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,nz,h", GRIDS + [(20, 300, 301, 0.375)])
+def test_allocation_free_call_matches_oracle(nx, ny, nz, h):
+    """ag_emap_noalloc on the same shapes, both dielectrics and a table that is not AutoGrid's
+    (sampled points on the largest, whose tiles are all ragged)."""
+    import ctypes
+
+    import torch
+
+    rng = np.random.default_rng(nx + ny)
+    xyzw = _atoms(rng, 500, 9.0)
+    g = fg.Grid(nx, ny, nz, h)
+    idx = np.unique(rng.integers(0, nx * ny * nz, 3000))
+    d_xyzw = torch.from_numpy(xyzw).cuda()
+    for eps in (fg.ddd_table(), None, fg.ddd_table() * 0.5):
+        d_eps = None if eps is None else torch.from_numpy(eps).float().cuda()
+        out = torch.full((nx * ny * nz,), float("nan"), device="cuda")
+        rc = fg.lib().ag_emap_noalloc(ctypes.byref(g), len(xyzw), d_xyzw.data_ptr(),
+                                      None if eps is None else d_eps.data_ptr(), out.data_ptr(),
+                                      torch.cuda.current_stream().cuda_stream)
+        assert rc == fg.AG_OK, fg.lib().ag_last_error()
+        want = oracle.emap_points(g, xyzw, eps, idx)
+        assert np.abs(out.cpu().numpy()[idx] - want).max() <= E_TOL
+
+
+@pytest.mark.gpu
 def test_other_tables_are_summed_point_by_point():
     """A table that is not AutoGrid's function keeps the point path: the same bits as with the
     node sums turned off."""
