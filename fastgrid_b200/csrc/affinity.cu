@@ -139,7 +139,12 @@ __device__ __forceinline__ void aff_unit(const AffParams& P, const int cta, unsi
 
   const int ch = valid ? P.closestH[pt] : -1;
   float rcx = 0.f, rcy = 0.f, rcz = 0.f;
-  if (ch >= 0) { rcx = P.rv[3 * ch]; rcy = P.rv[3 * ch + 1]; rcz = P.rv[3 * ch + 2]; }
+  if (ch >= 0) {
+    const float4 rc = P.rv8[2 * (size_t)ch];
+    rcx = rc.x;
+    rcy = rc.y;
+    rcz = rc.z;
+  }
 
   // Map sums in pairs (maps 2i, 2i+1): the table row's float4 halves add with
   // one packed FP32x2 instruction each (add.f32x2, rounded as two scalar adds).
@@ -450,8 +455,9 @@ __device__ __forceinline__ void aff_unit(const AffParams& P, const int cta, unsi
         c.vol = P.vol[atom];
         c.solq = P.solq[atom];
         c.info = P.info[atom];
-        c.rv[0] = P.rv[3 * atom]; c.rv[1] = P.rv[3 * atom + 1]; c.rv[2] = P.rv[3 * atom + 2];
-        c.rv2[0] = P.rv2[3 * atom]; c.rv2[1] = P.rv2[3 * atom + 1]; c.rv2[2] = P.rv2[3 * atom + 2];
+        const float4 va = P.rv8[2 * (size_t)atom], vb = P.rv8[2 * (size_t)atom + 1];
+        c.rv[0] = va.x; c.rv[1] = va.y; c.rv[2] = va.z;
+        c.rv2[0] = vb.x; c.rv2[1] = vb.y; c.rv2[2] = vb.z;
       }
       nb += tot;
       __syncthreads();

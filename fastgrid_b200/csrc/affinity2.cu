@@ -29,11 +29,15 @@
 //    before the map sums need it.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 
 #include "ag_device.cuh"
 #include "ag_kernels.h"
+
+// Lambdas that must be inlined: their captured sums stay in registers.
+#define AG_INLINE __attribute__((always_inline))
 
 namespace agk {
 
@@ -43,35 +47,83 @@ namespace {
 
 constexpr int kT = 256;              // threads per CTA, two points each
 constexpr int kW = kT / 32;
-constexpr int kCap = 640;            // candidate atoms per batch
 constexpr int kCellGroup = 128;      // cells per gather group (a CTA box reaches at most 4^3)
 constexpr float kBias = 8388608.f;   // 2^23
 
-struct A2Smem {
-  float4 pos[kCap];                  // CTA-local x, y, z; w = info bits
+constexpr int kPlaneRows = kA2PlaneRows;
+static_assert(kPlaneRows >= kAffRows && kPlaneRows * sizeof(float) % 16 == 0, "plane rows");
+
+// The pass is two kernels over the same CTA blocks: PLAIN forms the whole-row
+// map sums of every type, SLOTS the H-bond slots, from the types they apply to.
+enum { PART_PLAIN = 0, PART_SLOTS = 1 };
+
+// Candidate data only one of the parts needs.
+template <int PART>
+struct PartSmem;
+template <>
+struct PartSmem<PART_PLAIN> {
+  static constexpr int kCap = 640;   // candidate atoms per batch
   float2 vs[kCap];                   // vol, solq
+};
+template <>
+struct PartSmem<PART_SLOTS> {
+  static constexpr int kCap = 512;
   float4 rvA[kCap];                  // rvector x, y, z, rvector2 x
   float2 rvB[kCap];                  // rvector2 y, z
+  float4 rch[kT][2];                 // per thread and point: rvector of the nearest H donor
+};
+
+// The CTA's box in the grid-centred frame and the 8 A cells around it.
+struct Box {
+  double ox, oy, oz;                 // CTA frame origin (its first lattice point)
+  double lo[3], hi[3];               // CTA box
+  int c0[3], ncx, ncy, ncells;       // cells around the box
+};
+
+template <int PART>
+struct A2Smem : PartSmem<PART> {
+  using PartSmem<PART>::kCap;
+  float4 pos[kCap];                  // CTA-local x, y, z; w = info bits
   int idx[kCap];                     // atom index
   unsigned short wlist[kW][kCap];    // per warp: candidates within 8 A of its sub-box
-  int wStart[kW][kMaxTypes + 1];     // per warp: first wlist entry of each type
+  int wStart[kW][kMaxTypes + 1];     // per warp: first wlist entry of each type (in the part's type order)
   int typeCount[kMaxTypes];
   int typeStart[kMaxTypes + 1];
   int cellPre[kCellGroup + 1];
   int cellBeg[kCellGroup];
   int cnt[kW];
-  float sol[kAffRows + 1];           // + 0 at kAffRows (the out-of-cutoff entry)
-  float4 mask4[kMaxMapsPass / 4];    // current type: 1 for maps summed plainly, 0 for its H-bond slot maps
-  float4 rch[kT][2];                 // per thread and point: rvector of the nearest H donor
-  uint64_t bar;
-  // The nearest-donor search keeps each candidate's FP64 record where the map
-  // sums keep vs, rvA and rvB (the two phases do not overlap).
-  __device__ double4* d64() { return reinterpret_cast<double4*>(vs); }
+  Box box;
+  float sblo[kW][3], sbhi[kW][3];    // each warp's sub-box in the CTA frame (lo > hi: past the grid edge)
 };
-static_assert(offsetof(A2Smem, vs) % 32 == 0 && offsetof(A2Smem, idx) - offsetof(A2Smem, vs) == kCap * sizeof(double4),
-              "vs, rvA and rvB must hold kCap FP64 records");
 
-__host__ __device__ constexpr size_t tabOffset() { return ((sizeof(A2Smem) + 127) / 128) * 128; }
+// The barrier of a CTA's table copies.  It has shared memory of its own and is
+// set up once per CTA: the parts lay out the dynamic memory differently, and
+// an mbarrier's memory must not hold anything else while it is valid.
+struct TableBar {
+  uint64_t* bar;
+  unsigned phase;                    // copies waited for so far
+  __device__ __forceinline__ void init(uint64_t* b) {
+    bar = b;
+    phase = 0;
+    if (threadIdx.x == 0) {
+      mbar_init(b, 1);
+      fence_barrier_init();
+    }
+    __syncthreads();
+  }
+};
+
+// Dynamic shared memory: A2Smem, then the current type's table.  PLAIN: rows of
+// ncPad or nmPad columns, an extra all-zero row last (points beyond the
+// cutoff).  SLOTS: one plane per H-bond slot; the nearest-donor search keeps
+// each candidate's FP64 record there (the two phases do not overlap).
+template <int PART>
+__host__ __device__ constexpr size_t tabOffset() {
+  return ((sizeof(A2Smem<PART>) + 127) / 128) * 128;
+}
+constexpr size_t kSlotsRegion = kA2Slots * kPlaneRows * sizeof(float) > PartSmem<PART_SLOTS>::kCap * sizeof(double4)
+                                    ? kA2Slots * kPlaneRows * sizeof(float)
+                                    : PartSmem<PART_SLOTS>::kCap * sizeof(double4);
 
 __device__ __forceinline__ double rsq64(double ax, double ay, double az, double gx, double gy, double gz) {
   const double dx = __dsub_rn(ax, gx), dy = __dsub_rn(ay, gy), dz = __dsub_rn(az, gz);
@@ -90,68 +142,57 @@ __device__ double costheta64(double ax, double ay, double az, double gx, double 
 
 __device__ __forceinline__ float acos_clamped(float f) { return (f > 1.f) ? 0.f : (f < -1.f) ? 3.14159265f : acosf(f); }
 
-// Per-thread state: two points (p = 0, 1 at z and z + 1) and their sums.
-template <int NMAX>
+// A thread's two points (p = 0, 1 at z and z + 1).
 struct Pts {
   float px, py, pz[2];
   int ix, iy, iz0;
   bool valid[2];
-  int ch[2];                         // nearest H donor, or -1 (its rvector is in shared memory)
-  float2 em[2][NMAX / 2];            // plain map sums, maps (2i, 2i+1)
+};
+
+// Their plain sums.
+template <int NMAX>
+struct PlainSums {
+  float2 em[2][NMAX / 2];            // maps (2i, 2i+1)
   float s1[2], s2[2];                // desolvation sums (sol * vol, sol * solq)
-  float mn[2][kA2Slots], mx[2][kA2Slots];  // per slot: additive sum (acceptor probes) or min / max
+};
+
+// Their H-bond slots.
+struct SlotSums {
+  int ch[2];                         // nearest H donor, or -1 (its rvector is in shared memory)
+  float mn[2][kA2Slots], mx[2][kA2Slots];  // additive sum (acceptor probes) or min / max
   unsigned fl[2];                    // per slot: a min / max value was recorded
 };
 
 // FP64 grid-point coordinate as the reference forms it.
 __device__ __forceinline__ double gcoord(int i, int n2, double h) { return __dmul_rn((double)(i - n2), h); }
 
-// One receptor type's candidates in this warp's list, for both points.
-// ANG: angular class of the type; ISH: the type is "HD" (disordered ones are skipped).
-template <int NMAX, int ANG, bool ISH, bool PLAIN>
-__device__ __forceinline__ void run_type(const Aff2Params& P, const A2Smem& S, const float* tab, const int j0,
-                                         const int j1, const unsigned short* wl, const unsigned slots,
-                                         Pts<NMAX>& q) {
-  const int nmPad = P.nmPad;
-  const float4* tab4 = reinterpret_cast<const float4*>(tab);
-  const int rowQ = nmPad >> 2;       // float4 per row
-
-  // The next candidate's record is read one iteration ahead (its shared-memory
-  // latency overlaps the current candidate's arithmetic).
-  int cNext = j0 < j1 ? wl[j0] : 0;
-  float4 aNext = j0 < j1 ? S.pos[cNext] : make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int jj = j0; jj < j1; jj++) {
-    const int c = cNext;
-    const float4 a = aNext;
-    if (jj + 1 < j1) {
-      cNext = wl[jj + 1];
-      aNext = S.pos[cNext];
-    }
-    const float dx = a.x - q.px, dy = a.y - q.py;
+// One candidate against the two points: offsets, 1 / r, table row and whether
+// the point is within the 8 A cutoff.  Returns false if it is for no lane.
+struct Pair {
+  float dx, dy, dz[2], rs[2];
+  int iR[2];                         // table row; kAffRows (the zero row) beyond the cutoff
+  bool in[2];
+  __device__ __forceinline__ bool set(const Aff2Params& P, const int* idx, const int c, const float4 a, const Pts& q) {
+    dx = a.x - q.px;
+    dy = a.y - q.py;
     const float dxy = fmaf(dy, dy, dx * dx);
-    float dz[2], r2[2];
-    bool in[2];
+    float r2[2];
 #pragma unroll
     for (int p = 0; p < 2; p++) {
       dz[p] = a.z - q.pz[p];
       r2[p] = fmaf(dz[p], dz[p], dxy);
       in[p] = q.valid[p] && r2[p] <= 64.0002f;
     }
-    if (!__any_sync(0xffffffffu, in[0] || in[1])) continue;
-    const int info = __float_as_int(a.w);
-    const bool dis = (info >> 8) & 1;
-    if (ISH && dis) continue;        // the reference skips disordered hydrogens (:280); uniform: one candidate
+    if (!__any_sync(0xffffffffu, in[0] || in[1])) return false;
     // Exact 8 A cutoff near the edge.
 #pragma unroll
     for (int p = 0; p < 2; p++)
       if (in[p] && r2[p] > 63.9998f) {
-        const double4 a64 = P.xyz[S.idx[c]];
+        const double4 a64 = P.xyz[idx[c]];
         if (rsq64(a64.x, a64.y, a64.z, gcoord(q.ix, P.n2x, P.h), gcoord(q.iy, P.n2y, P.h),
                   gcoord(q.iz0 + p, P.n2z, P.h)) > 64.0)
           in[p] = false;
       }
-    float rs[2];
-    int iR[2];
 #pragma unroll
     for (int p = 0; p < 2; p++) {
       const float r2c = fmaxf(r2[p], 1.0e-24f);
@@ -165,46 +206,110 @@ __device__ __forceinline__ void run_type(const Aff2Params& P, const A2Smem& S, c
         // Within the guard band of a bin edge: the reference's FP64 bin
         // int(100 / (1 / sqrt(r^2))) through the table of r^2 thresholds.
         const int k = min(fr > 0.5f ? b + 1 : b, kAffRows);
-        const double4 a64 = P.xyz[S.idx[c]];
+        const double4 a64 = P.xyz[idx[c]];
         const double r64 = rsq64(a64.x, a64.y, a64.z, gcoord(q.ix, P.n2x, P.h), gcoord(q.iy, P.n2y, P.h),
                                  gcoord(q.iz0 + p, P.n2z, P.h));
         b = (r64 >= P.thr[k]) ? k : k - 1;
       }
-      iR[p] = in[p] ? min(max(b, 0), kAffRows - 1) : kAffRows;  // kAffRows: the zero row
+      iR[p] = in[p] ? min(max(b, 0), kAffRows - 1) : kAffRows;
     }
-    // Plain map sums: whole rows.  PLAIN (no H-bond slot applies to this type)
-    // adds them directly, otherwise through the type's 0/1 mask.  When the pass
-    // has a spare column the row's last entry holds the desolvation value.
+    return true;
+  }
+};
+
+// Whether a candidate is left out: the reference skips disordered hydrogens
+// (CalculateGridmaps.cpp:280).  ISH: the candidate's type is "HD".
+template <bool ISH>
+__device__ __forceinline__ bool skipped(const float4 a) {
+  return ISH && ((__float_as_int(a.w) >> 8) & 1);
+}
+
+// Distance between table rows of rowQ float4s, in float4s: odd, so that the
+// rows a quarter-warp reads at once start in any of the eight 16-byte bank
+// groups (rows 8 columns apart would meet in four of them).
+__host__ __device__ constexpr int row_stride(int rowQ) { return rowQ | 1; }
+
+// Plain sums of one receptor type's candidates in this warp's list: whole table
+// rows of rowQ float4s, whose last entry is the desolvation value.
+template <int NMAX, bool ISH>
+__device__ __forceinline__ void plain_sums(const Aff2Params& P, const A2Smem<PART_PLAIN>& S, const float* tab,
+                                           const int rowQ, const int j0, const int j1, const unsigned short* wl,
+                                           const Pts& q, PlainSums<NMAX>& s) {
+  const int strideQ = row_stride(rowQ);
+  const float4* tab4 = reinterpret_cast<const float4*>(tab);
+  // The next candidate's record is read one iteration ahead (its shared-memory
+  // latency overlaps the current candidate's arithmetic).
+  int cNext = j0 < j1 ? wl[j0] : 0;
+  float4 aNext = j0 < j1 ? S.pos[cNext] : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int jj = j0; jj < j1; jj++) {
+    const int c = cNext;
+    const float4 a = aNext;
+    if (jj + 1 < j1) {
+      cNext = wl[jj + 1];
+      aNext = S.pos[cNext];
+    }
+    Pair w;
+    if (skipped<ISH>(a) || !w.set(P, S.idx, c, a, q)) continue;  // uniform: one candidate
     float solv[2] = {0.f, 0.f};
-    const int lastQ = rowQ - 1;
 #pragma unroll
     for (int g4 = 0; g4 < NMAX / 4; g4++) {
-      if (4 * g4 >= P.nmaps) break;
-      float4 m4 = make_float4(1.f, 1.f, 1.f, 1.f);
-      if (!PLAIN) m4 = S.mask4[g4];  // same address in every lane: one broadcast for both points
+      if (g4 >= rowQ) break;         // uniform
 #pragma unroll
       for (int p = 0; p < 2; p++) {
-        const float4 e4 = tab4[iR[p] * rowQ + g4];
-        if (PLAIN) {
-          q.em[p][2 * g4] = __fadd2_rn(q.em[p][2 * g4], make_float2(e4.x, e4.y));
-          q.em[p][2 * g4 + 1] = __fadd2_rn(q.em[p][2 * g4 + 1], make_float2(e4.z, e4.w));
-        } else {
-          q.em[p][2 * g4] = __ffma2_rn(make_float2(e4.x, e4.y), make_float2(m4.x, m4.y), q.em[p][2 * g4]);
-          q.em[p][2 * g4 + 1] = __ffma2_rn(make_float2(e4.z, e4.w), make_float2(m4.z, m4.w), q.em[p][2 * g4 + 1]);
-        }
-        if (g4 == lastQ) solv[p] = e4.w;
+        const float4 e4 = tab4[w.iR[p] * strideQ + g4];
+        s.em[p][2 * g4] = __fadd2_rn(s.em[p][2 * g4], make_float2(e4.x, e4.y));
+        s.em[p][2 * g4 + 1] = __fadd2_rn(s.em[p][2 * g4 + 1], make_float2(e4.z, e4.w));
+        solv[p] = e4.w;
       }
     }
     const float2 v = S.vs[c];
 #pragma unroll
     for (int p = 0; p < 2; p++) {
-      const float sv = P.solInRow ? solv[p] : S.sol[iR[p]];
-      q.s1[p] = fmaf(sv, v.x, q.s1[p]);
-      q.s2[p] = fmaf(sv, v.y, q.s2[p]);
+      s.s1[p] = fmaf(solv[p], v.x, s.s1[p]);
+      s.s2[p] = fmaf(solv[p], v.y, s.s2[p]);
     }
-    if (PLAIN) continue;
+  }
+}
 
-    // Directional factors (CalculateGridmaps.cpp:84-197) and the H-bond slots (:199-232).
+// From column-class sums to map sums: each map takes its class's sum.
+template <int NMAX>
+__device__ __forceinline__ void expand_classes(const Aff2Params& P, PlainSums<NMAX>& s) {
+#pragma unroll
+  for (int p = 0; p < 2; p++) {
+    float old[NMAX], v[NMAX];
+#pragma unroll
+    for (int g = 0; g < NMAX; g++) old[g] = (g & 1) ? s.em[p][g >> 1].y : s.em[p][g >> 1].x;
+#pragma unroll
+    for (int g = 0; g < NMAX; g++) {
+      const int c = (int)(P.classOf >> (4 * g)) & 15;
+      v[g] = 0.f;
+#pragma unroll
+      for (int k = 0; k < NMAX; k++) v[g] = k == c ? old[k] : v[g];
+    }
+#pragma unroll
+    for (int g = 0; g < NMAX / 2; g++) s.em[p][g] = make_float2(v[2 * g], v[2 * g + 1]);
+  }
+}
+
+// H-bond slots of one receptor type's candidates (CalculateGridmaps.cpp:199-232)
+// with the directional factors of its angular class ANG (:84-197).
+template <int ANG, bool ISH>
+__device__ __forceinline__ void slot_terms(const Aff2Params& P, const A2Smem<PART_SLOTS>& S, const float* tab,
+                                           const int j0, const int j1, const unsigned short* wl, const unsigned slots,
+                                           const Pts& q, SlotSums& s) {
+  int cNext = j0 < j1 ? wl[j0] : 0;
+  float4 aNext = j0 < j1 ? S.pos[cNext] : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int jj = j0; jj < j1; jj++) {
+    const int c = cNext;
+    const float4 a = aNext;
+    if (jj + 1 < j1) {
+      cNext = wl[jj + 1];
+      aNext = S.pos[cNext];
+    }
+    Pair w;
+    if (skipped<ISH>(a) || !w.set(P, S.idx, c, a, q)) continue;  // uniform: one candidate
+    const int info = __float_as_int(a.w);
+    const bool dis = (info >> 8) & 1;
     float racc[2] = {1.f, 1.f}, rdon[2] = {1.f, 1.f}, hramp[2] = {1.f, 1.f};
     if (ANG != A2_SPH) {
       const int idx = S.idx[c];
@@ -212,8 +317,8 @@ __device__ __forceinline__ void run_type(const Aff2Params& P, const A2Smem& S, c
       const float2 rb = S.rvB[c];
 #pragma unroll
       for (int p = 0; p < 2; p++) {
-        if (!in[p]) continue;
-        const float ux = dx * rs[p], uy = dy * rs[p], uz = dz[p] * rs[p];
+        if (!w.in[p]) continue;
+        const float ux = w.dx * w.rs[p], uy = w.dy * w.rs[p], uz = w.dz[p] * w.rs[p];
         float cosT = -(ux * ra.x + uy * ra.y + uz * ra.z);
         bool gt0 = cosT > 0.f, ge0 = cosT >= 0.f;
         if ((ANG == A2_D1 || (ANG == A2_A2 && !dis)) && fabsf(cosT) < 1.0e-5f) {
@@ -233,7 +338,7 @@ __device__ __forceinline__ void run_type(const Aff2Params& P, const A2Smem& S, c
             if (rexp == 4) ra2 = ra2 * ra2;
             if (rexp == 4 || rexp == 2) ra2 = ra2 * ra2;
             racc[p] = ra2;
-            if (idx != q.ch[p] && q.ch[p] >= 0) {
+            if (idx != s.ch[p] && s.ch[p] >= 0) {
               const float4 rc = S.rch[threadIdx.x][p];
               const float cc = rc.x * ra.x + rc.y * ra.y + rc.z * ra.z;
               // cos on the SFU over [0, pi]; cos(x) = cos(2 pi - x) folds 4 theta / 3.
@@ -249,8 +354,8 @@ __device__ __forceinline__ void run_type(const Aff2Params& P, const A2Smem& S, c
             racc[p] = 0.f;
             rdon[p] = 0.f;
             if (cosT >= -0.94832352f) {
-              const float s = sqrtf(fmaxf(0.f, 1.f - cosT * cosT));
-              const float cs = cosT * 0.31730505f + s * 0.94832352f;  // cos(theta - 1.24791)
+              const float sn = sqrtf(fmaxf(0.f, 1.f - cosT * cosT));
+              const float cs = cosT * 0.31730505f + sn * 0.94832352f;  // cos(theta - 1.24791)
               rdon[p] = (cs * cs) * (cs * cs);
               racc[p] = rdon[p];
             }
@@ -279,22 +384,22 @@ __device__ __forceinline__ void run_type(const Aff2Params& P, const A2Smem& S, c
 #pragma unroll
     for (int k = 0; k < kA2Slots; k++) {
       if (!((slots >> k) & 1u)) continue;   // uniform
-      const int m = P.slotMap[k];
       const int kind = P.slotKind[k];
 #pragma unroll
       for (int p = 0; p < 2; p++) {
-        if (!in[p]) continue;
-        const float E = tab[iR[p] * nmPad + m];
+        if (!w.in[p]) continue;
+        const float E = tab[k * kPlaneRows + w.iR[p]];
         const float rsph = fminf(fmaxf(E * 0.01f, 0.f), 1.f);
         if (kind == A2_SLOT_ACC) {
-          const float e = dis ? (P.tableH ? __ldg(P.tableH + max(0, iR[p] - 110) * nmPad + m) : 0.f) : E;
-          q.mn[p][k] += e * hramp[p] * (racc[p] + (1.f - racc[p]) * rsph);
+          // Disordered donors take the "HD" type's row 1.1 A in.
+          const float e = dis ? (P.planeH ? __ldg(P.planeH + k * kPlaneRows + max(0, w.iR[p] - 110)) : 0.f) : E;
+          s.mn[p][k] += e * hramp[p] * (racc[p] + (1.f - racc[p]) * rsph);
         } else {
           const float f = (kind == A2_SLOT_A1) ? racc[p] : rdon[p];
           const float val = E * (f + (1.f - f) * rsph);
-          q.mn[p][k] = fminf(q.mn[p][k], val);
-          q.mx[p][k] = fmaxf(q.mx[p][k], val);
-          q.fl[p] |= 1u << k;
+          s.mn[p][k] = fminf(s.mn[p][k], val);
+          s.mx[p][k] = fmaxf(s.mx[p][k], val);
+          s.fl[p] |= 1u << k;
         }
       }
     }
@@ -303,21 +408,16 @@ __device__ __forceinline__ void run_type(const Aff2Params& P, const A2Smem& S, c
 
 }  // namespace
 
-size_t aff2_smem_bytes(int nmPad) { return tabOffset() + sizeof(float) * (size_t)(kAffRows + 1) * nmPad; }
-
-// The CTA's box in the grid-centred frame, the 8 A cells around it and the
-// calling warp's sub-box in the CTA frame.
-struct Box {
-  double ox, oy, oz;                 // CTA frame origin (its first lattice point)
-  double lo[3], hi[3];               // CTA box
-  int c0[3], ncx, ncy, ncells;       // cells around the box
-  float sblo[3], sbhi[3];            // this warp's sub-box
-  bool warpEmpty;
-};
+static size_t aff2_smem(int nmPad, bool slots) {
+  const size_t plain = tabOffset<PART_PLAIN>() + sizeof(float4) * (size_t)(kAffRows + 1) * row_stride(nmPad >> 2);
+  return slots ? std::max(plain, tabOffset<PART_SLOTS>() + kSlotsRegion) : plain;
+}
 
 // Cell ranges of receptor type t in cell group cg: S.cellBeg / S.cellPre.
 // Returns the group's cell count (S.cellPre[ncg] is its atom count).
-__device__ __forceinline__ int cell_prefix(const Aff2Params& P, A2Smem& S, const Box& B, const int t, const int cg) {
+template <int PART>
+__device__ __forceinline__ int cell_prefix(const Aff2Params& P, A2Smem<PART>& S, const int t, const int cg) {
+  const Box& B = S.box;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ncg = min(kCellGroup, B.ncells - cg);
   __syncthreads();  // the previous group's ranges are no longer read
@@ -359,11 +459,15 @@ __device__ __forceinline__ int cell_prefix(const Aff2Params& P, A2Smem& S, const
   return ncg;
 }
 
-// Up to kT atoms v0 .. v0 + kT of the current cell group (type t) that lie
+// Up to kT atoms v0 .. v0 + kT of the current cell group (the type at place
+// `pos` of the part's order) that lie
 // within 8 A of the CTA box, appended to the candidate arrays at slot nb
-// (full: with the fields the map sums need).  Returns the new count.
-__device__ __forceinline__ int gather_chunk(const Aff2Params& P, A2Smem& S, const Box& B, const int t, const int ncg,
-                                            const int total, const int v0, const int nb, const bool full) {
+// (d64: with their FP64 records there, else with the fields of the part's
+// sums).  Returns the new count.
+template <int PART>
+__device__ __forceinline__ int gather_chunk(const Aff2Params& P, A2Smem<PART>& S, const int pos, const int ncg,
+                                            const int total, const int v0, const int nb, double4* d64) {
+  const Box& B = S.box;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int v = v0 + tid;
   bool keep = false;
@@ -396,15 +500,17 @@ __device__ __forceinline__ int gather_chunk(const Aff2Params& P, A2Smem& S, cons
     const int inf = P.info[atom];
     S.pos[j] = make_float4((float)(a.x - B.ox), (float)(a.y - B.oy), (float)(a.z - B.oz), __int_as_float(inf));
     S.idx[j] = atom;
-    if (full) {
+    if constexpr (PART == PART_PLAIN) {
       S.vs[j] = make_float2(P.vol[atom], P.solq[atom]);
-      S.rvA[j] = make_float4(P.rv[3 * atom], P.rv[3 * atom + 1], P.rv[3 * atom + 2], P.rv2[3 * atom]);
-      S.rvB[j] = make_float2(P.rv2[3 * atom + 1], P.rv2[3 * atom + 2]);
+    } else if (d64) {
+      d64[j] = a;
     } else {
-      S.d64()[j] = a;
+      const float4 va = __ldg(P.rv8 + 2 * (size_t)atom), vb = __ldg(P.rv8 + 2 * (size_t)atom + 1);
+      S.rvA[j] = make_float4(va.x, va.y, va.z, vb.x);
+      S.rvB[j] = make_float2(vb.y, vb.z);
     }
   }
-  if (tid == 0) S.typeCount[t] += tot;
+  if (tid == 0) S.typeCount[pos] += tot;
   __syncthreads();
   return nb + tot;
 }
@@ -414,9 +520,8 @@ __device__ __forceinline__ int gather_chunk(const Aff2Params& P, A2Smem& S, cons
 // point's smallest r^2 in the batch; the FP64 distance (from the records in
 // shared memory) is formed only for the candidates within 1e-3 A^2 of it,
 // which the FP32 error (< 1e-4 A^2) cannot hide.
-template <int NMAX>
-__device__ __forceinline__ void scan_donors(const Aff2Params& P, A2Smem& S, const int nb, double (&best)[2],
-                                            int (&bi)[2], const Pts<NMAX>& q) {
+__device__ __forceinline__ void scan_donors(const Aff2Params& P, const A2Smem<PART_SLOTS>& S, const double4* d64,
+                                            const int nb, double (&best)[2], int (&bi)[2], const Pts& q) {
   __syncthreads();
   float lim[2] = {3.0e38f, 3.0e38f};
   for (int j = 0; j < nb; j++) {
@@ -431,7 +536,6 @@ __device__ __forceinline__ void scan_donors(const Aff2Params& P, A2Smem& S, cons
   }
 #pragma unroll
   for (int p = 0; p < 2; p++) lim[p] = fminf(lim[p], (float)best[p]) + 1.0e-3f;
-  const double4* d64 = S.d64();
   for (int j = 0; j < nb; j++) {
     const float4 a = S.pos[j];
     const float dx = a.x - q.px, dy = a.y - q.py;
@@ -454,36 +558,39 @@ __device__ __forceinline__ void scan_donors(const Aff2Params& P, A2Smem& S, cons
   __syncthreads();
 }
 
-// One batch of nb candidates: per-warp lists, then the types one by one.
-// Returns false if a table copy's bounded wait expired (status set).
-template <int NMAX>
-__device__ __forceinline__ bool process_batch(const Aff2Params& P, A2Smem& S, float* tab, const Box& B, const int nb,
-                                              unsigned& phase, Pts<NMAX>& q) {
+// One batch of nb candidates: per-warp lists, then the part's ntypes types one
+// by one.  load(pos) starts the copy of the table of the type at place `pos`
+// of the part's order (one thread), and sums(pos, ...) takes the type's
+// candidates [j0, j1) of the warp's list.  Returns false if a table copy's
+// bounded wait expired (status set).
+template <int PART, class Load, class Sums>
+__device__ __forceinline__ bool process_batch(const Aff2Params& P, A2Smem<PART>& S, const int ntypes, const int nb,
+                                              TableBar& tb, const Load& load, const Sums& sums) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nmPad = P.nmPad;
-  const unsigned tabBytes = (unsigned)(kAffRows * nmPad * sizeof(float));
   __syncthreads();  // candidate records and counts are complete
   if (tid == 0) {
     int s = 0;
-    for (int t = 0; t < P.ntypes; t++) {
+    for (int t = 0; t < ntypes; t++) {
       S.typeStart[t] = s;
       s += S.typeCount[t];
       S.typeCount[t] = 0;
     }
-    S.typeStart[P.ntypes] = s;
+    S.typeStart[ntypes] = s;
   }
   __syncthreads();
   // This warp's list: the candidates within 8 A of its sub-box (FP32 with margin).
   int nw = 0;
-  if (!B.warpEmpty)
+  const float* sblo = S.sblo[warp];
+  const float* sbhi = S.sbhi[warp];
+  if (sblo[0] <= sbhi[0])
     for (int base = 0; base < nb; base += 32) {
       const int j = base + lane;
       bool keep = false;
       if (j < nb) {
         const float4 a = S.pos[j];
-        const float ddx = fmaxf(fmaxf(B.sblo[0] - a.x, a.x - B.sbhi[0]), 0.f);
-        const float ddy = fmaxf(fmaxf(B.sblo[1] - a.y, a.y - B.sbhi[1]), 0.f);
-        const float ddz = fmaxf(fmaxf(B.sblo[2] - a.z, a.z - B.sbhi[2]), 0.f);
+        const float ddx = fmaxf(fmaxf(sblo[0] - a.x, a.x - sbhi[0]), 0.f);
+        const float ddy = fmaxf(fmaxf(sblo[1] - a.y, a.y - sbhi[1]), 0.f);
+        const float ddz = fmaxf(fmaxf(sblo[2] - a.z, a.z - sbhi[2]), 0.f);
         keep = fmaf(ddz, ddz, fmaf(ddy, ddy, ddx * ddx)) <= 64.01f;
       }
       const unsigned b = __ballot_sync(0xffffffffu, keep);
@@ -491,7 +598,7 @@ __device__ __forceinline__ bool process_batch(const Aff2Params& P, A2Smem& S, fl
       nw += __popc(b);
     }
   __syncwarp();
-  for (int t = lane; t <= P.ntypes; t += 32) {  // first entry of each type (the list is sorted)
+  for (int t = lane; t <= ntypes; t += 32) {  // first entry of each type (the list is sorted)
     const int target = S.typeStart[t];
     int a = 0, b = nw;
     while (a < b) {
@@ -501,249 +608,373 @@ __device__ __forceinline__ bool process_batch(const Aff2Params& P, A2Smem& S, fl
     S.wStart[warp][t] = a;
   }
   __syncwarp();
-  for (int t = 0; t < P.ntypes; t++) {
+  for (int t = 0; t < ntypes; t++) {
     if (S.typeStart[t + 1] == S.typeStart[t]) continue;  // uniform
     if (tid == 0) {
       fence_proxy_async();
-      mbar_arrive_expect_tx(&S.bar, tabBytes);
-      tma_load_1d(tab, P.table + (size_t)t * kAffRows * nmPad, tabBytes, &S.bar);
+      load(t);
     }
-    if (tid < kMaxMapsPass) {  // read after the __syncthreads_or below
-      const unsigned plain = P.typePlain[t];
-      reinterpret_cast<float*>(S.mask4)[tid] = (plain >> tid) & 1u ? 1.f : 0.f;
-    }
-    const bool ok = mbar_wait_bounded(&S.bar, phase & 1u, P.status);
+    const bool ok = mbar_wait_bounded(tb.bar, tb.phase & 1u, P.status);
     if (__syncthreads_or(!ok)) {
-      if (tid == 0) mbar_wait_bounded(&S.bar, phase & 1u, P.status);  // let the copy land before leaving
+      if (tid == 0) mbar_wait_bounded(tb.bar, tb.phase & 1u, P.status);  // let the copy land before leaving
       return false;
     }
-    phase++;
-    const int j0 = S.wStart[warp][t], j1 = S.wStart[warp][t + 1];
-    const unsigned slots = P.typeSlots[t];
-    const unsigned short* wl = S.wlist[warp];
-    const bool ish = (t == P.hydrogen);
-    if (slots == 0u) {  // uniform: no H-bond term, no angular factors
-      if (ish) run_type<NMAX, A2_SPH, true, true>(P, S, tab, j0, j1, wl, slots, q);
-      else run_type<NMAX, A2_SPH, false, true>(P, S, tab, j0, j1, wl, slots, q);
-    } else {
-      switch (P.typeAng[t]) {  // uniform
-        case A2_D1:
-          if (ish) run_type<NMAX, A2_D1, true, false>(P, S, tab, j0, j1, wl, slots, q);
-          else run_type<NMAX, A2_D1, false, false>(P, S, tab, j0, j1, wl, slots, q);
-          break;
-        case A2_A1: run_type<NMAX, A2_A1, false, false>(P, S, tab, j0, j1, wl, slots, q); break;
-        case A2_A2: run_type<NMAX, A2_A2, false, false>(P, S, tab, j0, j1, wl, slots, q); break;
-        default:
-          if (ish) run_type<NMAX, A2_SPH, true, false>(P, S, tab, j0, j1, wl, slots, q);
-          else run_type<NMAX, A2_SPH, false, false>(P, S, tab, j0, j1, wl, slots, q);
-          break;
-      }
-    }
+    tb.phase++;
+    sums(t, S.wStart[warp][t], S.wStart[warp][t + 1], S.wlist[warp]);
     __syncthreads();  // the table buffer is free for the next type
   }
   return true;
 }
 
-// One work unit: the CTA block `cta` of job P.  Called once per CTA by
-// affinity2_kernel and repeatedly by the persistent batch kernel.
-template <int NMAX>
-__device__ __forceinline__ void aff2_unit(const Aff2Params& P, const int cta, unsigned char* smem_raw) {
-  A2Smem& S = *reinterpret_cast<A2Smem*>(smem_raw);
-  float* tab = reinterpret_cast<float*>(smem_raw + tabOffset());
+// One work unit: a part of the CTA block `cta` of job P.  The two parts of a
+// block run in either order or together: maps with an H-bond slot start at
+// zero and both parts add to them (a sum of two terms, the same in any order).
+// Returns false if a wait expired (status set; the barrier is not used again).
+template <int NMAX, int PART>
+__device__ __forceinline__ bool aff2_unit(const Aff2Params& P, const int cta, unsigned char* smem_raw, TableBar& tb) {
+  A2Smem<PART>& S = *reinterpret_cast<A2Smem<PART>*>(smem_raw);
+  float* tab = reinterpret_cast<float*>(smem_raw + tabOffset<PART>());
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nmPad = P.nmPad;
+  constexpr int kCap = A2Smem<PART>::kCap;
 
   // This CTA's 8 x 8 x 8 points; this warp's 4 x 4 x 4 sub-box; this thread's two points.
   const int tbx = (P.nx + 7) / 8, tby = (P.ny + 7) / 8;
   const int x0 = (cta % tbx) * 8, y0 = ((cta / tbx) % tby) * 8, z0 = (cta / (tbx * tby)) * 8;
   const int wx = x0 + (warp & 1) * 4, wy = y0 + ((warp >> 1) & 1) * 4, wz = z0 + (warp >> 2) * 4;
-  Pts<NMAX> q;
+  Pts q;
   q.ix = wx + (lane & 3);
   q.iy = wy + ((lane >> 2) & 3);
   q.iz0 = wz + (lane >> 4) * 2;
   q.valid[0] = q.ix < P.nx && q.iy < P.ny && q.iz0 < P.nz;
   q.valid[1] = q.ix < P.nx && q.iy < P.ny && q.iz0 + 1 < P.nz;
-  const double h = P.h;
-  Box B;
-  B.ox = gcoord(x0, P.n2x, h);
-  B.oy = gcoord(y0, P.n2y, h);
-  B.oz = gcoord(z0, P.n2z, h);
-  q.px = (float)(gcoord(q.ix, P.n2x, h) - B.ox);
-  q.py = (float)(gcoord(q.iy, P.n2y, h) - B.oy);
-  q.pz[0] = (float)(gcoord(q.iz0, P.n2z, h) - B.oz);
-  q.pz[1] = (float)(gcoord(q.iz0 + 1, P.n2z, h) - B.oz);
-
-  // CTA box (FP64, grid-centred) and the 8 A cells around it.
-  B.lo[0] = B.ox; B.hi[0] = gcoord(min(x0 + 8, P.nx) - 1, P.n2x, h);
-  B.lo[1] = B.oy; B.hi[1] = gcoord(min(y0 + 8, P.ny) - 1, P.n2y, h);
-  B.lo[2] = B.oz; B.hi[2] = gcoord(min(z0 + 8, P.nz) - 1, P.n2z, h);
-  int c1[3];
+  {
+    const double h = P.h;
+    const double ox = gcoord(x0, P.n2x, h), oy = gcoord(y0, P.n2y, h), oz = gcoord(z0, P.n2z, h);
+    q.px = (float)(gcoord(q.ix, P.n2x, h) - ox);
+    q.py = (float)(gcoord(q.iy, P.n2y, h) - oy);
+    q.pz[0] = (float)(gcoord(q.iz0, P.n2z, h) - oz);
+    q.pz[1] = (float)(gcoord(q.iz0 + 1, P.n2z, h) - oz);
+    // CTA box (FP64, grid-centred) and the 8 A cells around it.
+    if (tid == 0) {
+      Box& B = S.box;
+      B.ox = ox;
+      B.oy = oy;
+      B.oz = oz;
+      B.lo[0] = ox; B.hi[0] = gcoord(min(x0 + 8, P.nx) - 1, P.n2x, h);
+      B.lo[1] = oy; B.hi[1] = gcoord(min(y0 + 8, P.ny) - 1, P.n2y, h);
+      B.lo[2] = oz; B.hi[2] = gcoord(min(z0 + 8, P.nz) - 1, P.n2z, h);
+      int nc[3];
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
-    B.c0[d] = max(0, (int)floor((B.lo[d] - 8.0 - P.cellLo[d]) / 8.0));
-    c1[d] = min(P.ncell[d] - 1, (int)floor((B.hi[d] + 8.0 - P.cellLo[d]) / 8.0));
-  }
-  B.ncx = c1[0] - B.c0[0] + 1;
-  B.ncy = c1[1] - B.c0[1] + 1;
-  const int ncz = c1[2] - B.c0[2] + 1;
-  B.ncells = (B.ncx > 0 && B.ncy > 0 && ncz > 0) ? B.ncx * B.ncy * ncz : 0;
-
-  // This warp's sub-box in the CTA frame (empty when it lies past the grid edge).
-  B.warpEmpty = wx >= P.nx || wy >= P.ny || wz >= P.nz;
-  B.sblo[0] = (float)(gcoord(wx, P.n2x, h) - B.ox); B.sbhi[0] = (float)(gcoord(min(wx + 3, P.nx - 1), P.n2x, h) - B.ox);
-  B.sblo[1] = (float)(gcoord(wy, P.n2y, h) - B.oy); B.sbhi[1] = (float)(gcoord(min(wy + 3, P.ny - 1), P.n2y, h) - B.oy);
-  B.sblo[2] = (float)(gcoord(wz, P.n2z, h) - B.oz); B.sbhi[2] = (float)(gcoord(min(wz + 3, P.nz - 1), P.n2z, h) - B.oz);
-
-  for (int i = tid; i < kAffRows + 1; i += kT) S.sol[i] = i < kAffRows ? P.sol[i] : 0.f;
-  for (int i = tid; i < nmPad; i += kT) tab[kAffRows * nmPad + i] = 0.f;
-  for (int t = tid; t < kMaxTypes; t += kT) S.typeCount[t] = 0;
-  if (tid == 0) {
-    mbar_init(&S.bar, 1);
-    fence_barrier_init();
-  }
-
-#pragma unroll
-  for (int p = 0; p < 2; p++) {
-    q.s1[p] = 0.f;
-    q.s2[p] = 0.f;
-    q.fl[p] = 0u;
-    q.ch[p] = -1;
-#pragma unroll
-    for (int g = 0; g < NMAX / 2; g++) q.em[p][g] = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int k = 0; k < kA2Slots; k++) {
-      q.mn[p][k] = (P.slotKind[k] == A2_SLOT_ACC) ? 0.f : 999999.f;
-      q.mx[p][k] = -999999.f;
+      for (int d = 0; d < 3; d++) {
+        B.c0[d] = max(0, (int)floor((B.lo[d] - 8.0 - P.cellLo[d]) / 8.0));
+        nc[d] = min(P.ncell[d] - 1, (int)floor((B.hi[d] + 8.0 - P.cellLo[d]) / 8.0)) - B.c0[d] + 1;
+      }
+      B.ncx = nc[0];
+      B.ncy = nc[1];
+      B.ncells = (nc[0] > 0 && nc[1] > 0 && nc[2] > 0) ? nc[0] * nc[1] * nc[2] : 0;
+    }
+    // This warp's sub-box in the CTA frame (empty when it lies past the grid edge).
+    if (lane == 0) {
+      const bool empty = wx >= P.nx || wy >= P.ny || wz >= P.nz;
+      S.sblo[warp][0] = empty ? 1.f : (float)(gcoord(wx, P.n2x, h) - ox);
+      S.sbhi[warp][0] = empty ? 0.f : (float)(gcoord(min(wx + 3, P.nx - 1), P.n2x, h) - ox);
+      S.sblo[warp][1] = (float)(gcoord(wy, P.n2y, h) - oy);
+      S.sbhi[warp][1] = (float)(gcoord(min(wy + 3, P.ny - 1), P.n2y, h) - oy);
+      S.sblo[warp][2] = (float)(gcoord(wz, P.n2z, h) - oz);
+      S.sbhi[warp][2] = (float)(gcoord(min(wz + 3, P.nz - 1), P.n2z, h) - oz);
     }
   }
-  __syncthreads();
-
-  // ---- the nearest H donor of both points, from the donors within 8 A of the box ----
+  for (int t = tid; t < kMaxTypes; t += kT) S.typeCount[t] = 0;
   int nb = 0;
-  if (P.needClosestH) {
-    double best[2] = {1e300, 1e300};
-    int bi[2] = {-1, -1};
-    for (int t = 0; t < P.ntypes; t++) {
-      if (!P.typeDonor[t]) continue;
-      for (int cg = 0; cg < B.ncells; cg += kCellGroup) {
-        const int ncg = cell_prefix(P, S, B, t, cg);
+
+  // Batches of candidates in type-major order, walked type by type.
+  auto walk = [&](const unsigned char* order, const int ntypes, auto load, auto sums) AG_INLINE -> bool {
+    for (int pos = 0; pos < ntypes; pos++) {
+      const int t = order[pos];
+      for (int cg = 0; cg < S.box.ncells; cg += kCellGroup) {
+        const int ncg = cell_prefix<PART>(P, S, t, cg);
         const int total = S.cellPre[ncg];
         for (int v0 = 0; v0 < total; v0 += kT) {
           if (nb + min(kT, total - v0) > kCap) {  // this round keeps at most that many atoms
-            scan_donors(P, S, nb, best, bi, q);
+            if (!process_batch<PART>(P, S, ntypes, nb, tb, load, sums)) return false;
             nb = 0;
           }
-          nb = gather_chunk(P, S, B, t, ncg, total, v0, nb, false);
+          nb = gather_chunk<PART>(P, S, pos, ncg, total, v0, nb, nullptr);
         }
       }
     }
-    scan_donors(P, S, nb, best, bi, q);
-    nb = 0;
-    for (int t = tid; t < kMaxTypes; t += kT) S.typeCount[t] = 0;
+    return nb == 0 || process_batch<PART>(P, S, ntypes, nb, tb, load, sums);
+  };
+
+  if constexpr (PART == PART_PLAIN) {
+    PlainSums<NMAX> s;
 #pragma unroll
     for (int p = 0; p < 2; p++) {
-      q.ch[p] = (best[p] <= 64.0) ? bi[p] : -1;
-      S.rch[tid][p] = q.ch[p] >= 0 ? make_float4(P.rv[3 * q.ch[p]], P.rv[3 * q.ch[p] + 1], P.rv[3 * q.ch[p] + 2], 0.f)
-                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+      s.s1[p] = 0.f;
+      s.s2[p] = 0.f;
+#pragma unroll
+      for (int g = 0; g < NMAX / 2; g++) s.em[p][g] = make_float2(0.f, 0.f);
     }
     __syncthreads();
-  }
-
-  // ---- map sums: batches of candidates in type-major order, walked type by type ----
-  unsigned phase = 0;
-  for (int t = 0; t < P.ntypes; t++)
-    for (int cg = 0; cg < B.ncells; cg += kCellGroup) {
-      const int ncg = cell_prefix(P, S, B, t, cg);
-      const int total = S.cellPre[ncg];
-      for (int v0 = 0; v0 < total; v0 += kT) {
-        if (nb + min(kT, total - v0) > kCap) {  // this round keeps at most that many atoms
-          if (!process_batch(P, S, tab, B, nb, phase, q)) return;
-          nb = 0;
-        }
-        nb = gather_chunk(P, S, B, t, ncg, total, v0, nb, true);
+    // The types come in two groups: first those whose equal columns are summed
+    // once per class, then those that need every map's own column.
+    bool classes = P.nClassTypes > 0;  // the sums are still per class
+    const bool ok = walk(
+        P.plainOrder, P.ntypes,
+        [&](int pos) AG_INLINE {
+          const int t = P.plainOrder[pos], pad = 4 * row_stride((pos < P.nClassTypes ? P.ncPad : P.nmPad) >> 2);
+          const float* src = (pos < P.nClassTypes ? P.classTable : P.table) + (size_t)t * kAffRows * pad;
+          const unsigned bytes = (unsigned)(kAffRows * pad * sizeof(float));
+          mbar_arrive_expect_tx(tb.bar, bytes);
+          tma_load_1d(tab, src, bytes, tb.bar);
+          for (int i = 0; i < pad; i += 4)  // the zero row, read after the barrier that follows
+            reinterpret_cast<float4*>(tab + kAffRows * pad + i)[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+        },
+        [&](int pos, int j0, int j1, const unsigned short* wl) AG_INLINE {
+          if (classes && pos >= P.nClassTypes) {
+            expand_classes(P, s);
+            classes = false;
+          }
+          const int rowQ = (classes ? P.ncPad : P.nmPad) >> 2;
+          if (P.plainOrder[pos] == P.hydrogen) plain_sums<NMAX, true>(P, S, tab, rowQ, j0, j1, wl, q, s);
+          else plain_sums<NMAX, false>(P, S, tab, rowQ, j0, j1, wl, q, s);
+        });
+    if (!ok) return false;
+    if (classes) expand_classes(P, s);
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+      if (!q.valid[p]) continue;
+      const int64_t pt = ((int64_t)(q.iz0 + p) * P.ny + q.iy) * P.nx + q.ix;
+#pragma unroll
+      for (int g = 0; g < NMAX; g++) {
+        if (g >= P.nmaps) break;
+        if (P.mapCov[g]) continue;
+        float* o = P.out + (int64_t)g * P.npoints + pt;
+        const float e = ((g & 1) ? s.em[p][g >> 1].y : s.em[p][g >> 1].x) +
+                        (P.solparProbe[g] * s.s1[p] + P.volProbe[g] * s.s2[p]);
+        if ((P.slotMaps >> g) & 1u) atomicAdd(o, e);
+        else *o = e;
       }
+      P.dmap[pt] = P.solparQ * s.s1[p];
     }
-  if (nb > 0 && !process_batch(P, S, tab, B, nb, phase, q)) return;
-
-  // ---- results ----
+  } else {
+    SlotSums s;
 #pragma unroll
-  for (int p = 0; p < 2; p++) {
-    if (!q.valid[p]) continue;
-    const int64_t pt = ((int64_t)(q.iz0 + p) * P.ny + q.iy) * P.nx + q.ix;
-#pragma unroll
-    for (int g = 0; g < NMAX; g++) {
-      if (g >= P.nmaps) break;
-      if (P.mapCov[g]) continue;
-      float e = ((g & 1) ? q.em[p][g >> 1].y : q.em[p][g >> 1].x) +
-                (P.solparProbe[g] * q.s1[p] + P.volProbe[g] * q.s2[p]);
+    for (int p = 0; p < 2; p++) {
+      s.fl[p] = 0u;
+      s.ch[p] = -1;
 #pragma unroll
       for (int k = 0; k < kA2Slots; k++) {
-        if (k < P.nslots && P.slotMap[k] == g) {
-          if (P.slotKind[k] == A2_SLOT_ACC) e += q.mn[p][k];
-          else if ((q.fl[p] >> k) & 1u) e += q.mn[p][k] + q.mx[p][k];
+        s.mn[p][k] = (P.slotKind[k] == A2_SLOT_ACC) ? 0.f : 999999.f;
+        s.mx[p][k] = -999999.f;
+      }
+    }
+    __syncthreads();
+    // The nearest H donor of both points, from the donors within 8 A of the box.
+    if (P.needClosestH) {
+      double4* d64 = reinterpret_cast<double4*>(tab);
+      double best[2] = {1e300, 1e300};
+      int bi[2] = {-1, -1};
+      for (int t = 0; t < P.ntypes; t++) {
+        if (!P.typeDonor[t]) continue;
+        for (int cg = 0; cg < S.box.ncells; cg += kCellGroup) {
+          const int ncg = cell_prefix<PART>(P, S, t, cg);
+          const int total = S.cellPre[ncg];
+          for (int v0 = 0; v0 < total; v0 += kT) {
+            if (nb + min(kT, total - v0) > kCap) {
+              scan_donors(P, S, d64, nb, best, bi, q);
+              nb = 0;
+            }
+            nb = gather_chunk<PART>(P, S, 0, ncg, total, v0, nb, d64);
+          }
         }
       }
-      P.out[(int64_t)g * P.npoints + pt] = e;
+      scan_donors(P, S, d64, nb, best, bi, q);
+      nb = 0;
+      for (int t = tid; t < kMaxTypes; t += kT) S.typeCount[t] = 0;
+#pragma unroll
+      for (int p = 0; p < 2; p++) {
+        s.ch[p] = (best[p] <= 64.0) ? bi[p] : -1;
+        S.rch[tid][p] = s.ch[p] >= 0 ? __ldg(P.rv8 + 2 * (size_t)s.ch[p]) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      __syncthreads();
     }
-    P.dmap[pt] = P.solparQ * q.s1[p];
+    const bool ok = walk(
+        P.slotOrder, P.nSlotTypes,
+        [&](int pos) AG_INLINE {
+          const unsigned bytes = (unsigned)(P.nslots * kPlaneRows * sizeof(float));
+          mbar_arrive_expect_tx(tb.bar, bytes);
+          tma_load_1d(tab, P.slotTable + (size_t)P.slotOrder[pos] * kA2Slots * kPlaneRows, bytes, tb.bar);
+        },
+        [&](int pos, int j0, int j1, const unsigned short* wl) AG_INLINE {
+          const int t = P.slotOrder[pos];
+          const unsigned slots = P.typeSlots[t];
+          const bool ish = t == P.hydrogen;
+          switch (P.typeAng[t]) {  // uniform
+            case A2_D1:
+              if (ish) slot_terms<A2_D1, true>(P, S, tab, j0, j1, wl, slots, q, s);
+              else slot_terms<A2_D1, false>(P, S, tab, j0, j1, wl, slots, q, s);
+              break;
+            case A2_A1: slot_terms<A2_A1, false>(P, S, tab, j0, j1, wl, slots, q, s); break;
+            case A2_A2: slot_terms<A2_A2, false>(P, S, tab, j0, j1, wl, slots, q, s); break;
+            default:
+              if (ish) slot_terms<A2_SPH, true>(P, S, tab, j0, j1, wl, slots, q, s);
+              else slot_terms<A2_SPH, false>(P, S, tab, j0, j1, wl, slots, q, s);
+              break;
+          }
+        });
+    if (!ok) return false;
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+      if (!q.valid[p]) continue;
+      const int64_t pt = ((int64_t)(q.iz0 + p) * P.ny + q.iy) * P.nx + q.ix;
+#pragma unroll
+      for (int k = 0; k < kA2Slots; k++) {
+        if (k >= P.nslots || !((P.slotMaps >> P.slotMap[k]) & 1u)) continue;
+        float v = 0.f;
+        if (P.slotKind[k] == A2_SLOT_ACC) v = s.mn[p][k];
+        else if ((s.fl[p] >> k) & 1u) v = s.mn[p][k] + s.mx[p][k];
+        atomicAdd(P.out + (int64_t)P.slotMap[k] * P.npoints + pt, v);
+      }
+    }
   }
+  return true;
 }
 
+// CTAs per SM: three (80 registers, 76 KB of shared memory), so that the plain
+// parts' table reads, which fill the shared-memory pipe, overlap the slot
+// parts' arithmetic; rows of 16 columns (51 KB tables) leave room for two.
 template <int NMAX>
-__global__ void __launch_bounds__(kT, 2) affinity2_kernel(const __grid_constant__ Aff2Params P) {
+constexpr int aff2_ctas_per_sm() {
+  return NMAX <= 12 ? 3 : 2;
+}
+
+// A block's parts are neighbouring CTAs, so that both kinds share every SM.
+template <int NMAX>
+__global__ void __launch_bounds__(kT, aff2_ctas_per_sm<NMAX>()) affinity2_kernel(const __grid_constant__ Aff2Params P) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  aff2_unit<NMAX>(P, P.ctaBase + blockIdx.x, smem_raw);
+  __shared__ uint64_t s_bar;
+  TableBar tb;
+  tb.init(&s_bar);
+  if (P.slotMaps == 0u)
+    aff2_unit<NMAX, PART_PLAIN>(P, P.ctaBase + blockIdx.x, smem_raw, tb);
+  else if (blockIdx.x & 1)
+    aff2_unit<NMAX, PART_PLAIN>(P, P.ctaBase + (blockIdx.x >> 1), smem_raw, tb);
+  else
+    aff2_unit<NMAX, PART_SLOTS>(P, P.ctaBase + (blockIdx.x >> 1), smem_raw, tb);
 }
 
 // Persistent kernel over the work units (job, CTA block) of a batch of
-// receptors, taken from an atomic counter in the host's (decreasing cost) order.
+// receptors, taken part by part from an atomic counter in the host's
+// (decreasing cost) order.
 template <int NMAX>
-__global__ void __launch_bounds__(kT, 2)
+__global__ void __launch_bounds__(kT, aff2_ctas_per_sm<NMAX>())
     affinity2_batch_kernel(const Aff2Params* __restrict__ jobs, const int2* __restrict__ units, int nunits,
                            int* counter) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int s_unit;
+  __shared__ uint64_t s_bar;
+  TableBar tb;
+  tb.init(&s_bar);
   for (;;) {
     __syncthreads();  // the previous unit is finished by every thread
     if (threadIdx.x == 0) s_unit = atomicAdd(counter, 1);
     __syncthreads();
     const int u = s_unit;
-    if (u >= nunits) return;
-    const int2 w = units[u];
-    aff2_unit<NMAX>(jobs[w.x], w.y, smem_raw);
+    if (u >= 2 * nunits) return;
+    const int2 w = units[u >> 1];
+    bool ok = true;
+    if (u & 1) {
+      ok = aff2_unit<NMAX, PART_PLAIN>(jobs[w.x], w.y, smem_raw, tb);
+    } else if (jobs[w.x].slotMaps != 0u) {
+      ok = aff2_unit<NMAX, PART_SLOTS>(jobs[w.x], w.y, smem_raw, tb);
+    }
+    if (!ok) return;  // uniform
   }
 }
 
+// Zero the values [off, off + cnt) of a pass's slot maps (blockIdx.y: slot).
+__device__ __forceinline__ void zero_slot(const Aff2Params& P, int64_t off, int64_t cnt) {
+  const int k = blockIdx.y;
+  if (k >= P.nslots || !((P.slotMaps >> P.slotMap[k]) & 1u)) return;
+  float* o = P.out + (int64_t)P.slotMap[k] * P.npoints + off;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x)
+    o[i] = 0.f;
+}
+__global__ void aff2_zero_kernel(const __grid_constant__ Aff2Params P, int64_t off, int64_t cnt) {
+  zero_slot(P, off, cnt);
+}
+__global__ void aff2_zero_batch_kernel(const Aff2Params* __restrict__ jobs) {
+  const Aff2Params& P = jobs[blockIdx.z];
+  zero_slot(P, 0, P.npoints);
+}
+
+// The tables of one pass from the pair energies (one thread per type and row):
+// the one-point kernel's rows, the two-point kernel's rows (slot maps' columns
+// zero, the desolvation value last), its class rows and its slot planes.
+__global__ void aff_tables_kernel(const __grid_constant__ AffTableJob J) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= J.ntypes * kAffRows) return;
+  const int t = u / kAffRows, i = u - t * kAffRows;
+  const float* e = J.energy + (size_t)u * J.nmAll + J.m0;
+  const float sol = J.sol[i];
+  for (int g = 0; g < J.pad1; g++) J.rows1[(size_t)u * J.pad1 + g] = g < J.nm ? e[g] : 0.f;
+  const int rowStride = 4 * row_stride(J.nmPad >> 2), classStride = 4 * row_stride(J.ncPad >> 2);
+  for (int g = 0; g < J.nmPad; g++)
+    J.rows[(size_t)u * rowStride + g] =
+        g == J.nmPad - 1 ? sol : (g < J.nm && ((J.typePlain[t] >> g) & 1u)) ? e[g] : 0.f;
+  for (int c = 0; c < J.ncPad; c++) {
+    const int g = (int)(J.classMap >> (4 * c)) & 15;
+    J.classRows[(size_t)u * classStride + c] =
+        c == J.ncPad - 1 ? sol : (c < J.nc && ((J.typePlain[t] >> g) & 1u)) ? e[g] : 0.f;
+  }
+  for (int k = 0; k < J.nslots; k++) J.planes[((size_t)t * kA2Slots + k) * kA2PlaneRows + i] = e[J.slotMap[k]];
+}
+
+cudaError_t aff_tables_launch(const AffTableJob& J, cudaStream_t st) {
+  aff_tables_kernel<<<(J.ntypes * kAffRows + 127) / 128, 128, 0, st>>>(J);
+  return cudaGetLastError();
+}
+
+int aff2_row_stride(int columns) { return 4 * row_stride(columns >> 2); }
+
 int aff2_ctas(int nx, int ny, int nz) { return ((nx + 7) / 8) * ((ny + 7) / 8) * ((nz + 7) / 8); }
 
-cudaError_t aff2_batch_launch(const Aff2Params* jobs, const int2* units, int nunits, int* counter, int nmPadMax,
-                              int nmapsMax, int grid, cudaStream_t st) {
-  const size_t smem = aff2_smem_bytes(nmPadMax);
+cudaError_t aff2_batch_launch(const Aff2Params* jobs, int njobs, const int2* units, int nunits, int* counter,
+                              int nmPadMax, bool anySlots, int sms, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
+  if (anySlots) aff2_zero_batch_kernel<<<dim3(16, kA2Slots, njobs), 256, 0, st>>>(jobs);
+  const size_t smem = aff2_smem(nmPadMax, anySlots);
 #define AG_AFF2B(N)                                                                                               \
   do {                                                                                                            \
     e = cudaFuncSetAttribute(affinity2_batch_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     if (e != cudaSuccess) return e;                                                                               \
-    affinity2_batch_kernel<N><<<grid, kT, smem, st>>>(jobs, units, nunits, counter);                              \
+    affinity2_batch_kernel<N><<<sms * aff2_ctas_per_sm<N>(), kT, smem, st>>>(jobs, units, nunits, counter);       \
   } while (0)
-  if (nmapsMax <= 4) AG_AFF2B(4);
-  else if (nmapsMax <= 8) AG_AFF2B(8);
-  else if (nmapsMax <= 12) AG_AFF2B(12);
+  if (nmPadMax <= 4) AG_AFF2B(4);
+  else if (nmPadMax <= 8) AG_AFF2B(8);
+  else if (nmPadMax <= 12) AG_AFF2B(12);
   else AG_AFF2B(16);
 #undef AG_AFF2B
   return cudaGetLastError();
 }
 
 cudaError_t aff2_launch_range(const Aff2Params& P0, int b0, int b1, cudaStream_t st) {
-  const int nb = ((P0.nx + 7) / 8) * ((P0.ny + 7) / 8) * ((P0.nz + 7) / 8);
+  const int tbxy = ((P0.nx + 7) / 8) * ((P0.ny + 7) / 8), nb = aff2_ctas(P0.nx, P0.ny, P0.nz);
   b0 = max(0, b0);
   b1 = min(nb, b1);
   if (b1 <= b0) return cudaSuccess;
   Aff2Params P = P0;
   P.ctaBase = b0;
-  const size_t smem = aff2_smem_bytes(P.nmPad);
-  const int grid = b1 - b0;
+  const bool slots = P.slotMaps != 0u;
+  if (slots) {  // the z slabs that hold the range (a range is whole slabs)
+    const int64_t plane = (int64_t)P.nx * P.ny;
+    const int64_t z0 = 8LL * (b0 / tbxy), z1 = std::min<int64_t>(P.nz, 8LL * ((b1 + tbxy - 1) / tbxy));
+    aff2_zero_kernel<<<dim3(74, kA2Slots), 256, 0, st>>>(P, z0 * plane, (z1 - z0) * plane);
+  }
+  const int grid = (b1 - b0) * (slots ? 2 : 1);
+  const size_t smem = aff2_smem(P.nmPad, slots);
   cudaError_t e;
 #define AG_AFF2(N)                                                                                           \
   do {                                                                                                       \
@@ -751,9 +982,9 @@ cudaError_t aff2_launch_range(const Aff2Params& P0, int b0, int b1, cudaStream_t
     if (e != cudaSuccess) return e;                                                                          \
     affinity2_kernel<N><<<grid, kT, smem, st>>>(P);                                                          \
   } while (0)
-  if (P.nmaps <= 4) AG_AFF2(4);
-  else if (P.nmaps <= 8) AG_AFF2(8);
-  else if (P.nmaps <= 12) AG_AFF2(12);
+  if (P.nmPad <= 4) AG_AFF2(4);
+  else if (P.nmPad <= 8) AG_AFF2(8);
+  else if (P.nmPad <= 12) AG_AFF2(12);
   else AG_AFF2(16);
 #undef AG_AFF2
   return cudaGetLastError();

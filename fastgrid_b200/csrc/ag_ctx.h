@@ -81,11 +81,19 @@ struct ag_ctx {
   agc::DevBuf<int> info, cellStart, cellAtoms, cellOf, count, fill, dStart, dAtoms, donorMask, closestH;
   agc::DevBuf<int> ctStart, ctAtoms;  // type-major cell list ((cell, type) segments) of the two-point kernel
   int affKernel = 2;                  // affinity kernel: 2 two-point (default), 1 one point per thread
-  agc::DevBuf<float> vol, solq, affTab, affTabH, sol, rv32, rv2_32;
+  agc::DevBuf<float> vol, solq, affTab, affRaw, sol;
+  agc::DevBuf<float4> rv8;            // per atom: rvector, 0, rvector2, 0
   agc::DevBuf<double> rv64, thrA;
   struct Pass {
     int m0, nm, nmPad;
-    size_t tabOff, tabHOff;
+    size_t tabOff, rowsOff, classOff, slotOff;  // in affTab: one-point rows; two-point rows, class rows, slot planes
+    // Two-point kernel (planPass).
+    int rowPad, nc, ncPad;
+    unsigned long long classMap, classOf;
+    unsigned classTypes;              // bit t: type t is summed in class rows
+    int nslots;                       // H-bond slots, -1: too many
+    int slotMap[agk::kA2Slots], slotKind[agk::kA2Slots];
+    unsigned typeSlots[agk::kMaxTypes], typePlain[agk::kMaxTypes];
     unsigned typeModes[agk::kMaxTypes];
     int typeNeedsAngular[agk::kMaxTypes];
     int mapMinMaxSlot[agk::kMaxMapsPass];

@@ -94,8 +94,7 @@ struct AffParams {
   const int* info;                // type | hbond << 5 | disorder << 8 | rexp << 9
   const float* vol;
   const float* solq;              // solpar + solparQ * |q|
-  const float* rv;                // rvector, 3 per atom (FP32)
-  const float* rv2;               // rvector2, 3 per atom (FP32)
+  const float4* rv8;              // per atom: rvector, 0, rvector2, 0 (FP32)
   const double* rv64;             // rvector, 3 per atom (FP64, for exact sign decisions)
   // cell list (8 A cells)
   const int* cellStart;           // ncell + 1
@@ -154,6 +153,7 @@ cudaError_t cells_launch(const CellBuild& C, int ncellTotal, cudaStream_t st);
 // Affinity + desolvation, two grid points per thread (affinity2.cu)
 // ---------------------------------------------------------------------------
 constexpr int kA2Slots = 4;         // H-bond maps per pass handled by the two-point kernel
+constexpr int kA2PlaneRows = 804;   // rows of a slot's table plane (kAffRows, padded to 16 bytes)
 enum { A2_SPH = 0, A2_D1 = 1, A2_A1 = 2, A2_A2 = 3 };          // angular class of a receptor type
 enum { A2_SLOT_ACC = 0, A2_SLOT_A1 = 1, A2_SLOT_DON = 2 };     // H-bond map kind (probe class)
 
@@ -163,8 +163,7 @@ struct Aff2Params {
   const int* info;                // type | hbond << 5 | disorder << 8 | rexp << 9
   const float* vol;
   const float* solq;
-  const float* rv;                // rvector (FP32, 3 per atom)
-  const float* rv2;               // rvector2 (FP32, 3 per atom)
+  const float4* rv8;              // per atom: rvector, 0, rvector2, 0 (FP32)
   const double* rv64;             // rvector (FP64) for exact sign decisions
   // type-major cell list: segment (cell, type) = atoms ctAtoms[ctStart[cell*ntypes+t] .. ctStart[...+1])
   const int* ctStart;
@@ -177,20 +176,30 @@ struct Aff2Params {
   double h;
   // maps of this pass
   int nmaps, nmPad, ntypes, hydrogen;
-  const float* table;             // [ntypes][kAffRows][nmPad] FP32
-  const float* tableH;            // [kAffRows][nmPad] rows of the "HD" type, or null
-  const float* sol;               // kAffRows
-  int solInRow;                   // the table rows' last column (nmPad - 1 >= nmaps) holds sol
+  // Rows [ntypes][kAffRows][aff2_row_stride(nmPad)] FP32: the maps' pair energies (0 where the
+  // map is an H-bond slot for the type), the desolvation value in the last
+  // column.  The first nClassTypes types of plainOrder take class rows
+  // (ncPad columns, strided likewise) instead: maps whose columns are equal for all of
+  // those types share a column (map g has column 4 bits of classOf from 4 g).
+  const float* table;
+  const float* classTable;
+  int nClassTypes, ncPad;
+  unsigned long long classOf;
+  unsigned char plainOrder[kMaxTypes];
+  int nSlotTypes;                 // types with H-bond slots, and their list
+  unsigned char slotOrder[kMaxTypes];
   const double* thr;              // affinity bin thresholds (kAffRows + 1)
   float delta;                    // guard half-width around bin edges (bins)
   int needClosestH;               // some D1 type meets an acceptor-probe slot: find the nearest donor
   int typeAng[kMaxTypes];         // A2_SPH / A2_D1 / A2_A1 / A2_A2
   int typeDonor[kMaxTypes];       // DS or D1 (candidates of the nearest-donor search)
   unsigned typeSlots[kMaxTypes];  // bit k: H-bond slot k applies to this type
-  unsigned typePlain[kMaxTypes];  // bit g: map g takes the plain table sum for this type
   int nslots;
   int slotMap[kA2Slots];          // map index of each H-bond slot
   int slotKind[kA2Slots];         // A2_SLOT_*
+  unsigned slotMaps;              // bit g: map g has an H-bond slot that applies to some type
+  const float* slotTable;         // [ntypes][kA2Slots][kA2PlaneRows] the slots' columns, a plane each
+  const float* planeH;            // the "HD" type's planes, or null
   int mapCov[kMaxMapsPass];
   float solparProbe[kMaxMapsPass], volProbe[kMaxMapsPass];
   float solparQ;
@@ -199,15 +208,29 @@ struct Aff2Params {
   unsigned* status;
   int ctaBase;                    // first CTA block of a launch (0, or a z-slab chunk's first block)
 };
-size_t aff2_smem_bytes(int nmPad);
 cudaError_t aff2_launch(const Aff2Params& P, cudaStream_t st);
 // Blocks [b0, b1) of the pass (the grid's CTA blocks run z-slab by z-slab).
 cudaError_t aff2_launch_range(const Aff2Params& P, int b0, int b1, cudaStream_t st);
+// Floats from one table row of `columns` (a multiple of 4) to the next.
+int aff2_row_stride(int columns);
 // CTA blocks (work units) of the two-point kernel on an nx x ny x nz grid.
 int aff2_ctas(int nx, int ny, int nz);
 // Persistent two-point pass over the units (job, CTA block) of many jobs.
-cudaError_t aff2_batch_launch(const Aff2Params* jobs, const int2* units, int nunits, int* counter, int nmPadMax,
-                              int nmapsMax, int grid, cudaStream_t st);
+cudaError_t aff2_batch_launch(const Aff2Params* jobs, int njobs, const int2* units, int nunits, int* counter,
+                              int nmPadMax, bool anySlots, int sms, cudaStream_t st);
+
+// Build a pass's tables on the device from the staged pair energies.
+struct AffTableJob {
+  const float* energy;            // [ntypes][kAffRows][nmAll]
+  const float* sol;               // kAffRows
+  int ntypes, nmAll, m0, nm;      // the pass: maps m0 .. m0 + nm
+  int pad1, nmPad, ncPad, nc, nslots;
+  unsigned long long classMap;    // 4 bits per class: a map of it
+  int slotMap[kA2Slots];
+  unsigned typePlain[kMaxTypes];  // bit g: map g takes the plain table sum for this type
+  float *rows1, *rows, *classRows, *planes;
+};
+cudaError_t aff_tables_launch(const AffTableJob& J, cudaStream_t st);
 
 struct ClosestHParams {
   const double4* xyz;

@@ -145,8 +145,9 @@ extern "C" int ag_ctx_destroy(ag_ctx* c) {
   if (!c) return AG_OK;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
-  for (auto* b : {&c->epsTab, &c->maps, &c->vol, &c->solq, &c->affTab, &c->affTabH, &c->sol, &c->rv32, &c->rv2_32})
+  for (auto* b : {&c->epsTab, &c->maps, &c->vol, &c->solq, &c->affTab, &c->affRaw, &c->sol})
     b->release();
+  c->rv8.release();
   c->atoms.release();
   c->thr.release();
   c->partial.release();
@@ -643,6 +644,115 @@ int runEmap(ag_ctx* c, float* dOut) {
   return AG_OK;
 }
 
+// Kind of H-bond slot map m takes in the two-point kernel, or -1: the H-bond
+// maps whose term differs from a plain table sum for some receptor type
+// (CalculateGridmaps.cpp:206-228).
+int slotKindOf(const ag_ctx* c, int m) {
+  const int mhb = c->mapHbond[m];
+  if (!c->mapIsHB[m] || c->mapCov[m]) return -1;
+  if (mhb == ag::AS || mhb == ag::A2) return agk::A2_SLOT_ACC;
+  if (mhb == ag::A1) return agk::A2_SLOT_A1;
+  if (mhb == ag::DS || mhb == ag::D1) return agk::A2_SLOT_DON;
+  return -1;
+}
+
+// H-bond slots of a pass for the two-point kernel.  Returns false if the pass
+// has more than kA2Slots of them (the one-point kernel then computes it).
+bool passSlots(const ag_ctx* c, const ag_ctx::Pass& ps, int& nslots, int slotMap[agk::kA2Slots],
+               int slotKind[agk::kA2Slots]) {
+  nslots = 0;
+  for (int g = 0; g < ps.nm; g++) {
+    const int kind = slotKindOf(c, ps.m0 + g);
+    if (kind < 0) continue;
+    if (nslots == agk::kA2Slots) return false;
+    slotMap[nslots] = g;
+    slotKind[nslots] = kind;
+    nslots++;
+  }
+  return true;
+}
+
+// The two-point kernel's plan of a pass: its H-bond slots and the types they
+// apply to, and which maps can share a column.  Two maps share one if their
+// pair energies agree, row by row in FP32, for every type of a group (NA and N,
+// SA and S, A and C differ only in H-bonding or desolvation), slot maps
+// counting as zero; the group is all types or, where more maps agree then, all
+// but the donors, whose acceptor-probe maps are slots.  Fewer columns mean
+// fewer 16-byte reads of shared memory per pair, the plain sums' bound.
+void planPass(const ag_ctx* c, ag_ctx::Pass& ps, const float* raw) {
+  const int nt = c->nTypes, nmAll = c->nMaps, nm = ps.nm;
+  ps.rowPad = (nm + 1 + 3) / 4 * 4;
+  ps.ncPad = 0;
+  ps.nc = 0;
+  ps.classMap = ps.classOf = 0;
+  ps.classTypes = 0;
+  for (int t = 0; t < agk::kMaxTypes; t++) {
+    ps.typeSlots[t] = 0;
+    ps.typePlain[t] = (1u << nm) - 1u;
+  }
+  if (!passSlots(c, ps, ps.nslots, ps.slotMap, ps.slotKind)) {
+    ps.nslots = -1;  // the one-point kernel
+    return;
+  }
+  unsigned donors = 0;
+  for (int t = 0; t < nt; t++) {
+    const int ahb = c->typeHbond[t];
+    const bool donor = ahb == ag::DS || ahb == ag::D1, acceptor = ahb >= ag::AS;
+    if (donor) donors |= 1u << t;
+    for (int k = 0; k < ps.nslots; k++)
+      if (ps.slotKind[k] == agk::A2_SLOT_DON ? acceptor : donor) {
+        ps.typeSlots[t] |= 1u << k;
+        ps.typePlain[t] &= ~(1u << ps.slotMap[k]);
+      }
+  }
+  // same[t]: per map, the first map with the same column for type t.
+  int same[agk::kMaxTypes][agk::kMaxMapsPass];
+  for (int t = 0; t < nt; t++)
+    for (int g = 0; g < nm; g++) {
+      same[t][g] = g;
+      const bool plain = (ps.typePlain[t] >> g) & 1u;
+      for (int f = 0; f < g && same[t][g] == g; f++) {
+        if (same[t][f] != f || plain != (bool)((ps.typePlain[t] >> f) & 1u)) continue;
+        bool eq = true;
+        const float* col = raw + (size_t)t * agk::kAffRows * nmAll + ps.m0;
+        // From the wells outwards first: clamped rows are equal for most pairs.
+        for (int i = 0; plain && eq && i < agk::kAffRows; i++) {
+          const int row = (i + 350) % agk::kAffRows;
+          eq = memcmp(col + (size_t)row * nmAll + f, col + (size_t)row * nmAll + g, sizeof(float)) == 0;
+        }
+        if (eq) same[t][g] = f;
+      }
+    }
+  const unsigned all = nt == 32 ? ~0u : (1u << nt) - 1u;
+  ps.ncPad = ps.rowPad;
+  for (unsigned group : {all, all & ~donors}) {
+    if (!group) continue;
+    int of[agk::kMaxMapsPass], rep[agk::kMaxMapsPass], nc = 0;
+    for (int g = 0; g < nm; g++) {
+      of[g] = -1;
+      for (int k = 0; k < nc && of[g] < 0; k++) {
+        bool eq = true;
+        for (int t = 0; t < nt && eq; t++)
+          if ((group >> t) & 1u) eq = same[t][g] == same[t][rep[k]];
+        if (eq) of[g] = k;
+      }
+      if (of[g] < 0) {
+        rep[nc] = g;
+        of[g] = nc++;
+      }
+    }
+    const int pad = (nc + 1 + 3) / 4 * 4;
+    if (pad >= ps.ncPad) continue;
+    ps.ncPad = pad;
+    ps.nc = nc;
+    ps.classTypes = group;
+    ps.classMap = ps.classOf = 0;
+    for (int k = 0; k < nc; k++) ps.classMap |= (unsigned long long)rep[k] << (4 * k);
+    for (int g = 0; g < nm; g++) ps.classOf |= (unsigned long long)of[g] << (4 * g);
+  }
+  if (!ps.classTypes) ps.ncPad = 0;
+}
+
 int stageAffinity(ag_ctx* c, const ag_receptor* r, const ag_affinity_params* p) {
   const int n = r->n_atoms;
   if (p->n_maps < 0 || p->n_maps > ag::kMaxAtomTypes) return fail(AG_E_INVALID, "n_maps %d outside 0..14", p->n_maps);
@@ -666,17 +776,20 @@ int stageAffinity(ag_ctx* c, const ag_receptor* r, const ag_affinity_params* p) 
       return fail(AG_E_INVALID, "atoms of receptor type %d have different H-bond classes", r->type[i]);
   }
   for (int t = 0; t < agk::kMaxTypes; t++) if (c->typeHbond[t] < 0) c->typeHbond[t] = ag::NON;
-  std::vector<float> rv32(3 * (size_t)n), rv2_32(3 * (size_t)n);
-  for (size_t i = 0; i < 3 * (size_t)n; i++) { rv32[i] = (float)r->rvector[i]; rv2_32[i] = (float)r->rvector2[i]; }
+  std::vector<float4> rv8(2 * (size_t)n);
+  for (size_t i = 0; i < (size_t)n; i++) {
+    const double *a = r->rvector + 3 * i, *b = r->rvector2 + 3 * i;
+    rv8[2 * i] = make_float4((float)a[0], (float)a[1], (float)a[2], 0.f);
+    rv8[2 * i + 1] = make_float4((float)b[0], (float)b[1], (float)b[2], 0.f);
+  }
   CK(c->info.ensure(n)); CK(c->donorMask.ensure(n)); CK(c->vol.ensure(n)); CK(c->solq.ensure(n));
-  CK(c->rv32.ensure(3 * (size_t)n)); CK(c->rv2_32.ensure(3 * (size_t)n)); CK(c->rv64.ensure(3 * (size_t)n));
+  CK(c->rv8.ensure(2 * (size_t)n)); CK(c->rv64.ensure(3 * (size_t)n));
   if (n) {
     CK(cudaMemcpyAsync(c->info.p, info.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->donorMask.p, donor.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->vol.p, vol.data(), sizeof(float) * n, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->solq.p, solq.data(), sizeof(float) * n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->rv32.p, rv32.data(), sizeof(float) * 3 * n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->rv2_32.p, rv2_32.data(), sizeof(float) * 3 * n, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->rv8.p, rv8.data(), sizeof(float4) * 2 * n, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->rv64.p, r->rvector, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
   }
   c->nMaps = p->n_maps;
@@ -689,19 +802,21 @@ int stageAffinity(ag_ctx* c, const ag_receptor* r, const ag_affinity_params* p) 
   c->solparProbe.assign(p->solpar_probe, p->solpar_probe + p->n_maps);
   c->volProbe.assign(p->vol_probe, p->vol_probe + p->n_maps);
 
-  // Split the maps into passes of at most 16 maps and 4 min/max maps.
+  // Split the maps into passes of at most 16 maps and 4 H-bonding ones (the
+  // two-point kernel's slots), or 4 min/max maps for the one-point kernel.
   const int nm = p->n_maps, nt = p->n_types;
   auto isMinMax = [&](int m) {
     const int hb = c->mapHbond[m];
     return c->mapIsHB[m] && !c->mapCov[m] && (hb == ag::A1 || hb == ag::DS || hb == ag::D1);
   };
+  auto counted = [&](int m) { return c->affKernel == 2 ? slotKindOf(c, m) >= 0 : isMinMax(m); };
   c->passes.clear();
   for (int m0 = 0; m0 < nm;) {
     ag_ctx::Pass ps{};
     ps.m0 = m0;
-    int mm = 0, k = 0;
+    int mm = 0, hb = 0, k = 0;
     while (m0 + k < nm && k < agk::kMaxMapsPass) {
-      if (isMinMax(m0 + k) && mm == agk::kMaxMinMax) break;
+      if (counted(m0 + k) && hb++ == agk::kMaxMinMax) break;
       ps.mapMinMaxSlot[k] = isMinMax(m0 + k) ? mm++ : -1;
       k++;
     }
@@ -727,28 +842,28 @@ int stageAffinity(ag_ctx* c, const ag_receptor* r, const ag_affinity_params* p) 
     c->passes.push_back(ps);
     m0 += k;
   }
-  // Pair-energy tables, FP32, rows r <= 8 A, per pass [type][row][nmPad].
-  size_t tabSize = 0, tabHSize = 0;
-  for (auto& ps : c->passes) {
-    ps.tabOff = tabSize;
-    ps.tabHOff = tabHSize;
-    tabSize += (size_t)nt * agk::kAffRows * ps.nmPad;
-    tabHSize += (size_t)agk::kAffRows * ps.nmPad;
+  if (c->passes.empty()) {  // no ligand maps: one pass for the d-map alone
+    ag_ctx::Pass ps{};
+    ps.nmPad = 4;
+    for (int k = 0; k < agk::kMaxMapsPass; k++) ps.mapMinMaxSlot[k] = -1;
+    c->passes.push_back(ps);
   }
-  std::vector<float> tab(std::max<size_t>(tabSize, 4), 0.f), tabH(std::max<size_t>(tabHSize, 4), 0.f);
+  // Pair energies, FP32, rows r <= 8 A: [type][row][map].  The kernels' tables
+  // are built from them on the device (aff_tables_kernel).
+  std::vector<float> raw(std::max<size_t>((size_t)nt * agk::kAffRows * nm, 4));
+  for (int t = 0; t < nt; t++) {
+    const double* src = p->energy + (size_t)t * 8192 * nm;
+    float* dst = raw.data() + (size_t)t * agk::kAffRows * nm;
+    for (int i = 0; i < agk::kAffRows * nm; i++) dst[i] = (float)src[i];
+  }
+  size_t tabSize = 0;
   for (auto& ps : c->passes) {
-    for (int t = 0; t < nt; t++)
-      for (int i = 0; i < agk::kAffRows; i++) {
-        for (int g = 0; g < ps.nm; g++)
-          tab[ps.tabOff + ((size_t)t * agk::kAffRows + i) * ps.nmPad + g] =
-              (float)p->energy[((size_t)t * 8192 + i) * nm + ps.m0 + g];
-        // A spare last column carries the desolvation value (read by the two-point kernel).
-        if (ps.nm < ps.nmPad) tab[ps.tabOff + ((size_t)t * agk::kAffRows + i) * ps.nmPad + ps.nmPad - 1] = (float)p->sol[i];
-      }
-    if (p->hydrogen >= 0 && p->hydrogen < nt)
-      for (int i = 0; i < agk::kAffRows; i++)
-        for (int g = 0; g < ps.nm; g++)
-          tabH[ps.tabHOff + (size_t)i * ps.nmPad + g] = (float)p->energy[((size_t)p->hydrogen * 8192 + i) * nm + ps.m0 + g];
+    planPass(c, ps, raw.data());
+    ps.tabOff = tabSize;
+    ps.rowsOff = ps.tabOff + (size_t)nt * agk::kAffRows * ps.nmPad;
+    ps.classOff = ps.rowsOff + (size_t)nt * agk::kAffRows * agk::aff2_row_stride(ps.rowPad);
+    ps.slotOff = ps.classOff + (size_t)nt * agk::kAffRows * agk::aff2_row_stride(ps.ncPad);
+    tabSize = ps.slotOff + (size_t)nt * agk::kA2Slots * agk::kA2PlaneRows;
   }
   if (!c->thrA.p) {
     const auto& thr = affinityBinThresholds();
@@ -757,11 +872,27 @@ int stageAffinity(ag_ctx* c, const ag_receptor* r, const ag_affinity_params* p) 
   }
   std::vector<float> sol(agk::kAffRows);
   for (int i = 0; i < agk::kAffRows; i++) sol[i] = (float)p->sol[i];
-  CK(c->affTab.ensure(tab.size())); CK(c->affTabH.ensure(tabH.size())); CK(c->sol.ensure(sol.size()));
-  CK(cudaMemcpyAsync(c->affTab.p, tab.data(), sizeof(float) * tab.size(), cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(c->affTabH.p, tabH.data(), sizeof(float) * tabH.size(), cudaMemcpyHostToDevice, c->stream));
+  CK(c->affTab.ensure(tabSize)); CK(c->affRaw.ensure(raw.size())); CK(c->sol.ensure(sol.size()));
+  CK(cudaMemcpyAsync(c->affRaw.p, raw.data(), sizeof(float) * raw.size(), cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->sol.p, sol.data(), sizeof(float) * sol.size(), cudaMemcpyHostToDevice, c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  for (const auto& ps : c->passes) {
+    agk::AffTableJob J{};
+    J.energy = c->affRaw.p;
+    J.sol = c->sol.p;
+    J.ntypes = nt; J.nmAll = nm; J.m0 = ps.m0; J.nm = ps.nm;
+    J.pad1 = ps.nmPad; J.nmPad = ps.rowPad; J.ncPad = ps.ncPad; J.nc = ps.nc;
+    J.nslots = std::max(0, ps.nslots);
+    J.classMap = ps.classMap;
+    for (int k = 0; k < J.nslots; k++) J.slotMap[k] = ps.slotMap[k];
+    for (int t = 0; t < agk::kMaxTypes; t++) J.typePlain[t] = ps.typePlain[t];
+    J.rows1 = c->affTab.p + ps.tabOff;
+    J.rows = c->affTab.p + ps.rowsOff;
+    J.classRows = c->affTab.p + ps.classOff;
+    J.planes = c->affTab.p + ps.slotOff;
+    CK(agk::aff_tables_launch(J, c->stream));
+    c->launches++;
+  }
   c->haveAff = true;
   return AG_OK;
 }
@@ -777,36 +908,11 @@ void cellGrid(const ag_grid& g, double lo[3], int ncell[3]) {
   }
 }
 
-// H-bond slots of a pass for the two-point kernel: the H-bond maps whose term
-// differs from a plain table sum for some receptor type
-// (CalculateGridmaps.cpp:206-228).  Returns false if the pass has more than
-// kA2Slots of them (the one-point kernel then computes it).
-bool passSlots(const ag_ctx* c, const ag_ctx::Pass& ps, int& nslots, int slotMap[agk::kA2Slots],
-               int slotKind[agk::kA2Slots]) {
-  nslots = 0;
-  for (int g = 0; g < ps.nm; g++) {
-    const int m = ps.m0 + g, mhb = c->mapHbond[m];
-    if (!c->mapIsHB[m] || c->mapCov[m]) continue;
-    int kind = -1;
-    if (mhb == ag::AS || mhb == ag::A2) kind = agk::A2_SLOT_ACC;
-    else if (mhb == ag::A1) kind = agk::A2_SLOT_A1;
-    else if (mhb == ag::DS || mhb == ag::D1) kind = agk::A2_SLOT_DON;
-    if (kind < 0) continue;
-    if (nslots == agk::kA2Slots) return false;
-    slotMap[nslots] = g;
-    slotKind[nslots] = kind;
-    nslots++;
-  }
-  return true;
-}
-
 // Whether every affinity pass of the staged job runs on the two-point kernel.
 bool useTwoPoint(const ag_ctx* c) {
   if (c->affKernel != 2) return false;
-  for (const auto& ps : c->passes) {
-    int n, sm[agk::kA2Slots], sk[agk::kA2Slots];
-    if (!passSlots(c, ps, n, sm, sk)) return false;
-  }
+  for (const auto& ps : c->passes)
+    if (ps.nslots < 0) return false;
   return true;
 }
 
@@ -864,48 +970,49 @@ int buildAff2Params(ag_ctx* c, float* dMaps, float* dDmap, std::vector<agk::Aff2
   cellGrid(g, lo, ncell);
   out.clear();
   const int nt = c->nTypes;
-  std::vector<ag_ctx::Pass> passes = c->passes;
-  if (passes.empty()) {  // no ligand maps: one pass for the d-map alone
-    ag_ctx::Pass ps{};
-    ps.nmPad = 4;
-    passes.push_back(ps);
-  }
-  for (const auto& ps : passes) {
+  for (const auto& ps : c->passes) {
     agk::Aff2Params P{};
     P.xyz = c->atoms.p; P.info = c->info.p; P.vol = c->vol.p; P.solq = c->solq.p;
-    P.rv = c->rv32.p; P.rv2 = c->rv2_32.p; P.rv64 = c->rv64.p;
+    P.rv8 = c->rv8.p; P.rv64 = c->rv64.p;
     P.ctStart = c->ctStart.p; P.ctAtoms = c->ctAtoms.p;
     for (int d = 0; d < 3; d++) { P.cellLo[d] = lo[d]; P.ncell[d] = ncell[d]; }
     P.nx = g.nx; P.ny = g.ny; P.nz = g.nz; P.n2x = g.nx / 2; P.n2y = g.ny / 2; P.n2z = g.nz / 2;
     P.npoints = c->npoints(); P.h = g.spacing;
-    P.nmaps = ps.nm; P.nmPad = ps.nmPad; P.ntypes = nt; P.hydrogen = c->hydrogen;
-    P.table = c->affTab.p + ps.tabOff;
-    P.tableH = (c->hydrogen >= 0 && c->hydrogen < nt) ? c->affTabH.p + ps.tabHOff : nullptr;
-    P.sol = c->sol.p;
-    P.solInRow = ps.nm < ps.nmPad ? 1 : 0;
+    P.nmaps = ps.nm; P.nmPad = ps.rowPad; P.ntypes = nt; P.hydrogen = c->hydrogen;
+    P.table = c->affTab.p + ps.rowsOff;
+    P.classTable = c->affTab.p + ps.classOff;
+    P.ncPad = ps.ncPad;
+    P.classOf = ps.classOf;
+    int no = 0;
+    for (int t = 0; t < nt; t++)
+      if ((ps.classTypes >> t) & 1u) P.plainOrder[no++] = (unsigned char)t;
+    P.nClassTypes = no;
+    for (int t = 0; t < nt; t++)
+      if (!((ps.classTypes >> t) & 1u)) P.plainOrder[no++] = (unsigned char)t;
     P.thr = c->thrA.p;
     P.delta = 1.0e-3f;
-    if (!passSlots(c, ps, P.nslots, P.slotMap, P.slotKind)) return fail(AG_E_INVALID, "too many H-bond maps");
-    for (int k = P.nslots; k < agk::kA2Slots; k++) { P.slotMap[k] = -1; P.slotKind[k] = agk::A2_SLOT_ACC; }
+    if (ps.nslots < 0) return fail(AG_E_INVALID, "too many H-bond maps");
+    P.nslots = ps.nslots;
+    for (int k = 0; k < agk::kA2Slots; k++) {
+      P.slotMap[k] = k < ps.nslots ? ps.slotMap[k] : -1;
+      P.slotKind[k] = k < ps.nslots ? ps.slotKind[k] : agk::A2_SLOT_ACC;
+    }
+    P.slotTable = c->affTab.p + ps.slotOff;
+    P.planeH = (c->hydrogen >= 0 && c->hydrogen < nt)
+                   ? P.slotTable + (size_t)c->hydrogen * agk::kA2Slots * agk::kA2PlaneRows : nullptr;
+    P.slotMaps = 0;
     P.needClosestH = 0;
     for (int t = 0; t < agk::kMaxTypes; t++) {
       const int ahb = t < nt ? c->typeHbond[t] : ag::NON;
-      const bool donor = ahb == ag::DS || ahb == ag::D1, acceptor = ahb >= ag::AS;
-      unsigned slots = 0;
-      for (int k = 0; k < P.nslots; k++)
-        if (((P.slotKind[k] == agk::A2_SLOT_ACC || P.slotKind[k] == agk::A2_SLOT_A1) && donor) ||
-            (P.slotKind[k] == agk::A2_SLOT_DON && acceptor))
-          slots |= 1u << k;
-      unsigned plain = 0;
-      for (int gg = 0; gg < ps.nm; gg++) plain |= 1u << gg;
-      for (int k = 0; k < P.nslots; k++)
-        if ((slots >> k) & 1u) plain &= ~(1u << P.slotMap[k]);
-      P.typeSlots[t] = slots;
-      P.typePlain[t] = plain;
-      P.typeDonor[t] = donor ? 1 : 0;
+      P.typeSlots[t] = t < nt ? ps.typeSlots[t] : 0u;
+      P.typeDonor[t] = ahb == ag::DS || ahb == ag::D1 ? 1 : 0;
       P.typeAng[t] = ahb == ag::D1 ? agk::A2_D1 : ahb == ag::A1 ? agk::A2_A1 : ahb == ag::A2 ? agk::A2_A2 : agk::A2_SPH;
+      if (P.typeSlots[t]) P.slotOrder[P.nSlotTypes++] = (unsigned char)t;
       for (int k = 0; k < P.nslots; k++)
-        if (((slots >> k) & 1u) && P.slotKind[k] == agk::A2_SLOT_ACC && ahb == ag::D1) P.needClosestH = 1;
+        if ((P.typeSlots[t] >> k) & 1u) {
+          P.slotMaps |= 1u << P.slotMap[k];
+          if (P.slotKind[k] == agk::A2_SLOT_ACC && ahb == ag::D1) P.needClosestH = 1;
+        }
     }
     for (int k = 0; k < agk::kMaxMapsPass; k++) {
       P.mapCov[k] = k < ps.nm ? c->mapCov[ps.m0 + k] : 1;
@@ -932,17 +1039,10 @@ int buildAffParams(ag_ctx* c, float* dMaps, float* dDmap, std::vector<agk::AffPa
   cellGrid(g, lo, ncell);
   out.clear();
   const int nt = c->nTypes;
-  std::vector<ag_ctx::Pass> passes = c->passes;
-  if (passes.empty()) {  // no ligand maps: one pass for the d-map alone
-    ag_ctx::Pass ps{};
-    ps.nmPad = 4;
-    for (int k = 0; k < agk::kMaxMapsPass; k++) ps.mapMinMaxSlot[k] = -1;
-    passes.push_back(ps);
-  }
-  for (const auto& ps : passes) {
+  for (const auto& ps : c->passes) {
     agk::AffParams P{};
     P.n_atoms = n; P.xyz = c->atoms.p; P.info = c->info.p; P.vol = c->vol.p; P.solq = c->solq.p;
-    P.rv = c->rv32.p; P.rv2 = c->rv2_32.p; P.rv64 = c->rv64.p;
+    P.rv8 = c->rv8.p; P.rv64 = c->rv64.p;
     P.cellStart = c->cellStart.p; P.cellAtoms = c->cellAtoms.p;
     for (int d = 0; d < 3; d++) { P.cellLo[d] = lo[d]; P.ncell[d] = ncell[d]; }
     P.closestH = c->closestH.p;
@@ -950,7 +1050,8 @@ int buildAffParams(ag_ctx* c, float* dMaps, float* dDmap, std::vector<agk::AffPa
     P.npoints = np; P.h = h;
     P.nmaps = ps.nm; P.nmPad = ps.nmPad; P.ntypes = nt; P.hydrogen = c->hydrogen;
     P.table = c->affTab.p + ps.tabOff;
-    P.tableH = (c->hydrogen >= 0 && c->hydrogen < nt) ? c->affTabH.p + ps.tabHOff : nullptr;
+    P.tableH = (c->hydrogen >= 0 && c->hydrogen < nt)
+                   ? P.table + (size_t)c->hydrogen * agk::kAffRows * ps.nmPad : nullptr;
     P.sol = c->sol.p;
     P.thr = c->thrA.p;
     P.delta = 1.0e-3f;
@@ -981,7 +1082,7 @@ int runAffinity(ag_ctx* c, float* dMaps, float* dDmap) {
     if (int e = buildAff2Params(c, dMaps, dDmap, passes)) return e;
     for (const auto& P : passes) {
       CK(agk::aff2_launch(P, c->stream));
-      c->launches += 1;
+      c->launches += P.slotMaps ? 2 : 1;
     }
     return AG_OK;
   }
@@ -1018,7 +1119,7 @@ int runAffinityChunked(ag_ctx* c, float* host, int nchunks) {
     if (s1 <= s0) continue;
     for (const auto& P : passes) {
       CK(agk::aff2_launch_range(P, s0 * tbx * tby, s1 * tbx * tby, c->stream));
-      c->launches += 1;
+      c->launches += P.slotMaps ? 2 : 1;
     }
     CK(cudaEventRecord(c->evChunk[k], c->stream));
     CK(cudaStreamWaitEvent(c->copyStream, c->evChunk[k], 0));
@@ -1385,7 +1486,8 @@ struct ag_batch {
   DevBuf<int> counters;
   DevBuf<double> checks;                 // per job: net-charge checksum of its e-map (FP64 weight sum)
   std::vector<double> hChecks;
-  int ne = 0, na = 0, nmPadMax = 4, nmapsMax = 0;
+  int ne = 0, na = 0, na2 = 0, nmPadMax = 4, nmapsMax = 0;  // na2: two-point jobs
+  bool anySlots = false;                 // some two-point pass has H-bond slots
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   double pairs = 0;
@@ -1421,6 +1523,7 @@ int batchBuild(ag_batch* b) {
   std::vector<std::pair<double, int2>> eu, au;
   b->nmPadMax = 4;
   b->nmapsMax = 0;
+  b->anySlots = false;
   b->pairs = 0;
   CK(b->checks.ensure(b->sub.size()));
   for (size_t i = 0; i < b->sub.size(); i++) {
@@ -1443,6 +1546,7 @@ int batchBuild(ag_batch* b) {
         a2j.push_back(A);
         b->nmPadMax = std::max(b->nmPadMax, A.nmPad);
         b->nmapsMax = std::max(b->nmapsMax, A.nmaps);
+        b->anySlots = b->anySlots || A.slotMaps;
         for (int k = 0; k < ncta; k++) au.push_back({(double)c->nAtoms, make_int2(ja, k)});
       }
       continue;
@@ -1470,6 +1574,7 @@ int batchBuild(ag_batch* b) {
   for (auto& u : au) aul.push_back(u.second);
   b->ne = (int)eul.size();
   b->na = (int)aul.size();
+  b->na2 = (int)a2j.size();
   CK(b->ejobs.ensure(ej.size()));
   CK(b->ajobs.ensure(std::max<size_t>(aj.size(), 1)));
   CK(b->a2jobs.ensure(std::max<size_t>(a2j.size(), 1)));
@@ -1563,8 +1668,8 @@ extern "C" int ag_batch_compute(ag_batch* b) {
       if (!err) err = prepAffinity(c, st);
     if (!err) {
       const cudaError_t ae =
-          b->twoPoint ? agk::aff2_batch_launch(b->a2jobs.p, b->aunits.p, b->na, b->counters.p + 1, b->nmPadMax,
-                                               b->nmapsMax, 2 * sms, st)
+          b->twoPoint ? agk::aff2_batch_launch(b->a2jobs.p, b->na2, b->aunits.p, b->na, b->counters.p + 1,
+                                               b->nmPadMax, b->anySlots, sms, st)
                       : agk::aff_batch_launch(b->ajobs.p, b->aunits.p, b->na, b->counters.p + 1, b->nmPadMax,
                                               b->nmapsMax, 2 * sms, st);
       if (ae != cudaSuccess) err = fail(AG_E_CUDA, "batch affinity launch failed");
