@@ -86,4 +86,11 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
+// min(|a|, |b|, |c|) in one instruction.
+__device__ __forceinline__ float min3_abs(float a, float b, float c) {
+  float v;
+  asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(a), "f"(b), "f"(c));
+  return v;
+}
+
 }  // namespace agd

@@ -572,7 +572,10 @@ int emapChunk(int nAtoms, int nblocks, int sms, int ctasPerSm) {
   const int want = 2 * sms * ctasPerSm;
   if (nblocks >= want) return std::max(nAtoms, 1);
   const int ns = (want + nblocks - 1) / nblocks;
-  const int chunk = std::max(256, nAtoms / ns / 256 * 256);
+  int chunk = std::max(256, nAtoms / ns / 256 * 256);
+  const int parts = (nAtoms + chunk - 1) / chunk;
+  if (parts > 1 && nAtoms - (parts - 1) * chunk < chunk / 4)  // no split of a few atoms
+    chunk = ((nAtoms + parts - 2) / (parts - 1) + 255) / 256 * 256;
   if (chunk == 256 && (int64_t)nblocks * ((nAtoms + 255) / 256) < 3 * sms) return 128;
   return chunk;
 }

@@ -77,9 +77,8 @@ __device__ __forceinline__ void near_batch(const NearSmem& S, const EmapParams& 
                                            float (&cmp)[kNX]) {
   const float cap = 0.02f;        // min(1/r, 2) in units of 1/(100 r)
   const float kBias = 8388608.f;  // 2^23: adding it with round-down leaves floor() in the low bits
-  const float2 bias2 = dup2(kBias), mone2 = dup2(-1.f), mhalf2 = dup2(-0.5f);
+  const float2 bias2 = dup2(kBias), mone2 = dup2(-1.f);
   const float2 np0 = dup2(-P.psi[0]), np1 = dup2(-P.psi[1]), np2 = dup2(-P.psi[2]);
-  const float edge = 0.5f - P.delta;
   const float rcut2 = P.rcut2;
   const float warpCut2 = rcut2 * 1.0001f;
   const uint32_t tabBiased = smem_u32(S.tab) - 0x2C000000u;  // address(tab) - 4 * bits(2^23)
@@ -103,9 +102,10 @@ __device__ __forceinline__ void near_batch(const NearSmem& S, const EmapParams& 
       // The 1e-30 keeps r2 > 0 (an atom on a grid point) without a per-point max.
       const float2 dyz2 = dup2(fmaf(dz, dz, dy * dy) + 1e-30f);
       const float2 ax = dup2(a.x);
-      float2 rs[kNX / 2], r2[kNX / 2], npsi[kNX / 2], fr5[kNX / 2];
+      float2 rs[kNX / 2], r2[kNX / 2], npsi[kNX / 2];
+      float2 kn[kNX / 2];  // 2^23 + the integer nearest 100 r
+      float2 d[kNX / 2];   // 100 r minus that integer
       uint32_t bits[kNX];
-      bool any = false;
 #pragma unroll
       for (int k = 0; k < kNX / 2; k++) {
         const float2 dx = __fadd2_rn(ax, gxn[k]);
@@ -117,10 +117,14 @@ __device__ __forceinline__ void near_batch(const NearSmem& S, const EmapParams& 
         f.y = fminf(f.y, kBias + (float)(kTabLen - 1));
         bits[2 * k] = __float_as_uint(f.x);
         bits[2 * k + 1] = __float_as_uint(f.y);
-        // fraction of 100 r, minus one half: within delta of a bin edge <=> |fr5| > 0.5 - delta
-        fr5[k] = __fadd2_rn(__fadd2_rn(__fmul2_rn(r2[k], rs[k]), __ffma2_rn(f, mone2, bias2)), mhalf2);
-        any |= ((r2[k].x < rcut2) & (fabsf(fr5[k].x) > edge)) | ((r2[k].y < rcut2) & (fabsf(fr5[k].y) > edge));
+        kn[k] = __ffma2_rn(r2[k], rs[k], bias2);
+        d[k] = __ffma2_rn(r2[k], rs[k], __ffma2_rn(kn[k], mone2, bias2));
       }
+      // Within delta of a bin edge <=> 100 r is within delta of an integer (for
+      // points beyond rcut too, whose term is zero either way).
+      static_assert(kNX == 8, "eight points");
+      const bool any = min3_abs(min3_abs(d[0].x, d[0].y, d[1].x), min3_abs(d[1].y, d[2].x, d[2].y),
+                                fminf(fabsf(d[3].x), fabsf(d[3].y))) < P.delta;
       if (__any_sync(0xffffffffu, any)) {
         if (any) {
           const double4 a64 = S.nearD[j];
@@ -130,9 +134,9 @@ __device__ __forceinline__ void near_batch(const NearSmem& S, const EmapParams& 
 #pragma unroll
           for (int k = 0; k < kNX; k++) {
             const float r2k = lo_hi(r2[k >> 1], k);
-            if (r2k < rcut2 && fabsf(lo_hi(fr5[k >> 1], k)) > edge) {
+            if (r2k < rcut2 && fabsf(lo_hi(d[k >> 1], k)) < P.delta) {
               // The reference's bin is kmid - 1 or kmid, kmid the integer nearest 100 r.
-              const int kmid = min(__float_as_int(r2k * lo_hi(rs[k >> 1], k) + 12582912.f) - 0x4B400000, kTabLen - 1);
+              const int kmid = min(__float_as_int(lo_hi(kn[k >> 1], k)) - 0x4B000000, kTabLen - 1);
               const double gx64 = __dmul_rn((double)(xc * kNX + k - P.n2x), h);
               const double ddx = __dsub_rn(a64.x, gx64);
               const double r2d = __dadd_rn(__dmul_rn(ddx, ddx), dydz);
