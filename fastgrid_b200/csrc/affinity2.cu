@@ -47,7 +47,7 @@ namespace {
 
 constexpr int kT = 256;              // threads per CTA, two points each
 constexpr int kW = kT / 32;
-constexpr int kCellGroup = 128;      // cells per gather group (a CTA box reaches at most 4^3)
+constexpr int kSegs = kT;            // cell-list segments per gather round (one per thread)
 constexpr float kBias = 8388608.f;   // 2^23
 
 constexpr int kPlaneRows = kA2PlaneRows;
@@ -73,11 +73,11 @@ struct PartSmem<PART_SLOTS> {
   float4 rch[kT][2];                 // per thread and point: rvector of the nearest H donor
 };
 
-// The CTA's box in the grid-centred frame and the 8 A cells around it.
+// The CTA's box in the grid-centred frame and the cells around it.
 struct Box {
   double ox, oy, oz;                 // CTA frame origin (its first lattice point)
   double lo[3], hi[3];               // CTA box
-  int c0[3], ncx, ncy, ncells;       // cells around the box
+  int c0[3], ncx, ncy, nrows;        // cells around the box: nrows rows of ncx cells along x
 };
 
 template <int PART>
@@ -89,8 +89,8 @@ struct A2Smem : PartSmem<PART> {
   int wStart[kW][kMaxTypes + 1];     // per warp: first wlist entry of each type (in the part's type order)
   int typeCount[kMaxTypes];
   int typeStart[kMaxTypes + 1];
-  int cellPre[kCellGroup + 1];
-  int cellBeg[kCellGroup];
+  int segPre[kSegs + 1];             // atoms before each segment of the round
+  int segBeg[kSegs];                 // each segment's first entry in the sorted atoms
   int cnt[kW];
   Box box;
   float sblo[kW][3], sbhi[kW][3];    // each warp's sub-box in the CTA frame (lo > hi: past the grid edge)
@@ -413,74 +413,67 @@ static size_t aff2_smem(int nmPad, bool slots) {
   return slots ? std::max(plain, tabOffset<PART_SLOTS>() + kSlotsRegion) : plain;
 }
 
-// Cell ranges of receptor type t in cell group cg: S.cellBeg / S.cellPre.
-// Returns the group's cell count (S.cellPre[ncg] is its atom count).
+// The segments g0 .. g0 + kSegs of the cells around the box (each type of the
+// part's order in turn, row by row: a row's cells are one run of the type-major
+// list): S.segBeg / S.segPre.  Returns the round's atom count.
 template <int PART>
-__device__ __forceinline__ int cell_prefix(const Aff2Params& P, A2Smem<PART>& S, const int t, const int cg) {
+__device__ __forceinline__ int segment_round(const Aff2Params& P, A2Smem<PART>& S, const unsigned char* order,
+                                             const int nsegs, const int g0) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const Box& B = S.box;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int ncg = min(kCellGroup, B.ncells - cg);
-  __syncthreads();  // the previous group's ranges are no longer read
-  if (warp == 0) {
-    constexpr int kPer = kCellGroup / 32;
-    int cnts[kPer];
-    int mine = 0;
-#pragma unroll
-    for (int u = 0; u < kPer; u++) {
-      const int i = lane * kPer + u;
-      int cn = 0;
-      if (i < ncg) {
-        const int ci = cg + i;
-        const int cx = B.c0[0] + ci % B.ncx, cy = B.c0[1] + (ci / B.ncx) % B.ncy, cz = B.c0[2] + ci / (B.ncx * B.ncy);
-        const int key = ((cz * P.ncell[1] + cy) * P.ncell[0] + cx) * P.ntypes + t;
-        const int beg = P.ctStart[key];
-        cn = P.ctStart[key + 1] - beg;
-        S.cellBeg[i] = beg;
-      }
-      cnts[u] = cn;
-      mine += cn;
-    }
-    int incl = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    int run = incl - mine;
-#pragma unroll
-    for (int u = 0; u < kPer; u++) {
-      const int i = lane * kPer + u;
-      if (i < ncg) S.cellPre[i] = run;
-      run += cnts[u];
-    }
-    if (lane == 31) S.cellPre[ncg] = incl;
+  int cnt = 0;
+  const int i = g0 + tid;
+  if (i < nsegs) {
+    const int pos = i / B.nrows, row = i - pos * B.nrows;
+    const int ry = row % B.ncy, rz = row / B.ncy;
+    const int key = (((int)order[pos] * P.ncell[2] + B.c0[2] + rz) * P.ncell[1] + B.c0[1] + ry) * P.ncell[0] + B.c0[0];
+    const int beg = P.ctStart[key];
+    cnt = P.ctStart[key + B.ncx] - beg;
+    S.segBeg[tid] = beg;
   }
+  int incl = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) S.cnt[warp] = incl;
   __syncthreads();
-  return ncg;
+  int off = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < kW; w++) {
+    if (w == warp) off = total;
+    total += S.cnt[w];
+  }
+  S.segPre[tid + 1] = off + incl;
+  if (tid == 0) S.segPre[0] = 0;
+  __syncthreads();
+  return total;
 }
 
-// Up to kT atoms v0 .. v0 + kT of the current cell group (the type at place
-// `pos` of the part's order) that lie
-// within 8 A of the CTA box, appended to the candidate arrays at slot nb
-// (d64: with their FP64 records there, else with the fields of the part's
-// sums).  Returns the new count.
+// Up to kT atoms v0 .. v0 + kT of the current round that lie within 8 A of the
+// CTA box, appended to the candidate arrays at slot nb (d64: with their FP64
+// records there, else with the fields of the part's sums).  Returns the new
+// count.
 template <int PART>
-__device__ __forceinline__ int gather_chunk(const Aff2Params& P, A2Smem<PART>& S, const int pos, const int ncg,
-                                            const int total, const int v0, const int nb, double4* d64) {
+__device__ __forceinline__ int gather_chunk(const Aff2Params& P, A2Smem<PART>& S, const int g0, const int total,
+                                            const int v0, const int nb, double4* d64) {
   const Box& B = S.box;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int v = v0 + tid;
   bool keep = false;
-  int atom = -1;
+  int seg = 0;
   double4 a = make_double4(0, 0, 0, 0);
+  float4 aux = make_float4(0.f, 0.f, 0.f, 0.f);
   if (v < total) {
-    int lo_i = 0, hi_i = ncg - 1;  // last cell with cellPre <= v
-    while (lo_i < hi_i) {
-      const int mid = (lo_i + hi_i + 1) >> 1;
-      if (S.cellPre[mid] <= v) lo_i = mid; else hi_i = mid - 1;
+    int hi_i = kSegs - 1;            // last segment with segPre <= v
+    while (seg < hi_i) {
+      const int mid = (seg + hi_i + 1) >> 1;
+      if (S.segPre[mid] <= v) seg = mid; else hi_i = mid - 1;
     }
-    atom = P.ctAtoms[S.cellBeg[lo_i] + (v - S.cellPre[lo_i])];
-    a = P.xyz[atom];
+    const int j = S.segBeg[seg] + (v - S.segPre[seg]);
+    a = P.ctXyz[j];
+    aux = P.ctAux[j];                // vol, solq, info bits, atom index
     const double ddx = fmax(fmax(B.lo[0] - a.x, a.x - B.hi[0]), 0.0);
     const double ddy = fmax(fmax(B.lo[1] - a.y, a.y - B.hi[1]), 0.0);
     const double ddz = fmax(fmax(B.lo[2] - a.z, a.z - B.hi[2]), 0.0);
@@ -497,22 +490,53 @@ __device__ __forceinline__ int gather_chunk(const Aff2Params& P, A2Smem<PART>& S
   }
   if (keep) {
     const int j = nb + off + __popc(kbal & ((1u << lane) - 1u));
-    const int inf = P.info[atom];
-    S.pos[j] = make_float4((float)(a.x - B.ox), (float)(a.y - B.oy), (float)(a.z - B.oz), __int_as_float(inf));
+    const int atom = __float_as_int(aux.w);
+    S.pos[j] = make_float4((float)(a.x - B.ox), (float)(a.y - B.oy), (float)(a.z - B.oz), aux.z);
     S.idx[j] = atom;
     if constexpr (PART == PART_PLAIN) {
-      S.vs[j] = make_float2(P.vol[atom], P.solq[atom]);
+      S.vs[j] = make_float2(aux.x, aux.y);
+      atomicAdd(&S.typeCount[(g0 + seg) / B.nrows], 1);
     } else if (d64) {
       d64[j] = a;
     } else {
       const float4 va = __ldg(P.rv8 + 2 * (size_t)atom), vb = __ldg(P.rv8 + 2 * (size_t)atom + 1);
       S.rvA[j] = make_float4(va.x, va.y, va.z, vb.x);
       S.rvB[j] = make_float2(vb.y, vb.z);
+      atomicAdd(&S.typeCount[(g0 + seg) / B.nrows], 1);
     }
   }
-  if (tid == 0) S.typeCount[pos] += tot;
   __syncthreads();
   return nb + tot;
+}
+
+// The candidates of the part's `ntypes` types, in type-major order, in batches
+// of at most kCap: batch(nb) takes each.  Returns false if batch does.
+template <int PART, class Batch>
+__device__ __forceinline__ bool gather_batches(const Aff2Params& P, A2Smem<PART>& S, const unsigned char* order,
+                                               const int ntypes, double4* d64, const Batch& batch) {
+  const int nsegs = ntypes * S.box.nrows;
+  int g = -kSegs, v0 = 0, total = 0, nb = 0;
+  for (;;) {
+    bool last = false;
+    for (;;) {
+      if (v0 >= total) {
+        g += kSegs;
+        if (g >= nsegs) {
+          last = true;
+          break;
+        }
+        total = segment_round<PART>(P, S, order, nsegs, g);
+        v0 = 0;
+        continue;
+      }
+      if (nb + min(kT, total - v0) > A2Smem<PART>::kCap) break;  // a chunk keeps at most that many atoms
+      nb = gather_chunk<PART>(P, S, g, total, v0, nb, d64);
+      v0 += kT;
+    }
+    if (nb > 0 && !batch(nb)) return false;
+    if (last) return true;
+    nb = 0;
+  }
 }
 
 // Nearest H donor of both points over candidates 0 .. nb (FP64 exact, ties to
@@ -654,7 +678,7 @@ __device__ __forceinline__ bool aff2_unit(const Aff2Params& P, const int cta, un
     q.py = (float)(gcoord(q.iy, P.n2y, h) - oy);
     q.pz[0] = (float)(gcoord(q.iz0, P.n2z, h) - oz);
     q.pz[1] = (float)(gcoord(q.iz0 + 1, P.n2z, h) - oz);
-    // CTA box (FP64, grid-centred) and the 8 A cells around it.
+    // CTA box (FP64, grid-centred) and the cells within 8 A of it.
     if (tid == 0) {
       Box& B = S.box;
       B.ox = ox;
@@ -666,12 +690,12 @@ __device__ __forceinline__ bool aff2_unit(const Aff2Params& P, const int cta, un
       int nc[3];
 #pragma unroll
       for (int d = 0; d < 3; d++) {
-        B.c0[d] = max(0, (int)floor((B.lo[d] - 8.0 - P.cellLo[d]) / 8.0));
-        nc[d] = min(P.ncell[d] - 1, (int)floor((B.hi[d] + 8.0 - P.cellLo[d]) / 8.0)) - B.c0[d] + 1;
+        B.c0[d] = max(0, (int)floor((B.lo[d] - 8.0 - P.cellLo[d]) / P.cellEdge));
+        nc[d] = min(P.ncell[d] - 1, (int)floor((B.hi[d] + 8.0 - P.cellLo[d]) / P.cellEdge)) - B.c0[d] + 1;
       }
       B.ncx = nc[0];
       B.ncy = nc[1];
-      B.ncells = (nc[0] > 0 && nc[1] > 0 && nc[2] > 0) ? nc[0] * nc[1] * nc[2] : 0;
+      B.nrows = (nc[0] > 0 && nc[1] > 0 && nc[2] > 0) ? nc[1] * nc[2] : 0;
     }
     // This warp's sub-box in the CTA frame (empty when it lies past the grid edge).
     if (lane == 0) {
@@ -685,25 +709,12 @@ __device__ __forceinline__ bool aff2_unit(const Aff2Params& P, const int cta, un
     }
   }
   for (int t = tid; t < kMaxTypes; t += kT) S.typeCount[t] = 0;
-  int nb = 0;
 
   // Batches of candidates in type-major order, walked type by type.
   auto walk = [&](const unsigned char* order, const int ntypes, auto load, auto sums) AG_INLINE -> bool {
-    for (int pos = 0; pos < ntypes; pos++) {
-      const int t = order[pos];
-      for (int cg = 0; cg < S.box.ncells; cg += kCellGroup) {
-        const int ncg = cell_prefix<PART>(P, S, t, cg);
-        const int total = S.cellPre[ncg];
-        for (int v0 = 0; v0 < total; v0 += kT) {
-          if (nb + min(kT, total - v0) > kCap) {  // this round keeps at most that many atoms
-            if (!process_batch<PART>(P, S, ntypes, nb, tb, load, sums)) return false;
-            nb = 0;
-          }
-          nb = gather_chunk<PART>(P, S, pos, ncg, total, v0, nb, nullptr);
-        }
-      }
-    }
-    return nb == 0 || process_batch<PART>(P, S, ntypes, nb, tb, load, sums);
+    return gather_batches<PART>(P, S, order, ntypes, nullptr, [&](int nb) AG_INLINE -> bool {
+      return process_batch<PART>(P, S, ntypes, nb, tb, load, sums);
+    });
   };
 
   if constexpr (PART == PART_PLAIN) {
@@ -775,23 +786,10 @@ __device__ __forceinline__ bool aff2_unit(const Aff2Params& P, const int cta, un
       double4* d64 = reinterpret_cast<double4*>(tab);
       double best[2] = {1e300, 1e300};
       int bi[2] = {-1, -1};
-      for (int t = 0; t < P.ntypes; t++) {
-        if (!P.typeDonor[t]) continue;
-        for (int cg = 0; cg < S.box.ncells; cg += kCellGroup) {
-          const int ncg = cell_prefix<PART>(P, S, t, cg);
-          const int total = S.cellPre[ncg];
-          for (int v0 = 0; v0 < total; v0 += kT) {
-            if (nb + min(kT, total - v0) > kCap) {
-              scan_donors(P, S, d64, nb, best, bi, q);
-              nb = 0;
-            }
-            nb = gather_chunk<PART>(P, S, 0, ncg, total, v0, nb, d64);
-          }
-        }
-      }
-      scan_donors(P, S, d64, nb, best, bi, q);
-      nb = 0;
-      for (int t = tid; t < kMaxTypes; t += kT) S.typeCount[t] = 0;
+      gather_batches<PART>(P, S, P.donorOrder, P.nDonorTypes, d64, [&](int nb) AG_INLINE -> bool {
+        scan_donors(P, S, d64, nb, best, bi, q);
+        return true;
+      });
 #pragma unroll
       for (int p = 0; p < 2; p++) {
         s.ch[p] = (best[p] <= 64.0) ? bi[p] : -1;

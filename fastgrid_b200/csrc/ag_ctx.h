@@ -78,8 +78,10 @@ struct ag_ctx {
   uint64_t atomsVersion = 0;      // bumped whenever new atoms are staged
   uint64_t atomsHostVersion = ~0ull;  // the staging atomsHost holds
   // affinity
-  agc::DevBuf<int> info, cellStart, cellAtoms, cellOf, count, fill, dStart, dAtoms, donorMask, closestH;
-  agc::DevBuf<int> ctStart, ctAtoms;  // type-major cell list ((cell, type) segments) of the two-point kernel
+  agc::DevBuf<int> info, cellStart, cellAtoms, cellOf, count, dStart, dAtoms, donorMask, closestH;
+  agc::DevBuf<int> ctStart, ctAtoms;  // type-major cell list of the two-point kernel, with the sorted records
+  agc::DevBuf<double4> ctXyz;
+  agc::DevBuf<float4> ctAux;
   int affKernel = 2;                  // affinity kernel: 2 two-point (default), 1 one point per thread
   agc::DevBuf<float> vol, solq, affTab, affRaw, sol;
   agc::DevBuf<float4> rv8;            // per atom: rvector, 0, rvector2, 0

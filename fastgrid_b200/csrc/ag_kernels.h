@@ -131,23 +131,28 @@ cudaError_t aff_launch(const AffParams& P, cudaStream_t st);
 cudaError_t aff_batch_launch(const AffParams* jobs, const int2* units, int nunits, int* counter, int nmPadMax,
                              int nmapsMax, int grid, cudaStream_t st);
 
-// Cell list build (counting sort of atoms into 8 A cells, file order kept inside each cell).
+// Cell list build (counting sort of atoms into cells, file order kept inside each cell).
 struct CellBuild {
   const double4* xyz;
   int n_atoms;
   double lo[3];
+  double edge;                    // A
   int ncell[3];
   int* cellOf;                    // n_atoms scratch
-  int* count;                     // ncell + 1 scratch (zeroed by the launcher)
-  int* cellStart;                 // ncell + 1
+  int* count;                     // 2 * (keys + 1) scratch
+  int* cellStart;                 // keys + 1
   int* cellAtoms;                 // n_atoms
-  int* fill;                      // ncell scratch
   const int* donorMask;           // optional: only atoms with mask[i] != 0 (null = all)
-  const int* typeInfo;            // optional: key = cell * ntypes + (typeInfo[i] & 31) (type-major segments)
+  // Type-major list of the two-point affinity kernel (ntypes > 0): key = type *
+  // cells + cell, and the atoms' records copied into sorted order.
   int ntypes;
+  const int* info;                // type in the low five bits
+  const float *vol, *solq;
+  double4* sXyz;
+  float4* sAux;                   // vol, solq, info bits, atom index bits
 };
-// ncellTotal: number of keys (cells, or cells x ntypes with typeInfo).
-cudaError_t cells_launch(const CellBuild& C, int ncellTotal, cudaStream_t st);
+// Returns the number of kernels it launched in *launched.
+cudaError_t cells_launch(const CellBuild& C, cudaStream_t st, int* launched);
 
 // ---------------------------------------------------------------------------
 // Affinity + desolvation, two grid points per thread (affinity2.cu)
@@ -160,14 +165,14 @@ enum { A2_SLOT_ACC = 0, A2_SLOT_A1 = 1, A2_SLOT_DON = 2 };     // H-bond map kin
 struct Aff2Params {
   // receptor (device)
   const double4* xyz;             // FP64 grid-centred x, y, z
-  const int* info;                // type | hbond << 5 | disorder << 8 | rexp << 9
-  const float* vol;
-  const float* solq;
   const float4* rv8;              // per atom: rvector, 0, rvector2, 0 (FP32)
   const double* rv64;             // rvector (FP64) for exact sign decisions
-  // type-major cell list: segment (cell, type) = atoms ctAtoms[ctStart[cell*ntypes+t] .. ctStart[...+1])
+  // type-major cell list: the atoms of type t in cell c, in file order, are the
+  // sorted entries ctStart[t * ncells + c] .. ctStart[t * ncells + c + 1]
   const int* ctStart;
-  const int* ctAtoms;
+  const double4* ctXyz;           // sorted: FP64 record
+  const float4* ctAux;            // sorted: vol, solq, info bits, atom index bits
+  double cellEdge;                // A
   double cellLo[3];
   int ncell[3];
   // grid
@@ -192,7 +197,8 @@ struct Aff2Params {
   float delta;                    // guard half-width around bin edges (bins)
   int needClosestH;               // some D1 type meets an acceptor-probe slot: find the nearest donor
   int typeAng[kMaxTypes];         // A2_SPH / A2_D1 / A2_A1 / A2_A2
-  int typeDonor[kMaxTypes];       // DS or D1 (candidates of the nearest-donor search)
+  int nDonorTypes;                // DS and D1 types (candidates of the nearest-donor search), and their list
+  unsigned char donorOrder[kMaxTypes];
   unsigned typeSlots[kMaxTypes];  // bit k: H-bond slot k applies to this type
   int nslots;
   int slotMap[kA2Slots];          // map index of each H-bond slot

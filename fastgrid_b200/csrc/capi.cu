@@ -148,6 +148,8 @@ extern "C" int ag_ctx_destroy(ag_ctx* c) {
   for (auto* b : {&c->epsTab, &c->maps, &c->vol, &c->solq, &c->affTab, &c->affRaw, &c->sol})
     b->release();
   c->rv8.release();
+  c->ctXyz.release();
+  c->ctAux.release();
   c->atoms.release();
   c->thr.release();
   c->partial.release();
@@ -158,7 +160,7 @@ extern "C" int ag_ctx_destroy(ag_ctx* c) {
   c->surr = nullptr;
   c->blocks.release();
   c->status.release();
-  for (auto* b : {&c->items, &c->info, &c->cellStart, &c->cellAtoms, &c->cellOf, &c->count, &c->fill, &c->dStart,
+  for (auto* b : {&c->items, &c->info, &c->cellStart, &c->cellAtoms, &c->cellOf, &c->count, &c->dStart,
                   &c->dAtoms, &c->donorMask, &c->closestH, &c->ctStart, &c->ctAtoms})
     b->release();
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -900,15 +902,25 @@ int stageAffinity(ag_ctx* c, const ag_receptor* r, const ag_affinity_params* p) 
   return AG_OK;
 }
 
-// 8 A cells over the grid box widened by 8 A (atoms further out cannot reach a point).
-void cellGrid(const ag_grid& g, double lo[3], int ncell[3]) {
+// Cells over the grid box widened by 8 A (atoms further out cannot reach a point).
+void cellGrid(const ag_grid& g, double edge, double lo[3], int ncell[3]) {
   const double h = g.spacing;
   const int nn[3] = {g.nx, g.ny, g.nz};
   for (int d = 0; d < 3; d++) {
     lo[d] = (double)(0 - nn[d] / 2) * h - 8.0;
     const double hi = (double)(nn[d] - 1 - nn[d] / 2) * h + 8.0;
-    ncell[d] = std::max(1, (int)std::ceil((hi - lo[d]) / 8.0));
+    ncell[d] = std::max(1, (int)std::ceil((hi - lo[d]) / edge));
   }
+}
+
+// Cell edge of the two-point kernel's list: 4 A cells around an 8^3 box hold
+// 0.6 of the atoms that 8 A cells do; 8 A where the keys would be too many.
+double twoPointCells(const ag_ctx* c, double lo[3], int ncell[3]) {
+  for (double edge : {4.0, 8.0}) {
+    cellGrid(c->grid, edge, lo, ncell);
+    if ((int64_t)ncell[0] * ncell[1] * ncell[2] * c->nTypes <= (1 << 21)) return edge;
+  }
+  return 8.0;
 }
 
 // Whether every affinity pass of the staged job runs on the two-point kernel.
@@ -929,32 +941,37 @@ int prepAffinity(ag_ctx* c, cudaStream_t st) {
   const double h = g.spacing;
   double lo[3];
   int ncell[3];
-  cellGrid(g, lo, ncell);
-  const int ncellT = ncell[0] * ncell[1] * ncell[2];
   agk::CellBuild C{};
   C.xyz = c->atoms.p; C.n_atoms = n;
-  for (int d = 0; d < 3; d++) { C.lo[d] = lo[d]; C.ncell[d] = ncell[d]; }
+  int launched = 0;
   if (useTwoPoint(c)) {
-    const int nkeys = ncellT * c->nTypes;
-    CK(c->ctStart.ensure(nkeys + 1)); CK(c->count.ensure(nkeys + 1)); CK(c->fill.ensure(nkeys + 1));
-    CK(c->ctAtoms.ensure(n)); CK(c->cellOf.ensure(n));
-    C.cellOf = c->cellOf.p; C.count = c->count.p; C.fill = c->fill.p;
+    C.edge = twoPointCells(c, lo, ncell);
+    const size_t nkeys = (size_t)ncell[0] * ncell[1] * ncell[2] * c->nTypes;
+    for (int d = 0; d < 3; d++) { C.lo[d] = lo[d]; C.ncell[d] = ncell[d]; }
+    CK(c->ctStart.ensure(nkeys + 1)); CK(c->count.ensure(2 * (nkeys + 1)));
+    CK(c->ctAtoms.ensure(n)); CK(c->cellOf.ensure(n)); CK(c->ctXyz.ensure(n)); CK(c->ctAux.ensure(n));
+    C.cellOf = c->cellOf.p; C.count = c->count.p;
     C.cellStart = c->ctStart.p; C.cellAtoms = c->ctAtoms.p; C.donorMask = nullptr;
-    C.typeInfo = c->info.p; C.ntypes = c->nTypes;
-    CK(agk::cells_launch(C, nkeys, st));
-    c->launches += 4;
+    C.ntypes = c->nTypes; C.info = c->info.p; C.vol = c->vol.p; C.solq = c->solq.p;
+    C.sXyz = c->ctXyz.p; C.sAux = c->ctAux.p;
+    CK(agk::cells_launch(C, st, &launched));
+    c->launches += launched;
     return AG_OK;
   }
-  CK(c->cellStart.ensure(ncellT + 1)); CK(c->count.ensure(ncellT + 1)); CK(c->fill.ensure(ncellT + 1));
+  C.edge = 8.0;
+  cellGrid(g, C.edge, lo, ncell);
+  const int ncellT = ncell[0] * ncell[1] * ncell[2];
+  for (int d = 0; d < 3; d++) { C.lo[d] = lo[d]; C.ncell[d] = ncell[d]; }
+  CK(c->cellStart.ensure(ncellT + 1)); CK(c->count.ensure(2 * ((size_t)ncellT + 1)));
   CK(c->cellAtoms.ensure(n)); CK(c->cellOf.ensure(n));
   CK(c->dStart.ensure(ncellT + 1)); CK(c->dAtoms.ensure(n));
   CK(c->closestH.ensure(np));
-  C.cellOf = c->cellOf.p; C.count = c->count.p; C.fill = c->fill.p;
+  C.cellOf = c->cellOf.p; C.count = c->count.p;
   C.cellStart = c->cellStart.p; C.cellAtoms = c->cellAtoms.p; C.donorMask = nullptr;
-  CK(agk::cells_launch(C, ncellT, st));
+  CK(agk::cells_launch(C, st, &launched));
   C.cellStart = c->dStart.p; C.cellAtoms = c->dAtoms.p; C.donorMask = c->donorMask.p;
-  CK(agk::cells_launch(C, ncellT, st));
-  c->launches += 8;
+  CK(agk::cells_launch(C, st, &launched));
+  c->launches += launched;
   agk::ClosestHParams H{};
   H.xyz = c->atoms.p; H.cellStart = c->dStart.p; H.cellAtoms = c->dAtoms.p;
   for (int d = 0; d < 3; d++) { H.cellLo[d] = lo[d]; H.ncell[d] = ncell[d]; }
@@ -970,14 +987,15 @@ int buildAff2Params(ag_ctx* c, float* dMaps, float* dDmap, std::vector<agk::Aff2
   const ag_grid& g = c->grid;
   double lo[3];
   int ncell[3];
-  cellGrid(g, lo, ncell);
+  const double edge = twoPointCells(c, lo, ncell);
   out.clear();
   const int nt = c->nTypes;
   for (const auto& ps : c->passes) {
     agk::Aff2Params P{};
-    P.xyz = c->atoms.p; P.info = c->info.p; P.vol = c->vol.p; P.solq = c->solq.p;
+    P.xyz = c->atoms.p;
     P.rv8 = c->rv8.p; P.rv64 = c->rv64.p;
-    P.ctStart = c->ctStart.p; P.ctAtoms = c->ctAtoms.p;
+    P.ctStart = c->ctStart.p; P.ctXyz = c->ctXyz.p; P.ctAux = c->ctAux.p;
+    P.cellEdge = edge;
     for (int d = 0; d < 3; d++) { P.cellLo[d] = lo[d]; P.ncell[d] = ncell[d]; }
     P.nx = g.nx; P.ny = g.ny; P.nz = g.nz; P.n2x = g.nx / 2; P.n2y = g.ny / 2; P.n2z = g.nz / 2;
     P.npoints = c->npoints(); P.h = g.spacing;
@@ -1008,7 +1026,7 @@ int buildAff2Params(ag_ctx* c, float* dMaps, float* dDmap, std::vector<agk::Aff2
     for (int t = 0; t < agk::kMaxTypes; t++) {
       const int ahb = t < nt ? c->typeHbond[t] : ag::NON;
       P.typeSlots[t] = t < nt ? ps.typeSlots[t] : 0u;
-      P.typeDonor[t] = ahb == ag::DS || ahb == ag::D1 ? 1 : 0;
+      if (ahb == ag::DS || ahb == ag::D1) P.donorOrder[P.nDonorTypes++] = (unsigned char)t;
       P.typeAng[t] = ahb == ag::D1 ? agk::A2_D1 : ahb == ag::A1 ? agk::A2_A1 : ahb == ag::A2 ? agk::A2_A2 : agk::A2_SPH;
       if (P.typeSlots[t]) P.slotOrder[P.nSlotTypes++] = (unsigned char)t;
       for (int k = 0; k < P.nslots; k++)
@@ -1039,7 +1057,7 @@ int buildAffParams(ag_ctx* c, float* dMaps, float* dDmap, std::vector<agk::AffPa
   const double h = g.spacing;
   double lo[3];
   int ncell[3];
-  cellGrid(g, lo, ncell);
+  cellGrid(g, 8.0, lo, ncell);
   out.clear();
   const int nt = c->nTypes;
   for (const auto& ps : c->passes) {
@@ -1696,7 +1714,7 @@ extern "C" int ag_batch_compute(ag_batch* b) {
   CK(cudaEventRecord(b->ev[0], st));
   CK(cudaGraphLaunch(b->exec, st));
   CK(cudaEventRecord(b->ev[1], st));
-  b->ctx->launches += 2 + 9 * (int64_t)b->sub.size();
+  b->ctx->launches += 2 + (int64_t)b->sub.size();
   CK(cudaStreamSynchronize(st));
   {
     float ms = 0.f;

@@ -1,5 +1,5 @@
 // Helper kernels of the affinity pass and the small per-point maps:
-//  * the device cell list (counting sort of atoms into 8 A cells, file order
+//  * the device cell list (counting sort of atoms into cells, file order
 //    kept inside each cell) that replaces FastGrid's cutoff grid
 //    (SpatialGrid.h:50-315),
 //  * the nearest H donor of every grid point (the role of FastGrid's ANN
@@ -22,81 +22,169 @@ __device__ __forceinline__ double rsq_exact_c(double ax, double ay, double az, d
 }
 
 // ---------------------------------------------------------------------------
-// Cell list: counting sort into 8 A cells (or into (cell, type) segments);
-// file order inside each cell or segment.
+// Cell list: counting sort into cells (or into type-major (type, cell) keys);
+// file order inside each key.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ int cell_key(const CellBuild& C, int i) {
+  if (C.donorMask && !C.donorMask[i]) return -1;
+  const double4 a = C.xyz[i];
+  const int cx = (int)floor((a.x - C.lo[0]) / C.edge), cy = (int)floor((a.y - C.lo[1]) / C.edge),
+            cz = (int)floor((a.z - C.lo[2]) / C.edge);
+  if (cx < 0 || cy < 0 || cz < 0 || cx >= C.ncell[0] || cy >= C.ncell[1] || cz >= C.ncell[2]) return -1;
+  const int type = C.ntypes > 0 ? C.info[i] & 31 : 0;
+  return ((type * C.ncell[2] + cz) * C.ncell[1] + cy) * C.ncell[0] + cx;
+}
+
+// Atom v's record at place `at` of the sorted order.
+__device__ __forceinline__ void place_record(const CellBuild& C, int at, int v) {
+  C.sXyz[at] = C.xyz[v];
+  C.sAux[at] = make_float4(C.vol[v], C.solq[v], __int_as_float(C.info[v]), __int_as_float(v));
+}
+
 __global__ void cell_count_kernel(CellBuild C) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < C.n_atoms; i += gridDim.x * blockDim.x) {
-    int cell = -1;
-    if (!C.donorMask || C.donorMask[i]) {
-      const double4 a = C.xyz[i];
-      const int cx = (int)floor((a.x - C.lo[0]) / 8.0), cy = (int)floor((a.y - C.lo[1]) / 8.0),
-                cz = (int)floor((a.z - C.lo[2]) / 8.0);
-      if (cx >= 0 && cy >= 0 && cz >= 0 && cx < C.ncell[0] && cy < C.ncell[1] && cz < C.ncell[2]) {
-        cell = (cz * C.ncell[1] + cy) * C.ncell[0] + cx;
-        if (C.typeInfo) cell = cell * C.ntypes + (C.typeInfo[i] & 31);
-      }
-    }
-    C.cellOf[i] = cell;
-    if (cell >= 0) atomicAdd(&C.count[cell], 1);
+    const int key = cell_key(C, i);
+    C.cellOf[i] = key;
+    if (key >= 0) atomicAdd(&C.count[key], 1);
   }
 }
 
-// Exclusive scan of the counts by one CTA (cells are at most a few hundred thousand).
-__global__ void cell_scan_kernel(const int* count, int n, int* start) {
-  __shared__ int part[1024];
-  const int tid = threadIdx.x;
-  const int per = (n + 1023) / 1024;
-  const int b = tid * per, e = min(n, b + per);
-  int s = 0;
-  for (int i = b; i < e; i++) s += count[i];
-  part[tid] = s;
+// Exclusive scan over the CTA's threads of v; `sum` receives the total.
+__device__ __forceinline__ int block_scan(int v, int* warpSums, int& sum) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  __syncthreads();  // the previous scan's sums are read
+  if (lane == 31) warpSums[warp] = incl;
   __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {
-    int v = tid >= off ? part[tid - off] : 0;
-    __syncthreads();
-    part[tid] += v;
-    __syncthreads();
+  int off = 0;
+  sum = 0;
+  for (int w = 0; w < nw; w++) {
+    if (w == warp) off = sum;
+    sum += warpSums[w];
   }
-  int run = part[tid] - s;
-  for (int i = b; i < e; i++) { start[i] = run; run += count[i]; }
-  if (tid == 1023) start[n] = part[1023];
+  return off + incl - v;
 }
 
-__global__ void cell_scatter_kernel(CellBuild C) {
+// Exclusive scan of the counts by one CTA, 8,192 keys per round.
+__global__ void __launch_bounds__(1024) cell_scan_kernel(const int* count, int n, int* start) {
+  __shared__ int warpSums[32];
+  int carry = 0;
+  for (int b = 0; b < n; b += 8192) {
+    const int i0 = b + 8 * threadIdx.x;
+    int c[8], s = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      c[k] = i0 + k < n ? count[i0 + k] : 0;
+      s += c[k];
+    }
+    int total;
+    int run = carry + block_scan(s, warpSums, total);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      if (i0 + k < n) start[i0 + k] = run;
+      run += c[k];
+    }
+    carry += total;
+  }
+  if (threadIdx.x == 0) start[n] = carry;
+}
+
+__global__ void cell_scatter_kernel(CellBuild C, int* fill) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < C.n_atoms; i += gridDim.x * blockDim.x) {
     const int cell = C.cellOf[i];
-    if (cell >= 0) C.cellAtoms[C.cellStart[cell] + atomicAdd(&C.fill[cell], 1)] = i;
+    if (cell >= 0) C.cellAtoms[C.cellStart[cell] + atomicAdd(&fill[cell], 1)] = i;
   }
 }
 
-// Restore file order inside each cell (one warp per cell, rank sort).
-__global__ void cell_sort_kernel(const int* cellStart, int ncell, int* cellAtoms, int* tmp) {
+// Restore file order inside each key (one warp per key, rank sort); the
+// type-major list gets the sorted records instead of the indexes.
+__global__ void cell_sort_kernel(CellBuild C, int nkeys) {
   const int warpsPerBlock = blockDim.x / 32;
   const int lane = threadIdx.x & 31;
-  for (int c = blockIdx.x * warpsPerBlock + threadIdx.x / 32; c < ncell; c += gridDim.x * warpsPerBlock) {
-    const int b = cellStart[c], e = cellStart[c + 1];
+  int* tmp = C.cellOf;  // n_atoms entries, free after the scatter
+  for (int c = blockIdx.x * warpsPerBlock + threadIdx.x / 32; c < nkeys; c += gridDim.x * warpsPerBlock) {
+    const int b = C.cellStart[c], e = C.cellStart[c + 1];
     for (int i = b + lane; i < e; i += 32) {
-      const int v = cellAtoms[i];
+      const int v = C.cellAtoms[i];
       int rank = 0;
-      for (int j = b; j < e; j++) rank += cellAtoms[j] < v;
-      tmp[b + rank] = v;
+      for (int j = b; j < e; j++) rank += C.cellAtoms[j] < v;
+      if (C.ntypes > 0) place_record(C, b + rank, v);
+      else tmp[b + rank] = v;
     }
+    if (C.ntypes > 0) continue;
     __syncwarp();
-    for (int i = b + lane; i < e; i += 32) cellAtoms[i] = tmp[i];
+    for (int i = b + lane; i < e; i += 32) C.cellAtoms[i] = tmp[i];
   }
 }
 
-cudaError_t cells_launch(const CellBuild& C, int ncellTotal, cudaStream_t st) {
-  cudaMemsetAsync(C.count, 0, sizeof(int) * (ncellTotal + 1), st);
-  cudaMemsetAsync(C.fill, 0, sizeof(int) * (ncellTotal + 1), st);
+// The whole type-major list by one CTA, its counts in shared memory: small
+// receptors are bound by the launches of the four kernels, not by their work
+// (2,000 atoms: one launch of 9 us instead of six of 3 us each).
+__global__ void __launch_bounds__(1024) cell_list_kernel(CellBuild C, int nkeys) {
+  extern __shared__ int cnt[];  // nkeys + 1
+  __shared__ int warpSums[32];
+  for (int k = threadIdx.x; k <= nkeys; k += blockDim.x) cnt[k] = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < C.n_atoms; i += blockDim.x) {
+    const int key = cell_key(C, i);
+    C.cellOf[i] = key;
+    if (key >= 0) atomicAdd(&cnt[key], 1);
+  }
+  __syncthreads();
+  const int per = (nkeys + blockDim.x - 1) / blockDim.x;
+  const int b = min(nkeys, (int)threadIdx.x * per), e = min(nkeys, b + per);
+  int s = 0;
+  for (int k = b; k < e; k++) s += cnt[k];
+  int total;
+  int run = block_scan(s, warpSums, total);
+  for (int k = b; k < e; k++) {
+    const int c = cnt[k];
+    cnt[k] = run;
+    C.cellStart[k] = run;
+    run += c;
+  }
+  if (threadIdx.x == 0) C.cellStart[nkeys] = total;
+  __syncthreads();
+  for (int i = threadIdx.x; i < C.n_atoms; i += blockDim.x) {
+    const int key = C.cellOf[i];
+    if (key >= 0) C.cellAtoms[atomicAdd(&cnt[key], 1)] = i;
+  }
+  __syncthreads();  // cnt[key] is now the end of the key's atoms
+  for (int i = threadIdx.x; i < C.n_atoms; i += blockDim.x) {
+    const int key = C.cellOf[i];
+    if (key < 0) continue;
+    const int kb = key > 0 ? cnt[key - 1] : 0, ke = cnt[key];
+    int rank = 0;
+    for (int j = kb; j < ke; j++) rank += C.cellAtoms[j] < i;
+    place_record(C, kb + rank, i);
+  }
+}
+
+cudaError_t cells_launch(const CellBuild& C, cudaStream_t st, int* launched) {
+  const int nkeys = C.ncell[0] * C.ncell[1] * C.ncell[2] * (C.ntypes > 0 ? C.ntypes : 1);
+  // One CTA where its serial work is short (a round of 1,024 atoms takes about
+  // 1 us and 1,024 keys 0.5 us) and the counts fit shared memory.
+  if (C.ntypes > 0 && C.n_atoms <= 8192 && nkeys <= 32768) {
+    const size_t smem = sizeof(int) * (size_t)(nkeys + 1);
+    cudaError_t e = cudaFuncSetAttribute(cell_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cell_list_kernel<<<1, 1024, smem, st>>>(C, nkeys);
+    *launched += 1;
+    return cudaGetLastError();
+  }
+  cudaError_t e = cudaMemsetAsync(C.count, 0, sizeof(int) * 2 * ((size_t)nkeys + 1), st);
+  if (e != cudaSuccess) return e;
   const int blocks = max(1, min(1184, (C.n_atoms + 255) / 256));
   cell_count_kernel<<<blocks, 256, 0, st>>>(C);
-  cell_scan_kernel<<<1, 1024, 0, st>>>(C.count, ncellTotal, C.cellStart);
-  cell_scatter_kernel<<<blocks, 256, 0, st>>>(C);
-  // cellOf (n_atoms entries) is free after the scatter and serves as the sort's scratch.
-  cell_sort_kernel<<<max(1, min(2048, (ncellTotal + 7) / 8)), 256, 0, st>>>(C.cellStart, ncellTotal, C.cellAtoms,
-                                                                         C.cellOf);
+  cell_scan_kernel<<<1, 1024, 0, st>>>(C.count, nkeys, C.cellStart);
+  cell_scatter_kernel<<<blocks, 256, 0, st>>>(C, C.count + nkeys + 1);
+  cell_sort_kernel<<<max(1, min(2048, (nkeys + 7) / 8)), 256, 0, st>>>(C, nkeys);
+  *launched += 4;
   return cudaGetLastError();
 }
 
