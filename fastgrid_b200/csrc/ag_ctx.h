@@ -72,6 +72,8 @@ struct ag_ctx {
   int tile[3] = {2, 8, 16};   // e-map CTA tile in work items (x chunks of 8 points, y rows, z planes)
   int warpCompact = 2;        // e-map item order: 0 rows, 1 warp-compact, 2 warp-compact with x-interleaved lane pairs
   int itemsCompact = -1;      // the order hItems was built with
+  bool itemsDense = false;    // ... and whether cut into full CTAs
+  double atomLo[3] = {0, 0, 0}, atomHi[3] = {0, 0, 0};  // extent of the staged atoms
   bool itemsOnDevice = false; // items / blocks hold hItems / hBlocks
   std::vector<double> epsHost;  // the staged 332/eps table (FP64), empty for the constant dielectric
   std::vector<double> atomsHost;  // host copy of the staged atoms (x, y, z, w), read back on demand
@@ -111,7 +113,8 @@ struct ag_ctx {
   std::vector<float> solparProbe, volProbe;
   int emapMode = agk::kEmapKahan;
   float rNear = 11.25f;
-  float rNode = 27.0f;              // AG_TUNE_EMAP_NODE_RADIUS (0: no node sums)
+  static constexpr float kNodeRadius = 27.0f;
+  float rNode = kNodeRadius;        // AG_TUNE_EMAP_NODE_RADIUS (0: no node sums)
   bool smoothTail = false;          // the staged dielectric table is AutoGrid's function
   float delta = 2.0e-3f;
   int packedTable = 1;              // AG_TUNE_EMAP_PACKED_TABLE

@@ -418,19 +418,38 @@ void makeItems(const ag_grid& g, const int tile[3], int warpCompact, bool dense,
   blocks.resize(nb);
 }
 
+// Whether the direct e-map's CTAs are cut densely and no node sums are formed:
+// where they could not take a fair share of the atoms, that is where no atom is 1.5 (default) node
+// radii from a grid point along any axis (2,000 atoms on 61^3 points: 0.334 ms dense,
+// 0.367 ms with a CTA per tile; 1,017 atoms on 150^3: 1.23 and 1.00 ms).
+bool denseItems(const ag_ctx* c) {
+  if (c->ddd && !c->smoothTail) return true;  // no node sums
+  const ag_grid& g = c->grid;
+  const int n[3] = {g.nx, g.ny, g.nz};
+  const double radius = std::max<double>(std::max(c->rNear, c->ddd ? ag_ctx::kNodeRadius : 0.f), 9.5 * 7.5 * g.spacing);
+  for (int d = 0; d < 3; d++) {
+    const double lo = -(n[d] / 2) * g.spacing, hi = (n[d] - 1 - n[d] / 2) * g.spacing;
+    if (std::max(c->atomHi[d] - lo, hi - c->atomLo[d]) >= 1.5 * radius) return false;
+  }
+  return true;
+}
+
 void buildItems(ag_ctx* c) {
   const ag_grid& g = c->grid;
+  const int tile = c->tile[0] * 10000 + c->tile[1] * 100 + c->tile[2];
+  const bool dense = denseItems(c);
   if (c->itemsFor[0] == g.nx && c->itemsFor[1] == g.ny && c->itemsFor[2] == g.nz && c->itemsH == g.spacing &&
-      c->itemsTile == c->tile[0] * 10000 + c->tile[1] * 100 + c->tile[2] && c->itemsCompact == c->warpCompact)
+      c->itemsTile == tile && c->itemsCompact == c->warpCompact && c->itemsDense == dense)
     return;
-  makeItems(g, c->tile, c->warpCompact, false, c->hItems, c->hBlocks);
+  makeItems(g, c->tile, c->warpCompact, dense, c->hItems, c->hBlocks);
   c->itemsOnDevice = false;
   c->itemsCompact = c->warpCompact;
+  c->itemsDense = dense;
   c->itemsFor[0] = g.nx;
   c->itemsFor[1] = g.ny;
   c->itemsFor[2] = g.nz;
   c->itemsH = g.spacing;
-  c->itemsTile = c->tile[0] * 10000 + c->tile[1] * 100 + c->tile[2];
+  c->itemsTile = tile;
 }
 
 // 16- and 8-bit copies of the FP32 table's saturating tail.  With g = t[n-1]
@@ -527,9 +546,17 @@ int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const doub
       if (!std::isfinite(xyzw[i])) return fail(AG_E_INVALID, "non-finite atom coordinate or weight at atom %lld", (long long)(i / 4));
     c->wSum = 0;
     c->wAbsSum = 0;
+    for (int d = 0; d < 3; d++) {
+      c->atomLo[d] = DBL_MAX;
+      c->atomHi[d] = -DBL_MAX;
+    }
     for (int i = 0; i < n; i++) {
       c->wSum += xyzw[4 * (size_t)i + 3];
       c->wAbsSum += std::fabs(xyzw[4 * (size_t)i + 3]);
+      for (int d = 0; d < 3; d++) {
+        c->atomLo[d] = std::min(c->atomLo[d], xyzw[4 * (size_t)i + d]);
+        c->atomHi[d] = std::max(c->atomHi[d], xyzw[4 * (size_t)i + d]);
+      }
     }
     CK(c->atoms.ensure(n));
     if (n) CK(cudaMemcpyAsync(c->atoms.p, xyzw, sizeof(double) * 4 * n, cudaMemcpyHostToDevice, c->stream));
@@ -566,19 +593,22 @@ int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const doub
 }
 
 // Atoms per CTA when the grid alone does not give every SM enough waves of
-// resident CTAs to even out their unequal costs: whole 256-atom tiles (a tile
-// costs its barriers and its latency however few atoms it holds), half tiles
-// only where whole ones would not give every SM three CTAs.  With CTAs for 16 per SM 8,000
-// atoms on 101^3 points took 2.45 ms and with 6 per SM 2.63 ms.
+// resident CTAs to even out their unequal costs (with CTAs for 16 per SM 8,000
+// atoms on 101^3 points took 2.45 ms, with 6 per SM 2.63 ms).  Whole 256-atom
+// tiles, since a tile costs its barriers and its latency however few atoms it
+// holds; two at least where the grid gives every SM two waves of CTAs or nearly
+// (a CTA's set-up is worth about 100 atoms: 1,017 atoms on 125 x 101 x 120
+// points took 1.39 ms in quarters and 1.26 ms in halves, copies included); half
+// tiles where whole ones would not give every SM three CTAs.
 int emapChunk(int nAtoms, int nblocks, int sms, int ctasPerSm) {
   const int want = 2 * sms * ctasPerSm;
   if (nblocks >= want) return std::max(nAtoms, 1);
+  if ((int64_t)nblocks * ((nAtoms + 255) / 256) < 3 * sms) return 128;
   const int ns = (want + nblocks - 1) / nblocks;
-  int chunk = std::max(256, nAtoms / ns / 256 * 256);
+  int chunk = std::max(nblocks >= 5 * sms ? 512 : 256, nAtoms / ns / 256 * 256);
   const int parts = (nAtoms + chunk - 1) / chunk;
   if (parts > 1 && nAtoms - (parts - 1) * chunk < chunk / 4)  // no split of a few atoms
     chunk = ((nAtoms + parts - 2) / (parts - 1) + 255) / 256 * 256;
-  if (chunk == 256 && (int64_t)nblocks * ((nAtoms + 255) / 256) < 3 * sms) return 128;
   return chunk;
 }
 
@@ -603,8 +633,9 @@ int buildEmapParams(ag_ctx* c, float* dOut, bool allowSplit, agk::EmapParams& P)
   // Node sums: the smooth dielectric leaves out the 0.01 A steps of the table,
   // which matter up to rNode; the constant dielectric has none.  Near atoms
   // (the cap of 1/r, compensated terms) are never summed at the nodes.
-  P.rnodeMin = (c->rNode > 0.f && (!c->ddd || c->smoothTail)) ? 100.f * std::max(c->rNear, c->ddd ? c->rNode : 0.f)
-                                                              : INFINITY;
+  P.rnodeMin = (c->rNode > 0.f && (!c->ddd || c->smoothTail) && !c->itemsDense)
+                   ? 100.f * std::max(c->rNear, c->ddd ? c->rNode : 0.f)
+                   : INFINITY;
   if (c->ddd && c->packedTable && c->pkVecs > 0) {
     P.packed = c->epsPacked.p;
     P.packedVecs = c->pkVecs;

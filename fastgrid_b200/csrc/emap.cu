@@ -429,7 +429,8 @@ __device__ __forceinline__ void near_exact(const EmapSmem& S, const EmapParams& 
 
 // One work unit: CTA box `blk` of job P against atom split `split`.  Called
 // once per CTA by emap_kernel, and repeatedly by the persistent batch kernel.
-template <bool DDD, int MODE>
+// NODES: far atoms are summed at the box's nodes (else rnodeMin is infinite).
+template <bool DDD, int MODE, bool NODES>
 __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, const int split, EmapSmem& S) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const EmapBlock B = P.blocks[blk];
@@ -439,6 +440,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
 
   // This thread's points, in the CTA-local frame scaled by 100.
   const bool active = tid < B.nitems;
+  const bool busy = warp * 32 < B.nitems;  // a warp without items only helps with the atom handling and the nodes
   int xc = 0, iy = 0, iz = 0;
   const int item = P.items[B.item0 + (active ? tid : 0)];
   unpack_item(item, xc, iy, iz);
@@ -459,11 +461,11 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
   for (int k = 0; k < kNX / 2; k++) gxn[k] = make_float2(-gx[2 * k], -gx[2 * k + 1]);
 
   // Atoms this far (0.01 A) from the box are summed at its nodes.
-  const float rnode = MODE == kEmapKahan ? fmaxf(B.rnode, P.rnodeMin) : __int_as_float(0x7F800000);
+  const float rnode = NODES ? fmaxf(B.rnode, P.rnodeMin) : __int_as_float(0x7F800000);
   // Mid-list bins may pass the table's end (not if the node atoms begin before).
   const bool clampMid = B.clampMid && !(rnode + 2.f * sqrtf(B.hx * B.hx + B.hy * B.hy + B.hz * B.hz) < 8100.f);
   int nodeTotal = 0;  // node atoms seen so far (uniform)
-  S.nodeAcc[tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (NODES) S.nodeAcc[tid] = make_float4(0.f, 0.f, 0.f, 0.f);
 
   // Packed tail tables for this box: only when no bin can pass the table's end.
   const bool pk = DDD && P.packed != nullptr && !clampMid;
@@ -559,7 +561,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
       const float dx = fmaxf(fabsf(loc.x) - B.hx, 0.f), dy = fmaxf(fabsf(loc.y) - B.hy, 0.f),
                   dz = fmaxf(fabsf(loc.z) - B.hz, 0.f);
       const float d2 = dx * dx + dy * dy + dz * dz;
-      if (d2 >= rnode * rnode) {
+      if (NODES && d2 >= rnode * rnode) {
         cls = kClsNode;
         loc.w *= gFar;
       } else if (d2 < P.rnear2) {
@@ -590,7 +592,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
     const unsigned lt = (1u << lane) - 1u;
     unsigned myBallot = 0;
 #pragma unroll
-    for (int c = 0; c < kNumCls; c++) {
+    for (int c = NODES ? kClsNode : kClsNear; c < kNumCls; c++) {
       const unsigned b = __ballot_sync(0xffffffffu, cls == c);
       if (cls == c) myBallot = b;
       if (lane == 0) S.cnt[c][warp] = __popc(b);
@@ -600,7 +602,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
     int base[kNumCls];
     int run = 0, myPos = 0, nodeCnt = 0;
 #pragma unroll
-    for (int c = 0; c < kNumCls; c++) {
+    for (int c = NODES ? kClsNode : kClsNear; c < kNumCls; c++) {
       base[c] = run;
       int off = 0;
 #pragma unroll
@@ -615,8 +617,8 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
         run = (run + 1) & ~1;
       }
     }
-    const int nNode = base[kClsNear];
-    if (cls == kClsNode) {
+    const int nNode = NODES ? base[kClsNear] : 0;
+    if (NODES && cls == kClsNode) {
       float* pr = reinterpret_cast<float*>(S.list) + 8 * (myPos >> 1) + (myPos & 1);
       pr[0] = loc.x;
       pr[2] = loc.y;
@@ -629,7 +631,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
         S.nearMask[myPos] = (unsigned short)nearBits;
       }
     }
-    if (tid == 0 && (nodeCnt & 1)) {
+    if (NODES && tid == 0 && (nodeCnt & 1)) {
       // An odd last pair is completed by an atom of no weight far away.
       float* pr = reinterpret_cast<float*>(S.list) + 8 * (nodeCnt >> 1) + 1;
       pr[0] = 1.0e7f;
@@ -638,13 +640,13 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
       pr[6] = 0.f;
     }
     __syncthreads();
-    if (nNode > 0) {
+    if (NODES && nNode > 0) {
       node_atoms<DDD>(S, nNode >> 1, B.hx, B.hy, B.hz);
       nodeTotal += nNode;
     }
 
     // Mid atoms: table read, or a packed tail table.
-    if (DDD) {
+    if (DDD && busy) {
       const uint32_t tabBiased = smem_u32(S.tab) - 0x2C000000u;
       const int nMid = base[kClsMid16] - base[kClsMid];
       if (clampMid)
@@ -662,7 +664,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
     }
 
     // Far atoms: saturated dielectric (or the constant dielectric), no table.
-    const int nFar = run - base[kClsFar];
+    const int nFar = busy ? run - base[kClsFar] : 0;
     const float4* farA = S.list + base[kClsFar];
 #pragma unroll 1
     for (int j0 = 0; j0 < nFar; j0 += kChunk) {
@@ -688,7 +690,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
 
     // Near atoms: clamp 1/r at 2 and decide bins near an edge exactly.
 #pragma unroll 1
-    for (int j = base[kClsNear]; j < base[kClsMid]; j++) {
+    for (int j = busy ? base[kClsNear] : base[kClsMid]; j < base[kClsMid]; j++) {
       const float4 a = S.list[j];
       const float dy = a.y - gy, dz = a.z - gz;
       // The 1e-30 keeps r2 > 0 (an atom on a grid point) without a per-point max.
@@ -741,7 +743,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
 
   // The node atoms' part: their sums at the nodes, interpolated to the points.
   float fld[kNX] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (nodeTotal > 0) {
+  if (NODES && nodeTotal > 0) {
     float* F = reinterpret_cast<float*>(S.list);
     if (tid < kNodes) {
       double f = 0.0;
@@ -772,11 +774,11 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
   }
 }
 
-template <bool DDD, int MODE>
+template <bool DDD, int MODE, bool NODES>
 __global__ void __launch_bounds__(kThreads, kEmapCtasPerSm) emap_kernel(const __grid_constant__ EmapParams P) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   EmapSmem& S = *reinterpret_cast<EmapSmem*>(smem_raw);
-  emap_unit<DDD, MODE>(P, blockIdx.x % P.nblocks, blockIdx.x / P.nblocks, S);
+  emap_unit<DDD, MODE, NODES>(P, blockIdx.x % P.nblocks, blockIdx.x / P.nblocks, S);
 }
 
 // Persistent kernel over the work units of many jobs (a batch of receptors):
@@ -796,7 +798,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     const int u = S.unit;
     if (u >= nunits) return;
     const int2 w = units[u];
-    emap_unit<true, MODE>(jobs[w.x], w.y, 0, S);
+    emap_unit<true, MODE, MODE == kEmapKahan>(jobs[w.x], w.y, 0, S);
   }
 }
 
@@ -831,7 +833,7 @@ __global__ void __launch_bounds__(kThreads, kEmapCtasPerSm)
       if (threadIdx.x == 0) atomicOr(P.status, ST_BAD_INPUT);
       continue;
     }
-    emap_unit<true, MODE>(P, blk, 0, S);
+    emap_unit<true, MODE, MODE == kEmapKahan>(P, blk, 0, S);
   }
 }
 
@@ -861,16 +863,21 @@ size_t emap_smem_bytes() { return sizeof(EmapSmem); }
 cudaError_t emap_launch(const EmapParams& P, bool ddd, int mode, int grid, cudaStream_t st) {
   const size_t smem = sizeof(EmapSmem);
   cudaError_t e = cudaSuccess;
-#define AG_LAUNCH(D, M)                                                                               \
-  do {                                                                                                \
-    e = cudaFuncSetAttribute(emap_kernel<D, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    if (e != cudaSuccess) return e;                                                                   \
-    emap_kernel<D, M><<<grid, kThreads, smem, st>>>(P);                                               \
+#define AG_LAUNCH(D, M, N)                                                                                  \
+  do {                                                                                                      \
+    e = cudaFuncSetAttribute(emap_kernel<D, M, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    if (e != cudaSuccess) return e;                                                                         \
+    emap_kernel<D, M, N><<<grid, kThreads, smem, st>>>(P);                                                  \
   } while (0)
-  if (ddd) {
-    if (mode == kEmapKahan) AG_LAUNCH(true, kEmapKahan); else AG_LAUNCH(true, kEmapPlain);
+  // Without node sums a kernel without their code: small grids, whose CTAs see
+  // one or two tiles each, took 5-8 % longer with it.
+  const bool nodes = mode == kEmapKahan && P.rnodeMin < 1.0e30f;
+  if (mode != kEmapKahan) {
+    if (ddd) AG_LAUNCH(true, kEmapPlain, false); else AG_LAUNCH(false, kEmapPlain, false);
+  } else if (nodes) {
+    if (ddd) AG_LAUNCH(true, kEmapKahan, true); else AG_LAUNCH(false, kEmapKahan, true);
   } else {
-    if (mode == kEmapKahan) AG_LAUNCH(false, kEmapKahan); else AG_LAUNCH(false, kEmapPlain);
+    if (ddd) AG_LAUNCH(true, kEmapKahan, false); else AG_LAUNCH(false, kEmapKahan, false);
   }
 #undef AG_LAUNCH
   e = cudaGetLastError();
