@@ -117,6 +117,8 @@ cudaError_t surr_conv_tc_launch(int layer, int epi, const ConvArgs& A, const uin
 // Training: loss = mean (o - y / sOut)^2; dO8[p] = (2 (o - y/sOut) / n, 0 x 7) in BF16.
 cudaError_t surr_loss_launch(const float* o, const float* y, int64_t n, float invSOut, uint4* do8, double* loss,
                              cudaStream_t st);
+// FP32 features (two float4 per point) rounded to BF16 (nearest, ties to even).
+cudaError_t surr_round_launch(const float4* featF, int64_t n, uint4* feat, cudaStream_t st);
 cudaError_t surr_adam_launch(float* w, float* m, float* v, const float* g, int n, float lr, float b1, float b2,
                              float eps, int step, cudaStream_t st);
 // y = a - b (FP32), and the sums of squares of y and of each feature channel (FP64, 9 values).

@@ -11,9 +11,11 @@
 // copies, two-slot ring, bounded mbarrier waits).  The atoms of those tiles
 // within rcut of the CTA box are gathered into one near batch (FP32 local
 // coordinates plus the FP64 record for exact bin decisions), which the CTA
-// then sums behind a single barrier; each warp skips the atoms farther than
-// rcut from its own 32 work items' box.  Terms are summed in plain FP32 over
-// chunks of 16 atoms, the chunk sums Kahan-compensated.
+// then sums behind a single barrier; each warp first lists the atoms within
+// rcut of its own 32 work items' box (testing every atom of the batch in the
+// pair loop instead took 4.74 ms per surrogate e-map on 161^3 against 4.63).
+// Terms are summed in plain FP32 over chunks of 16 atoms, the chunk sums
+// Kahan-compensated.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -31,7 +33,7 @@ constexpr int kThreads = 256;
 constexpr int kTile = 256;
 constexpr int kTabLen = 8192;
 constexpr int kListCap = 1024;    // tiles listed per round (262,144 atoms)
-constexpr int kNearCap = 1024;    // near batch capacity (atoms)
+constexpr int kNearCap = 768;     // near batch capacity (atoms)
 constexpr int kChunk = 16;        // atoms per plain-FP32 chunk sum
 
 struct NearSmem {
@@ -39,6 +41,7 @@ struct NearSmem {
   double4 ring[2][kTile];
   float4 nearA[kNearCap];         // CTA-local x, y, z scaled by 100 and 100 w
   double4 nearD[kNearCap];        // the FP64 record, for exact bin decisions
+  unsigned short wlist[kThreads / 32][kNearCap];  // per warp: batch atoms within rcut of its points' box
   int cnt[kThreads / 32];
   int tileList[kListCap];
   uint64_t bar[2];
@@ -71,7 +74,7 @@ __device__ __forceinline__ float lo_hi(const float2& v, int k) { return (k & 1) 
 // pairs (x0, x1), (x2, x3), ... go through Blackwell's packed FP32
 // instructions (add/mul/fma .f32x2, each half rounded as the scalar one).
 // gxn holds minus the thread's x coordinates in those pairs.
-__device__ __forceinline__ void near_batch(const NearSmem& S, const EmapParams& P, int n,
+__device__ __forceinline__ void near_batch(NearSmem& S, const EmapParams& P, int n,
                                            const float2 (&gxn)[kNX / 2], float gy, float gz, int xc, int iy, int iz,
                                            const float (&wlo)[3], const float (&whi)[3], float (&sum)[kNX],
                                            float (&cmp)[kNX]) {
@@ -83,21 +86,34 @@ __device__ __forceinline__ void near_batch(const NearSmem& S, const EmapParams& 
   const float warpCut2 = rcut2 * 1.0001f;
   const uint32_t tabBiased = smem_u32(S.tab) - 0x2C000000u;  // address(tab) - 4 * bits(2^23)
   const double h = P.h;
+  // This warp's atoms: those within rcut of its points' box.
+  const int lane = threadIdx.x & 31;
+  unsigned short* wl = S.wlist[threadIdx.x >> 5];
+  int nw = 0;
+  for (int base = 0; base < n; base += 32) {
+    bool keep = false;
+    if (base + lane < n) {
+      const float4 a = S.nearA[base + lane];
+      const float ex = fmaxf(fmaxf(wlo[0] - a.x, a.x - whi[0]), 0.f);
+      const float ey = fmaxf(fmaxf(wlo[1] - a.y, a.y - whi[1]), 0.f);
+      const float ez = fmaxf(fmaxf(wlo[2] - a.z, a.z - whi[2]), 0.f);
+      keep = fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < warpCut2;
+    }
+    const unsigned b = __ballot_sync(0xffffffffu, keep);
+    if (keep) wl[nw + __popc(b & ((1u << lane) - 1u))] = (unsigned short)(base + lane);
+    nw += __popc(b);
+  }
+  __syncwarp();
 #pragma unroll 1
-  for (int j0 = 0; j0 < n; j0 += kChunk) {
+  for (int j0 = 0; j0 < nw; j0 += kChunk) {
     float2 cs[kNX / 2];
 #pragma unroll
     for (int k = 0; k < kNX / 2; k++) cs[k] = make_float2(0.f, 0.f);
-    const int j1 = min(n, j0 + kChunk);
+    const int j1 = min(nw, j0 + kChunk);
 #pragma unroll 1
-    for (int j = j0; j < j1; j++) {
+    for (int jj = j0; jj < j1; jj++) {
+      const int j = wl[jj];
       const float4 a = S.nearA[j];
-      {  // skip atoms beyond rcut of every point of this warp (warp-uniform)
-        const float ex = fmaxf(fmaxf(wlo[0] - a.x, a.x - whi[0]), 0.f);
-        const float ey = fmaxf(fmaxf(wlo[1] - a.y, a.y - whi[1]), 0.f);
-        const float ez = fmaxf(fmaxf(wlo[2] - a.z, a.z - whi[2]), 0.f);
-        if (fmaf(ex, ex, fmaf(ey, ey, ez * ez)) >= warpCut2) continue;
-      }
       const float dy = a.y - gy, dz = a.z - gz;
       // The 1e-30 keeps r2 > 0 (an atom on a grid point) without a per-point max.
       const float2 dyz2 = dup2(fmaf(dz, dz, dy * dy) + 1e-30f);

@@ -567,6 +567,23 @@ __global__ void surr_loss_kernel(const float* __restrict__ o, const float* __res
   }
 }
 
+// BF16 bits of v, rounded to nearest even (infinities and NaN payloads cut).
+__device__ __forceinline__ uint32_t bf16_bits(float v) {
+  uint32_t b = __float_as_uint(v);
+  if ((b & 0x7F800000u) != 0x7F800000u) b += 0x7FFFu + ((b >> 16) & 1u);
+  return b >> 16;
+}
+
+// The caller's FP32 features as the network's BF16 input.  The host used to
+// round them: 0.8 ms of the 2.0 ms of a pass over 300,000 points.
+__global__ void surr_round_kernel(const float4* __restrict__ featF, int64_t n, uint4* __restrict__ feat) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const float4 a = featF[2 * i], b = featF[2 * i + 1];
+    feat[i] = make_uint4(bf16_bits(a.x) | bf16_bits(a.y) << 16, bf16_bits(a.z) | bf16_bits(a.w) << 16,
+                         bf16_bits(b.x) | bf16_bits(b.y) << 16, bf16_bits(b.z) | bf16_bits(b.w) << 16);
+  }
+}
+
 __global__ void surr_adam_kernel(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
                                  const float* __restrict__ g, int n, float lr, float b1, float b2, float eps, float bc1,
                                  float bc2) {
@@ -784,6 +801,11 @@ cudaError_t surr_pack_launch(const float* w, const PackedWeights& pw, cudaStream
 cudaError_t surr_loss_launch(const float* o, const float* y, int64_t n, float invSOut, uint4* do8, double* loss,
                              cudaStream_t st) {
   surr_loss_kernel<<<592, 256, 0, st>>>(o, y, n, invSOut, (float)(2.0 / (double)n), do8, loss);
+  return cudaGetLastError();
+}
+
+cudaError_t surr_round_launch(const float4* featF, int64_t n, uint4* feat, cudaStream_t st) {
+  surr_round_kernel<<<592, 256, 0, st>>>(featF, n, feat);
   return cudaGetLastError();
 }
 

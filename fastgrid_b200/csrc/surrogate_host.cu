@@ -32,7 +32,7 @@ struct SurrState {
   DevBuf<uint16_t> wtc1, wtc2, wtc3;  // tcgen05 layouts
   bool useTc = true;                  // inference convolutions on tcgen05 (mma.sync when false)
   DevBuf<double> cPartial, field, tab64, loss, sums;
-  DevBuf<float4> rec;
+  DevBuf<float4> rec, featF;
   DevBuf<uint4> feat, do8;
   DevBuf<uint16_t> a1, a2, dz1, dz2;
   DevBuf<int> flags, list, count, counter;
@@ -55,6 +55,7 @@ struct SurrState {
     for (auto* b : {&wk1, &wk2, &wk3, &wk2t, &wk3t, &a1, &a2, &dz1, &dz2, &wtc1, &wtc2, &wtc3}) b->release();
     for (auto* b : {&cPartial, &field, &tab64, &loss, &sums}) b->release();
     rec.release();
+    featF.release();
     feat.release();
     do8.release();
     for (auto* b : {&flags, &list, &count, &counter, &dItems}) b->release();
@@ -758,19 +759,10 @@ extern "C" int ag_surrogate_net_grad(ag_ctx* c, const ag_grid* g, const float* f
   if (int e = ensureNet(S, np)) return e;
   if (target)
     if (int e = ensureTrain(S, np)) return e;
-  std::vector<uint4> f(np);
-  for (int64_t i = 0; i < np; i++) {
-    uint32_t w[4];
-    for (int k = 0; k < 4; k++) {
-      const float lo = bf16Round(features[8 * i + 2 * k]), hi = bf16Round(features[8 * i + 2 * k + 1]);
-      uint32_t a, b;
-      memcpy(&a, &lo, 4);
-      memcpy(&b, &hi, 4);
-      w[k] = (a >> 16) | (b & 0xFFFF0000u);
-    }
-    f[i] = make_uint4(w[0], w[1], w[2], w[3]);
-  }
-  CK(cudaMemcpyAsync(S.feat.p, f.data(), sizeof(uint4) * np, cudaMemcpyHostToDevice, c->stream));
+  CK(S.featF.ensure(2 * (size_t)np));
+  CK(cudaMemcpyAsync(S.featF.p, features, sizeof(float) * 8 * np, cudaMemcpyHostToDevice, c->stream));
+  CK(agk::surr_round_launch(S.featF.p, np, S.feat.p, c->stream));
+  c->launches += 1;
   agk::SurrGeom G{};
   G.nx = g->nx;
   G.ny = g->ny;
