@@ -41,6 +41,49 @@ struct DevBuf {
   }
 };
 
+// An array inside a device buffer that something else owns.
+template <class T>
+struct DevView {
+  T* p = nullptr;
+};
+
+// Page-locked staging memory for the inputs of one kind of call: they are
+// written here and go to the device in one asynchronous copy.  begin() waits
+// until the last copy out of it is done and makes room.
+struct Staging {
+  unsigned char* p = nullptr;
+  size_t cap = 0;
+  cudaEvent_t done = nullptr;
+  bool inFlight = false;
+  cudaError_t begin(size_t bytes) {
+    cudaError_t e = cudaSuccess;
+    if (!done) e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+    if (e == cudaSuccess && inFlight) e = cudaEventSynchronize(done);
+    inFlight = false;
+    if (e != cudaSuccess || bytes <= cap) return e;
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    cap = 0;
+    const size_t want = bytes + bytes / 4;  // room for a somewhat larger next job
+    e = cudaHostAlloc((void**)&p, want, cudaHostAllocDefault);
+    if (e == cudaSuccess) cap = want;
+    return e;
+  }
+  cudaError_t copy(void* dst, size_t bytes, cudaStream_t st) {
+    cudaError_t e = bytes ? cudaMemcpyAsync(dst, p, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
+    if (e == cudaSuccess) e = cudaEventRecord(done, st);
+    inFlight = e == cudaSuccess;
+    return e;
+  }
+  void release() {
+    if (done) cudaEventDestroy(done);
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    done = nullptr;
+    cap = 0;
+  }
+};
+
 const std::vector<double>& binThresholds();
 // The same table written into thr[0 .. 8192], without allocating.
 void emapBinThresholdsInto(double* thr);
@@ -57,7 +100,9 @@ struct ag_ctx {
   int64_t launches = 0;
   // e-map
   agc::DevBuf<double4> atoms;
-  agc::DevBuf<float> epsTab;
+  agc::Staging epsStage, affStage;    // staging memory of the table and of the affinity inputs
+  agc::DevBuf<float> epsBuf;          // epsTab, then epsPacked
+  agc::DevView<float> epsTab;
   agc::DevBuf<double> thr;
   agc::DevBuf<int> items;
   agc::DevBuf<agk::EmapBlock> blocks;
@@ -80,14 +125,18 @@ struct ag_ctx {
   uint64_t atomsVersion = 0;      // bumped whenever new atoms are staged
   uint64_t atomsHostVersion = ~0ull;  // the staging atomsHost holds
   // affinity
-  agc::DevBuf<int> info, cellStart, cellAtoms, cellOf, count, dStart, dAtoms, donorMask, closestH;
+  agc::DevBuf<int> cellStart, cellAtoms, cellOf, count, dStart, dAtoms, closestH;
   agc::DevBuf<int> ctStart, ctAtoms;  // type-major cell list of the two-point kernel, with the sorted records
   agc::DevBuf<double4> ctXyz;
   agc::DevBuf<float4> ctAux;
   int affKernel = 2;                  // affinity kernel: 2 two-point (default), 1 one point per thread
-  agc::DevBuf<float> vol, solq, affTab, affRaw, sol;
-  agc::DevBuf<float4> rv8;            // per atom: rvector, 0, rvector2, 0
-  agc::DevBuf<double> rv64, thrA;
+  agc::DevBuf<float> affTab;
+  agc::DevBuf<unsigned char> affIn;   // the staged affinity inputs:
+  agc::DevView<double> rv64;
+  agc::DevView<float4> rv8;           // per atom: rvector, 0, rvector2, 0
+  agc::DevView<int> info;
+  agc::DevView<float> vol, solq, sol, affRaw;
+  agc::DevBuf<double> thrA;
   struct Pass {
     int m0, nm, nmPad;
     size_t tabOff, rowsOff, classOff, slotOff;  // in affTab: one-point rows; two-point rows, class rows, slot planes
@@ -118,7 +167,7 @@ struct ag_ctx {
   bool smoothTail = false;          // the staged dielectric table is AutoGrid's function
   float delta = 2.0e-3f;
   int packedTable = 1;              // AG_TUNE_EMAP_PACKED_TABLE
-  agc::DevBuf<uint4> epsPacked;     // 16- and 8-bit copies of the staged table's saturating tail
+  agc::DevView<uint4> epsPacked;    // 16- and 8-bit copies of the staged table's saturating tail
   int pkVecs = 0, pkVec8 = 0, pkB16 = 8192, pkB8 = 8192;  // pkVecs == 0: no packed table
   float pkScale = 0;
   int ctasPerSm = 8;                // AG_TUNE_EMAP_CTAS_PER_SM

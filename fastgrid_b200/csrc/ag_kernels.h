@@ -142,11 +142,11 @@ struct CellBuild {
   int* count;                     // 2 * (keys + 1) scratch
   int* cellStart;                 // keys + 1
   int* cellAtoms;                 // n_atoms
-  const int* donorMask;           // optional: only atoms with mask[i] != 0 (null = all)
+  int donorsOnly;                 // only H donors (by their info bits)
   // Type-major list of the two-point affinity kernel (ntypes > 0): key = type *
   // cells + cell, and the atoms' records copied into sorted order.
   int ntypes;
-  const int* info;                // type in the low five bits
+  const int* info;                // type | hbond << 5 | ...
   const float *vol, *solq;
   double4* sXyz;
   float4* sAux;                   // vol, solq, info bits, atom index bits

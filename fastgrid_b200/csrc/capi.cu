@@ -145,23 +145,23 @@ extern "C" int ag_ctx_destroy(ag_ctx* c) {
   if (!c) return AG_OK;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
-  for (auto* b : {&c->epsTab, &c->maps, &c->vol, &c->solq, &c->affTab, &c->affRaw, &c->sol})
-    b->release();
-  c->rv8.release();
+  for (auto* b : {&c->epsBuf, &c->maps, &c->affTab}) b->release();
+  c->affIn.release();
+  c->epsStage.release();
+  c->affStage.release();
   c->ctXyz.release();
   c->ctAux.release();
   c->atoms.release();
   c->thr.release();
   c->partial.release();
-  c->rv64.release();
   c->thrA.release();
   c->checksum.release();
   agc::surrFree(c->surr);
   c->surr = nullptr;
   c->blocks.release();
   c->status.release();
-  for (auto* b : {&c->items, &c->info, &c->cellStart, &c->cellAtoms, &c->cellOf, &c->count, &c->dStart,
-                  &c->dAtoms, &c->donorMask, &c->closestH, &c->ctStart, &c->ctAtoms})
+  for (auto* b : {&c->items, &c->cellStart, &c->cellAtoms, &c->cellOf, &c->count, &c->dStart,
+                  &c->dAtoms, &c->closestH, &c->ctStart, &c->ctAtoms})
     b->release();
   if (c->stream) cudaStreamDestroy(c->stream);
   if (c->copyStream) cudaStreamDestroy(c->copyStream);
@@ -525,15 +525,6 @@ bool tableIsSmooth(const float* t, int n) {
   return true;
 }
 
-// The same, into 16-byte vectors (empty: no usable tail).
-std::vector<uint4> packTableTail(const std::vector<float>& t, int& b16, int& b8, int& vec8, float& kScale) {
-  std::vector<uint4> out(agk::kEmapPackedBytes / 16);
-  const int bytes = packTableTailInto(t.data(), (int)t.size(), reinterpret_cast<unsigned char*>(out.data()),
-                                      agk::kEmapPackedBytes, b16, b8, vec8, kScale);
-  out.resize((size_t)bytes / 16);
-  return out;
-}
-
 int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const double* inv_eps, bool deviceInputs) {
   if (int r = checkGrid(g)) return r;
   if (n < 0 || (n > 0 && !xyzw)) return fail(AG_E_INVALID, "bad atom array");
@@ -565,18 +556,19 @@ int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const doub
   c->epsHost.clear();
   if (c->ddd) {
     c->epsHost.assign(inv_eps, inv_eps + 8192);
-    std::vector<float> t(8192);
+    // The FP32 table and its packed tail, one copy.
+    const size_t tabBytes = sizeof(float) * 8192;
+    CK(c->epsStage.begin(tabBytes + agk::kEmapPackedBytes));
+    float* t = reinterpret_cast<float*>(c->epsStage.p);
     for (int i = 0; i < 8192; i++) t[i] = (float)inv_eps[i];
-    CK(c->epsTab.ensure(8192));
-    CK(cudaMemcpyAsync(c->epsTab.p, t.data(), sizeof(float) * 8192, cudaMemcpyHostToDevice, c->stream));
-    c->smoothTail = tableIsSmooth(t.data(), 8192);
-    const std::vector<uint4> pk = packTableTail(t, c->pkB16, c->pkB8, c->pkVec8, c->pkScale);
-    c->pkVecs = (int)pk.size();
-    if (!pk.empty()) {
-      CK(c->epsPacked.ensure(pk.size()));
-      CK(cudaMemcpyAsync(c->epsPacked.p, pk.data(), sizeof(uint4) * pk.size(), cudaMemcpyHostToDevice, c->stream));
-    }
-    CK(cudaStreamSynchronize(c->stream));
+    c->smoothTail = tableIsSmooth(t, 8192);
+    const int pkBytes = packTableTailInto(t, 8192, c->epsStage.p + tabBytes, agk::kEmapPackedBytes, c->pkB16, c->pkB8,
+                                          c->pkVec8, c->pkScale);
+    c->pkVecs = pkBytes / 16;
+    CK(c->epsBuf.ensure(8192 + agk::kEmapPackedBytes / sizeof(float)));
+    c->epsTab.p = c->epsBuf.p;
+    c->epsPacked.p = reinterpret_cast<uint4*>(c->epsBuf.p + 8192);
+    CK(c->epsStage.copy(c->epsBuf.p, tabBytes + pkBytes, c->stream));
   }
   buildItems(c);
   if (!c->itemsOnDevice) {  // the work items and CTA boxes depend on the grid only
@@ -793,13 +785,23 @@ int stageAffinity(ag_ctx* c, const ag_receptor* r, const ag_affinity_params* p) 
   const int n = r->n_atoms;
   if (p->n_maps < 0 || p->n_maps > ag::kMaxAtomTypes) return fail(AG_E_INVALID, "n_maps %d outside 0..14", p->n_maps);
   if (p->n_types < 1 || p->n_types > ag::kNumAllTypes) return fail(AG_E_INVALID, "n_types %d outside 1..32", p->n_types);
-  std::vector<int> info(n), donor(n);
-  std::vector<float> vol(n), solq(n);
+  // All inputs in one block of staging memory, and one copy: FP64 and FP32 bond
+  // vectors, the atoms' info bits, volumes and solvation parameters, the pair
+  // energies and the desolvation values.
+  const int nm = p->n_maps, nt = p->n_types;
+  const size_t nRaw = (size_t)nt * agk::kAffRows * nm;
+  const size_t offRv8 = (sizeof(double) * 3 * (size_t)n + 15) / 16 * 16, offInfo = offRv8 + sizeof(float4) * 2 * (size_t)n;
+  const size_t offVol = offInfo + sizeof(int) * (size_t)n, offSolq = offVol + sizeof(float) * (size_t)n;
+  const size_t offRaw = offSolq + sizeof(float) * (size_t)n, offSol = offRaw + sizeof(float) * nRaw;
+  const size_t inBytes = offSol + sizeof(float) * agk::kAffRows;
+  CK(c->affStage.begin(inBytes));
+  unsigned char* in = c->affStage.p;
+  int* info = reinterpret_cast<int*>(in + offInfo);
+  float *vol = reinterpret_cast<float*>(in + offVol), *solq = reinterpret_cast<float*>(in + offSolq);
   for (int i = 0; i < n; i++) {
     if (r->type[i] < 0 || r->type[i] >= p->n_types) return fail(AG_E_INVALID, "atom %d has type %d outside 0..%d", i, r->type[i], p->n_types - 1);
     if (r->hbond[i] < 0 || r->hbond[i] > 5) return fail(AG_E_INVALID, "atom %d has H-bond class %d", i, r->hbond[i]);
     info[i] = r->type[i] | (r->hbond[i] << 5) | ((r->disorder[i] ? 1 : 0) << 8) | ((r->rexp[i] & 7) << 9);
-    donor[i] = (r->hbond[i] == ag::DS || r->hbond[i] == ag::D1) ? 1 : 0;
     vol[i] = (float)r->vol[i];
     solq[i] = (float)(r->solpar[i] + p->solpar_q * fabs(r->charge[i]));
   }
@@ -812,22 +814,13 @@ int stageAffinity(ag_ctx* c, const ag_receptor* r, const ag_affinity_params* p) 
       return fail(AG_E_INVALID, "atoms of receptor type %d have different H-bond classes", r->type[i]);
   }
   for (int t = 0; t < agk::kMaxTypes; t++) if (c->typeHbond[t] < 0) c->typeHbond[t] = ag::NON;
-  std::vector<float4> rv8(2 * (size_t)n);
+  float4* rv8 = reinterpret_cast<float4*>(in + offRv8);
   for (size_t i = 0; i < (size_t)n; i++) {
     const double *a = r->rvector + 3 * i, *b = r->rvector2 + 3 * i;
     rv8[2 * i] = make_float4((float)a[0], (float)a[1], (float)a[2], 0.f);
     rv8[2 * i + 1] = make_float4((float)b[0], (float)b[1], (float)b[2], 0.f);
   }
-  CK(c->info.ensure(n)); CK(c->donorMask.ensure(n)); CK(c->vol.ensure(n)); CK(c->solq.ensure(n));
-  CK(c->rv8.ensure(2 * (size_t)n)); CK(c->rv64.ensure(3 * (size_t)n));
-  if (n) {
-    CK(cudaMemcpyAsync(c->info.p, info.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->donorMask.p, donor.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->vol.p, vol.data(), sizeof(float) * n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->solq.p, solq.data(), sizeof(float) * n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->rv8.p, rv8.data(), sizeof(float4) * 2 * n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->rv64.p, r->rvector, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
-  }
+  if (n) memcpy(in, r->rvector, sizeof(double) * 3 * (size_t)n);
   c->nMaps = p->n_maps;
   c->nTypes = p->n_types;
   c->hydrogen = p->hydrogen;
@@ -840,7 +833,6 @@ int stageAffinity(ag_ctx* c, const ag_receptor* r, const ag_affinity_params* p) 
 
   // Split the maps into passes of at most 16 maps and 4 H-bonding ones (the
   // two-point kernel's slots), or 4 min/max maps for the one-point kernel.
-  const int nm = p->n_maps, nt = p->n_types;
   auto isMinMax = [&](int m) {
     const int hb = c->mapHbond[m];
     return c->mapIsHB[m] && !c->mapCov[m] && (hb == ag::A1 || hb == ag::DS || hb == ag::D1);
@@ -886,15 +878,15 @@ int stageAffinity(ag_ctx* c, const ag_receptor* r, const ag_affinity_params* p) 
   }
   // Pair energies, FP32, rows r <= 8 A: [type][row][map].  The kernels' tables
   // are built from them on the device (aff_tables_kernel).
-  std::vector<float> raw(std::max<size_t>((size_t)nt * agk::kAffRows * nm, 4));
+  float* raw = reinterpret_cast<float*>(in + offRaw);
   for (int t = 0; t < nt; t++) {
     const double* src = p->energy + (size_t)t * 8192 * nm;
-    float* dst = raw.data() + (size_t)t * agk::kAffRows * nm;
+    float* dst = raw + (size_t)t * agk::kAffRows * nm;
     for (int i = 0; i < agk::kAffRows * nm; i++) dst[i] = (float)src[i];
   }
   size_t tabSize = 0;
   for (auto& ps : c->passes) {
-    planPass(c, ps, raw.data());
+    planPass(c, ps, raw);
     ps.tabOff = tabSize;
     ps.rowsOff = ps.tabOff + (size_t)nt * agk::kAffRows * ps.nmPad;
     ps.classOff = ps.rowsOff + (size_t)nt * agk::kAffRows * agk::aff2_row_stride(ps.rowPad);
@@ -906,12 +898,18 @@ int stageAffinity(ag_ctx* c, const ag_receptor* r, const ag_affinity_params* p) 
     CK(c->thrA.ensure(thr.size()));
     CK(cudaMemcpyAsync(c->thrA.p, thr.data(), sizeof(double) * thr.size(), cudaMemcpyHostToDevice, c->stream));
   }
-  std::vector<float> sol(agk::kAffRows);
+  float* sol = reinterpret_cast<float*>(in + offSol);
   for (int i = 0; i < agk::kAffRows; i++) sol[i] = (float)p->sol[i];
-  CK(c->affTab.ensure(tabSize)); CK(c->affRaw.ensure(raw.size())); CK(c->sol.ensure(sol.size()));
-  CK(cudaMemcpyAsync(c->affRaw.p, raw.data(), sizeof(float) * raw.size(), cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(c->sol.p, sol.data(), sizeof(float) * sol.size(), cudaMemcpyHostToDevice, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  CK(c->affTab.ensure(tabSize));
+  CK(c->affIn.ensure(inBytes));
+  c->rv64.p = reinterpret_cast<double*>(c->affIn.p);
+  c->rv8.p = reinterpret_cast<float4*>(c->affIn.p + offRv8);
+  c->info.p = reinterpret_cast<int*>(c->affIn.p + offInfo);
+  c->vol.p = reinterpret_cast<float*>(c->affIn.p + offVol);
+  c->solq.p = reinterpret_cast<float*>(c->affIn.p + offSolq);
+  c->affRaw.p = reinterpret_cast<float*>(c->affIn.p + offRaw);
+  c->sol.p = reinterpret_cast<float*>(c->affIn.p + offSol);
+  CK(c->affStage.copy(c->affIn.p, inBytes, c->stream));
   for (const auto& ps : c->passes) {
     agk::AffTableJob J{};
     J.energy = c->affRaw.p;
@@ -982,7 +980,7 @@ int prepAffinity(ag_ctx* c, cudaStream_t st) {
     CK(c->ctStart.ensure(nkeys + 1)); CK(c->count.ensure(2 * (nkeys + 1)));
     CK(c->ctAtoms.ensure(n)); CK(c->cellOf.ensure(n)); CK(c->ctXyz.ensure(n)); CK(c->ctAux.ensure(n));
     C.cellOf = c->cellOf.p; C.count = c->count.p;
-    C.cellStart = c->ctStart.p; C.cellAtoms = c->ctAtoms.p; C.donorMask = nullptr;
+    C.cellStart = c->ctStart.p; C.cellAtoms = c->ctAtoms.p;
     C.ntypes = c->nTypes; C.info = c->info.p; C.vol = c->vol.p; C.solq = c->solq.p;
     C.sXyz = c->ctXyz.p; C.sAux = c->ctAux.p;
     CK(agk::cells_launch(C, st, &launched));
@@ -998,9 +996,9 @@ int prepAffinity(ag_ctx* c, cudaStream_t st) {
   CK(c->dStart.ensure(ncellT + 1)); CK(c->dAtoms.ensure(n));
   CK(c->closestH.ensure(np));
   C.cellOf = c->cellOf.p; C.count = c->count.p;
-  C.cellStart = c->cellStart.p; C.cellAtoms = c->cellAtoms.p; C.donorMask = nullptr;
+  C.cellStart = c->cellStart.p; C.cellAtoms = c->cellAtoms.p;
   CK(agk::cells_launch(C, st, &launched));
-  C.cellStart = c->dStart.p; C.cellAtoms = c->dAtoms.p; C.donorMask = c->donorMask.p;
+  C.cellStart = c->dStart.p; C.cellAtoms = c->dAtoms.p; C.info = c->info.p; C.donorsOnly = 1;
   CK(agk::cells_launch(C, st, &launched));
   c->launches += launched;
   agk::ClosestHParams H{};
@@ -1191,10 +1189,16 @@ int runAffinityChunked(ag_ctx* c, float* host, int nchunks) {
 }
 
 int checkStatus(ag_ctx* c) {
+  // The status word and the checksum's partial sums in one round trip.
+  std::vector<double> cs(1 + (size_t)c->checksumSplits);
   unsigned st = 0;
   CK(cudaMemcpyAsync(&st, c->status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+  if (c->checksumSplits > 0)
+    CK(cudaMemcpyAsync(cs.data(), c->checksum.p, sizeof(double) * c->checksumSplits, cudaMemcpyDeviceToHost,
+                       c->stream));
   CK(cudaStreamSynchronize(c->stream));
   if (st) {
+    c->checksumSplits = 0;
     cudaMemsetAsync(c->status.p, 0, sizeof(unsigned), c->stream);
     cudaStreamSynchronize(c->stream);
     return fail(AG_E_DEVICE, "a kernel reported error status 0x%x (1 = bounded wait expired, 2 = bad input)", st);
@@ -1202,11 +1206,8 @@ int checkStatus(ag_ctx* c) {
   // Net-charge checksum of the last e-map: the FP64 sum of the weights the
   // kernel consumed must equal the host's sum of the input weights.
   if (c->checksumSplits > 0) {
-    std::vector<double> cs(c->checksumSplits);
-    CK(cudaMemcpyAsync(cs.data(), c->checksum.p, sizeof(double) * cs.size(), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
     double s = 0.0;
-    for (double v : cs) s += v;
+    for (int k = 0; k < c->checksumSplits; k++) s += cs[k];
     c->checksumSplits = 0;
     c->lastChecksum = s;
     const double want = c->wSum + c->testChecksumOffset;
@@ -1229,6 +1230,7 @@ extern "C" int ag_upload(ag_ctx* c, const ag_grid* g, const ag_receptor* r, cons
     if (int e = stageAffinity(c, r, p)) return e;
   CK(c->maps.ensure((size_t)(c->nMaps + 2) * c->npoints()));
   CK(cudaMemsetAsync(c->status.p, 0, sizeof(unsigned), c->stream));
+  CK(cudaStreamSynchronize(c->stream));  // the caller's arrays are no longer read (they may be page-locked)
   c->haveJob = true;
   return AG_OK;
 }

@@ -26,7 +26,7 @@ __device__ __forceinline__ double rsq_exact_c(double ax, double ay, double az, d
 // file order inside each key.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int cell_key(const CellBuild& C, int i) {
-  if (C.donorMask && !C.donorMask[i]) return -1;
+  if (C.donorsOnly && ((C.info[i] >> 5) & 7) != 1 && ((C.info[i] >> 5) & 7) != 2) return -1;  // DS, D1
   const double4 a = C.xyz[i];
   const int cx = (int)floor((a.x - C.lo[0]) / C.edge), cy = (int)floor((a.y - C.lo[1]) / C.edge),
             cz = (int)floor((a.z - C.lo[2]) / C.edge);
