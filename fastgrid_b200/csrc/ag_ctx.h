@@ -161,8 +161,11 @@ struct ag_ctx {
   std::vector<int> mapHbond, mapIsHB, mapCov;
   std::vector<float> solparProbe, volProbe;
   int emapMode = agk::kEmapKahan;
-  float rNear = 11.25f;
-  static constexpr float kNodeRadius = 27.0f;
+  float rNear = 0.f;                // AG_TUNE_EMAP_RNEAR (0: the default, which nearRadius() gives)
+  // 11.75 A where atoms beyond the node radius are taken without the table's
+  // steps: the exact bins' larger share then keeps the map's error what it was.
+  float nearRadius() const { return rNear > 0.f ? rNear : ddd && !itemsDense ? 11.75f : 11.0f; }
+  static constexpr float kNodeRadius = 24.0f, kNodeHalfWidths = 8.5f, kNodeHalfWidthsConst = 9.5f;
   float rNode = kNodeRadius;        // AG_TUNE_EMAP_NODE_RADIUS (0: no node sums)
   bool smoothTail = false;          // the staged dielectric table is AutoGrid's function
   float delta = 2.0e-3f;

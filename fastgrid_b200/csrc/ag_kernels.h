@@ -22,7 +22,7 @@ struct EmapBlock {
   float hx, hy, hz;
   float rfar2;                    // (100 * rFar)^2, rFar >= 50 A
   int clampMid;                   // 1 if rFar + box diagonal can reach 81.9 A: clamp mid-list bins at 8191
-  float rnode;                    // 0.01 A: least distance at which the box's node interpolation is accurate
+  float rnode;                    // the largest half extent (0.01 A)
 };
 
 struct EmapParams {
@@ -47,7 +47,9 @@ struct EmapParams {
   int b16, b8;
   float r16sq, r8sq;              // (b16 + 2)^2, (b8 + 2)^2: mid atoms at least that far (0.01 A units) from the box
   float kScale;                   // 2^(e + 126) / g, g = table[8191] = 2^e * m: turns 100 w g 2^-16 into 100 w ulp(g) 2^133
-  float rnodeMin;                 // 0.01 A: atoms at least max(rnodeMin, EmapBlock::rnode) from the box are summed at its nodes (+inf: none)
+  // Atoms at least max(rnodeMin, rnodeHalfWidths * EmapBlock::rnode) from the box (0.01 A) are summed at its nodes.
+  float rnodeMin;                 // +inf: none
+  float rnodeHalfWidths;
   int testIdleWait;               // test hook: > 0 adds a wait of that many polls on a barrier nothing arrives on
   float* out;
   double* partial;                // nsplit * npoints, when nsplit > 1

@@ -285,9 +285,9 @@ static void emapBox(const ag_grid& g, const int* items, agk::EmapBlock& b) {
   b.rfar2 = (float)((100.0 * rFar) * (100.0 * rFar));
   b.clampMid = rFar + diag >= 81.0 ? 1 : 0;  // mid-list bins may then exceed the table
   // Interpolation from the box's nodes: with five nodes per axis the error of
-  // an atom's term is below 1.3e-6 of it (rms 3e-7) from 9.5 half-widths on,
-  // and falls with the fifth power of the distance.
-  b.rnode = 9.5f * std::max(b.hx, std::max(b.hy, b.hz));
+  // a 1/r term is below 1.5e-6 of it (rms 3e-7) from 8.5 half-widths on, and
+  // falls with the fifth power of the distance.
+  b.rnode = std::max(b.hx, std::max(b.hy, b.hz));
 }
 
 // Tiles along y and z for tiles of `w` items along x and at most T[1] x T[2]
@@ -419,17 +419,19 @@ void makeItems(const ag_grid& g, const int tile[3], int warpCompact, bool dense,
 }
 
 // Whether the direct e-map's CTAs are cut densely and no node sums are formed:
-// where they could not take a fair share of the atoms, that is where no atom is 1.5 (default) node
+// where they could not take a fair share of the atoms, that is where no atom is 1.7 (default) node
 // radii from a grid point along any axis (2,000 atoms on 61^3 points: 0.334 ms dense,
 // 0.367 ms with a CTA per tile; 1,017 atoms on 150^3: 1.23 and 1.00 ms).
 bool denseItems(const ag_ctx* c) {
   if (c->ddd && !c->smoothTail) return true;  // no node sums
   const ag_grid& g = c->grid;
   const int n[3] = {g.nx, g.ny, g.nz};
-  const double radius = std::max<double>(std::max(c->rNear, c->ddd ? ag_ctx::kNodeRadius : 0.f), 9.5 * 7.5 * g.spacing);
+  const double radius = std::max<double>(
+      std::max(c->rNear > 0.f ? c->rNear : 11.f, c->ddd ? ag_ctx::kNodeRadius : 0.f),
+      (c->ddd ? ag_ctx::kNodeHalfWidths : ag_ctx::kNodeHalfWidthsConst) * 7.5 * g.spacing);
   for (int d = 0; d < 3; d++) {
     const double lo = -(n[d] / 2) * g.spacing, hi = (n[d] - 1 - n[d] / 2) * g.spacing;
-    if (std::max(c->atomHi[d] - lo, hi - c->atomLo[d]) >= 1.5 * radius) return false;
+    if (std::max(c->atomHi[d] - lo, hi - c->atomLo[d]) >= 1.7 * radius) return false;
   }
   return true;
 }
@@ -620,13 +622,17 @@ int buildEmapParams(ag_ctx* c, float* dOut, bool allowSplit, agk::EmapParams& P)
   P.h = c->grid.spacing;
   P.table = c->epsTab.p;
   P.thr = c->thr.p;
-  P.rnear2 = (100.f * c->rNear) * (100.f * c->rNear);
+  P.rnear2 = (100.f * c->nearRadius()) * (100.f * c->nearRadius());
   P.delta = c->delta;
   // Node sums: the smooth dielectric leaves out the 0.01 A steps of the table,
-  // which matter up to rNode; the constant dielectric has none.  Near atoms
+  // which matter up to rNode (24 A with exact bins to 11.75 A: 1.74e-7 relative
+  // error on 20,000 atoms and 161^3 points, 10.6 ms; 27 A and 11.25 A: 1.80e-7,
+  // 11.7 ms; no node sums, 11 A: 1.87e-7, 29.5 ms).  The constant dielectric
+  // has no steps and takes the interpolation's own error lower instead.  Near atoms
   // (the cap of 1/r, compensated terms) are never summed at the nodes.
+  P.rnodeHalfWidths = c->ddd ? ag_ctx::kNodeHalfWidths : ag_ctx::kNodeHalfWidthsConst;
   P.rnodeMin = (c->rNode > 0.f && (!c->ddd || c->smoothTail) && !c->itemsDense)
-                   ? 100.f * std::max(c->rNear, c->ddd ? c->rNode : 0.f)
+                   ? 100.f * std::max(c->nearRadius(), c->ddd ? c->rNode : 0.f)
                    : INFINITY;
   if (c->ddd && c->packedTable && c->pkVecs > 0) {
     P.packed = c->epsPacked.p;

@@ -38,7 +38,7 @@
 //    100 w 2^-16 (g + k_b ulp(g)) = 100 w 2^-16 invEps[b] from it.
 //    Mid and far terms are summed in plain FP32 over chunks of kChunk atoms
 //    and the chunk sums are Kahan-compensated.
-//  * Atoms at least R from the box (27 A; more for boxes wider than 5.7 A) do
+//  * Atoms at least R from the box (24 A; more for boxes wider than 5.6 A) do
 //    not enter point by point: their sum is a smooth function over the box,
 //    so it is formed at 5 x 5 x 5 Chebyshev nodes of the box and interpolated
 //    to the box's 2,048 points at the end (node_atoms, node_field).
@@ -461,7 +461,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
   for (int k = 0; k < kNX / 2; k++) gxn[k] = make_float2(-gx[2 * k], -gx[2 * k + 1]);
 
   // Atoms this far (0.01 A) from the box are summed at its nodes.
-  const float rnode = NODES ? fmaxf(B.rnode, P.rnodeMin) : __int_as_float(0x7F800000);
+  const float rnode = NODES ? fmaxf(P.rnodeHalfWidths * B.rnode, P.rnodeMin) : __int_as_float(0x7F800000);
   // Mid-list bins may pass the table's end (not if the node atoms begin before).
   const bool clampMid = B.clampMid && !(rnode + 2.f * sqrtf(B.hx * B.hx + B.hy * B.hy + B.hz * B.hz) < 8100.f);
   int nodeTotal = 0;  // node atoms seen so far (uniform)

@@ -290,6 +290,7 @@ extern "C" int ag_emap_noalloc(const ag_grid* grid, int n_atoms, const double* d
   P.thr = D.thr;
   P.rnear2 = (100.f * kNaNear) * (100.f * kNaNear);
   P.delta = 2.0e-3f;
+  P.rnodeHalfWidths = 9.5f;
   P.rnodeMin = smooth ? 100.f * (d_inv_eps ? kNaNode : kNaNear) : INFINITY;
   P.out = d_out;
   P.status = D.status;

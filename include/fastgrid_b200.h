@@ -90,7 +90,8 @@ int64_t ag_ctx_launch_count(const ag_ctx* ctx);
 /* Tuning knobs of a context (no reference counterpart; the reference's
  * --cuda-* switches played this role for its kernels).  Results stay within
  * the stated tolerances for every allowed value. */
-#define AG_TUNE_EMAP_RNEAR 1          /* A, >= 8: atoms nearer the CTA box take the exact-bin path (default 11.25) */
+#define AG_TUNE_EMAP_RNEAR 1          /* A, >= 8: atoms nearer the CTA box take the exact-bin path (default 11,
+                                         11.75 where far atoms are summed at interpolation nodes) */
 #define AG_TUNE_EMAP_PACKED_TABLE 2   /* 0/1: mid atoms in the table's saturating tail (from about 22 A) read 16- and 8-bit copies of it (1, default) or the FP32 table (0) */
 #define AG_TUNE_EMAP_CTAS_PER_SM 3    /* 1..8: half the CTAs per SM the atom split aims for on small grids (default 8) */
 #define AG_TUNE_EMAP_WARP_COMPACT 4   /* e-map item order: 0 rows, 1 each warp's items form a compact box, 2 as 1 with
@@ -103,8 +104,8 @@ int64_t ag_ctx_launch_count(const ag_ctx* ctx);
                                          than 4 H-bond maps) */
 #define AG_TUNE_CONCURRENT_PASSES 10 /* 0/1: a map set's e-map and affinity pass run concurrently, the e-map on a
                                          high-priority stream (1, default), or one after the other (0) */
-#define AG_TUNE_EMAP_NODE_RADIUS 11   /* A, >= 24 (default 27): atoms this far from a CTA box (further for boxes wider
-                                         than 5.7 A) are summed at the box's 125 interpolation nodes; 0: point by point */
+#define AG_TUNE_EMAP_NODE_RADIUS 11   /* A, >= 24 (default 24): atoms this far from a CTA box (further for boxes wider
+                                         than 5.6 A) are summed at the box's 125 interpolation nodes; 0: point by point */
 /* Failure-detection test hooks (default 0 = off).  IDLE_WAIT: 1..64 polls of an
  * extra wait, after each direct e-map CTA's first atom tile has landed, on a
  * barrier nothing arrives on; the wait expires, the kernel records it in its
