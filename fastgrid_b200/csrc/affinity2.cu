@@ -144,9 +144,10 @@ __device__ __forceinline__ float acos_clamped(float f) { return (f > 1.f) ? 0.f 
 
 // A thread's two points (p = 0, 1 at z and z + 1).
 struct Pts {
-  float px, py, pz[2];
+  float px, py;
+  float2 npz;                        // minus their z; 1e4 for a point past the grid edge: candidates have z >= -8 A,
+                                     // so it is beyond every cutoff
   int ix, iy, iz0;
-  bool valid[2];
 };
 
 // Their plain sums.
@@ -166,53 +167,51 @@ struct SlotSums {
 // FP64 grid-point coordinate as the reference forms it.
 __device__ __forceinline__ double gcoord(int i, int n2, double h) { return __dmul_rn((double)(i - n2), h); }
 
+constexpr uint32_t kBiasBits = 0x4B000000u;  // bits of 2^23
+
 // One candidate against the two points: offsets, 1 / r, table row and whether
-// the point is within the 8 A cutoff.  Returns false if it is for no lane.
+// the point is within the 8 A cutoff.  Packed FP32 over the two points.
+// Returns false if the candidate is for no lane.
 struct Pair {
-  float dx, dy, dz[2], rs[2];
-  int iR[2];                         // table row; kAffRows (the zero row) beyond the cutoff
+  float dx, dy;
+  float2 dz, rs;
+  uint32_t row[2];                   // kBiasBits + table row; row kAffRows (all zero) beyond the cutoff
   bool in[2];
   __device__ __forceinline__ bool set(const Aff2Params& P, const int* idx, const int c, const float4 a, const Pts& q) {
     dx = a.x - q.px;
     dy = a.y - q.py;
-    const float dxy = fmaf(dy, dy, dx * dx);
-    float r2[2];
-#pragma unroll
-    for (int p = 0; p < 2; p++) {
-      dz[p] = a.z - q.pz[p];
-      r2[p] = fmaf(dz[p], dz[p], dxy);
-      in[p] = q.valid[p] && r2[p] <= 64.0002f;
-    }
+    // The 1e-30 keeps r^2 > 0 (an atom on a grid point).
+    const float dxy = fmaf(dy, dy, dx * dx) + 1.0e-30f;
+    dz = __fadd2_rn(make_float2(a.z, a.z), q.npz);
+    const float2 r2 = __ffma2_rn(dz, dz, make_float2(dxy, dxy));
+    in[0] = r2.x <= 64.0002f;
+    in[1] = r2.y <= 64.0002f;
     if (!__any_sync(0xffffffffu, in[0] || in[1])) return false;
-    // Exact 8 A cutoff near the edge.
+    rs = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
+    const float2 rs100 = __fmul2_rn(rs, make_float2(100.f, 100.f)), bias = make_float2(kBias, kBias);
+    const float2 kf = __ffma2_rd(r2, rs100, bias);   // 2^23 + floor(100 r)
+    const float2 kn = __ffma2_rn(r2, rs100, bias);   // 2^23 + the integer nearest 100 r
+    const float2 d = __ffma2_rn(r2, rs100, __ffma2_rn(kn, make_float2(-1.f, -1.f), bias));  // 100 r minus it
+    const float2 t = __fadd2_rn(r2, make_float2(-64.f, -64.f));
+    uint32_t b[2] = {__float_as_uint(kf.x), __float_as_uint(kf.y)};
+    // Within the guard band of a bin edge or of the cutoff: the reference's
+    // FP64 decisions (its bin int(100 / (1 / sqrt(r^2))) through the table of
+    // r^2 thresholds).
+    if (min(fabsf(d.x), fabsf(d.y)) < P.delta || min(fabsf(t.x), fabsf(t.y)) < 2.0e-4f) {
+      const double4 a64 = P.xyz[idx[c]];
 #pragma unroll
-    for (int p = 0; p < 2; p++)
-      if (in[p] && r2[p] > 63.9998f) {
-        const double4 a64 = P.xyz[idx[c]];
-        if (rsq64(a64.x, a64.y, a64.z, gcoord(q.ix, P.n2x, P.h), gcoord(q.iy, P.n2y, P.h),
-                  gcoord(q.iz0 + p, P.n2z, P.h)) > 64.0)
-          in[p] = false;
-      }
-#pragma unroll
-    for (int p = 0; p < 2; p++) {
-      const float r2c = fmaxf(r2[p], 1.0e-24f);
-      rs[p] = rsqrt_approx(r2c);
-      const float rs100 = rs[p] * 100.f;
-      const float T = r2c * rs100;
-      const float kf = __fmaf_rd(r2c, rs100, kBias);   // 2^23 + floor(100 r) in the low bits
-      int b = __float_as_int(kf) - 0x4B000000;
-      const float fr = T - (kf - kBias);
-      if (in[p] && fabsf(fr - 0.5f) > 0.5f - P.delta) {
-        // Within the guard band of a bin edge: the reference's FP64 bin
-        // int(100 / (1 / sqrt(r^2))) through the table of r^2 thresholds.
-        const int k = min(fr > 0.5f ? b + 1 : b, kAffRows);
-        const double4 a64 = P.xyz[idx[c]];
+      for (int p = 0; p < 2; p++) {
+        const float dp = p ? d.y : d.x, tp = p ? t.y : t.x;
+        if (!in[p] || !(fabsf(dp) < P.delta || fabsf(tp) < 2.0e-4f)) continue;
         const double r64 = rsq64(a64.x, a64.y, a64.z, gcoord(q.ix, P.n2x, P.h), gcoord(q.iy, P.n2y, P.h),
                                  gcoord(q.iz0 + p, P.n2z, P.h));
-        b = (r64 >= P.thr[k]) ? k : k - 1;
+        if (r64 > 64.0) in[p] = false;
+        const int k = min((int)(__float_as_uint(p ? kn.y : kn.x) - kBiasBits), kAffRows);
+        if (fabsf(dp) < P.delta) b[p] = kBiasBits + (uint32_t)(k == 0 ? 0 : r64 >= P.thr[k] ? k : k - 1);
       }
-      iR[p] = in[p] ? min(max(b, 0), kAffRows - 1) : kAffRows;
     }
+#pragma unroll
+    for (int p = 0; p < 2; p++) row[p] = in[p] ? b[p] : kBiasBits + kAffRows;
     return true;
   }
 };
@@ -236,7 +235,9 @@ __device__ __forceinline__ void plain_sums(const Aff2Params& P, const A2Smem<PAR
                                            const int rowQ, const int j0, const int j1, const unsigned short* wl,
                                            const Pts& q, PlainSums<NMAX>& s) {
   const int strideQ = row_stride(rowQ);
-  const float4* tab4 = reinterpret_cast<const float4*>(tab);
+  // Shared-window address of the row with bits kBiasBits + row: the bias is in
+  // the base (mod 2^32).
+  const uint32_t stride = 16u * (uint32_t)strideQ, base = smem_u32(tab) - kBiasBits * stride;
   // The next candidate's record is read one iteration ahead (its shared-memory
   // latency overlaps the current candidate's arithmetic).
   int cNext = j0 < j1 ? wl[j0] : 0;
@@ -251,12 +252,16 @@ __device__ __forceinline__ void plain_sums(const Aff2Params& P, const A2Smem<PAR
     Pair w;
     if (skipped<ISH>(a) || !w.set(P, S.idx, c, a, q)) continue;  // uniform: one candidate
     float solv[2] = {0.f, 0.f};
+    const uint32_t at[2] = {base + w.row[0] * stride, base + w.row[1] * stride};
 #pragma unroll
     for (int g4 = 0; g4 < NMAX / 4; g4++) {
       if (g4 >= rowQ) break;         // uniform
 #pragma unroll
       for (int p = 0; p < 2; p++) {
-        const float4 e4 = tab4[w.iR[p] * strideQ + g4];
+        float4 e4;
+        asm("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+            : "=f"(e4.x), "=f"(e4.y), "=f"(e4.z), "=f"(e4.w)
+            : "r"(at[p] + 16u * g4));
         s.em[p][2 * g4] = __fadd2_rn(s.em[p][2 * g4], make_float2(e4.x, e4.y));
         s.em[p][2 * g4 + 1] = __fadd2_rn(s.em[p][2 * g4 + 1], make_float2(e4.z, e4.w));
         solv[p] = e4.w;
@@ -318,7 +323,8 @@ __device__ __forceinline__ void slot_terms(const Aff2Params& P, const A2Smem<PAR
 #pragma unroll
       for (int p = 0; p < 2; p++) {
         if (!w.in[p]) continue;
-        const float ux = w.dx * w.rs[p], uy = w.dy * w.rs[p], uz = w.dz[p] * w.rs[p];
+        const float rsp = p ? w.rs.y : w.rs.x;
+        const float ux = w.dx * rsp, uy = w.dy * rsp, uz = (p ? w.dz.y : w.dz.x) * rsp;
         float cosT = -(ux * ra.x + uy * ra.y + uz * ra.z);
         bool gt0 = cosT > 0.f, ge0 = cosT >= 0.f;
         if ((ANG == A2_D1 || (ANG == A2_A2 && !dis)) && fabsf(cosT) < 1.0e-5f) {
@@ -388,11 +394,12 @@ __device__ __forceinline__ void slot_terms(const Aff2Params& P, const A2Smem<PAR
 #pragma unroll
       for (int p = 0; p < 2; p++) {
         if (!w.in[p]) continue;
-        const float E = tab[k * kPlaneRows + w.iR[p]];
+        const int iR = (int)(w.row[p] - kBiasBits);
+        const float E = tab[k * kPlaneRows + iR];
         const float rsph = fminf(fmaxf(E * 0.01f, 0.f), 1.f);
         if (kind == A2_SLOT_ACC) {
           // Disordered donors take the "HD" type's row 1.1 A in.
-          const float e = dis ? (P.planeH ? __ldg(P.planeH + k * kPlaneRows + max(0, w.iR[p] - 110)) : 0.f) : E;
+          const float e = dis ? (P.planeH ? __ldg(P.planeH + k * kPlaneRows + max(0, iR - 110)) : 0.f) : E;
           s.mn[p][k] += e * hramp[p] * (racc[p] + (1.f - racc[p]) * rsph);
         } else {
           const float f = (kind == A2_SLOT_A1) ? racc[p] : rdon[p];
@@ -554,7 +561,7 @@ __device__ __forceinline__ void scan_donors(const Aff2Params& P, const A2Smem<PA
     const float dxy = fmaf(dy, dy, dx * dx);
 #pragma unroll
     for (int p = 0; p < 2; p++) {
-      const float dz = a.z - q.pz[p];
+      const float dz = a.z + (p ? q.npz.y : q.npz.x);
       lim[p] = fminf(lim[p], fmaf(dz, dz, dxy));
     }
   }
@@ -566,8 +573,8 @@ __device__ __forceinline__ void scan_donors(const Aff2Params& P, const A2Smem<PA
     const float dxy = fmaf(dy, dy, dx * dx);
 #pragma unroll
     for (int p = 0; p < 2; p++) {
-      const float dz = a.z - q.pz[p];
-      if (q.valid[p] && fmaf(dz, dz, dxy) <= lim[p]) {
+      const float dz = a.z + (p ? q.npz.y : q.npz.x);
+      if (fmaf(dz, dz, dxy) <= lim[p]) {
         const int id = S.idx[j];
         const double4 a64 = d64[j];
         const double r64 = rsq64(a64.x, a64.y, a64.z, gcoord(q.ix, P.n2x, P.h), gcoord(q.iy, P.n2y, P.h),
@@ -669,15 +676,14 @@ __device__ __forceinline__ bool aff2_unit(const Aff2Params& P, const int cta, un
   q.ix = wx + (lane & 3);
   q.iy = wy + ((lane >> 2) & 3);
   q.iz0 = wz + (lane >> 4) * 2;
-  q.valid[0] = q.ix < P.nx && q.iy < P.ny && q.iz0 < P.nz;
-  q.valid[1] = q.ix < P.nx && q.iy < P.ny && q.iz0 + 1 < P.nz;
+  const bool valid[2] = {q.ix < P.nx && q.iy < P.ny && q.iz0 < P.nz, q.ix < P.nx && q.iy < P.ny && q.iz0 + 1 < P.nz};
   {
     const double h = P.h;
     const double ox = gcoord(x0, P.n2x, h), oy = gcoord(y0, P.n2y, h), oz = gcoord(z0, P.n2z, h);
     q.px = (float)(gcoord(q.ix, P.n2x, h) - ox);
     q.py = (float)(gcoord(q.iy, P.n2y, h) - oy);
-    q.pz[0] = (float)(gcoord(q.iz0, P.n2z, h) - oz);
-    q.pz[1] = (float)(gcoord(q.iz0 + 1, P.n2z, h) - oz);
+    q.npz.x = valid[0] ? -(float)(gcoord(q.iz0, P.n2z, h) - oz) : 1.0e4f;
+    q.npz.y = valid[1] ? -(float)(gcoord(q.iz0 + 1, P.n2z, h) - oz) : 1.0e4f;
     // CTA box (FP64, grid-centred) and the cells within 8 A of it.
     if (tid == 0) {
       Box& B = S.box;
@@ -754,7 +760,7 @@ __device__ __forceinline__ bool aff2_unit(const Aff2Params& P, const int cta, un
     if (classes) expand_classes(P, s);
 #pragma unroll
     for (int p = 0; p < 2; p++) {
-      if (!q.valid[p]) continue;
+      if (!valid[p]) continue;
       const int64_t pt = ((int64_t)(q.iz0 + p) * P.ny + q.iy) * P.nx + q.ix;
 #pragma unroll
       for (int g = 0; g < NMAX; g++) {
@@ -824,7 +830,7 @@ __device__ __forceinline__ bool aff2_unit(const Aff2Params& P, const int cta, un
     if (!ok) return false;
 #pragma unroll
     for (int p = 0; p < 2; p++) {
-      if (!q.valid[p]) continue;
+      if (!valid[p]) continue;
       const int64_t pt = ((int64_t)(q.iz0 + p) * P.ny + q.iy) * P.nx + q.ix;
 #pragma unroll
       for (int k = 0; k < kA2Slots; k++) {
