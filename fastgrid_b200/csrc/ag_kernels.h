@@ -16,8 +16,11 @@ constexpr int kEmapPackedBytes = 16384;  // e-map: shared-memory region of the p
 // A CTA's work in the e-map: items [item0, item0+nitems) of the item list and
 // the CTA's box: local origin (grid-centred frame, A) and half extents
 // (scaled by 100) that contain every point of those items.
+// A CTA that is one tile names it (tileMode != 0) and forms its items itself.
 struct EmapBlock {
   int item0, nitems;
+  short x0, x1, y0, y1, z0, z1;   // tile: items x in [x0, x1) (8 points each), rows y, planes z
+  int tileMode;                   // 0: items from the list; 1 rows, 2 warp-compact, 3 warp-compact and interleaved order
   double ox, oy, oz;
   float hx, hy, hz;
   float rfar2;                    // (100 * rFar)^2, rFar >= 50 A

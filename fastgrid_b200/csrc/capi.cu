@@ -248,20 +248,9 @@ int checkGrid(const ag_grid* g) {
   return AG_OK;
 }
 
-// The box of the items [b.item0, b.item0 + b.nitems).
-static void emapBox(const ag_grid& g, const int* items, agk::EmapBlock& b) {
+// The box of the grid points i0 .. i1 (inclusive).
+static void emapBox(const ag_grid& g, const int i0[3], const int i1[3], agk::EmapBlock& b) {
   const double h = g.spacing;
-  int i0[3] = {1 << 30, 1 << 30, 1 << 30}, i1[3] = {-1, -1, -1};  // grid points
-  for (int k = b.item0; k < b.item0 + b.nitems; k++) {
-    const int v = items[k];
-    const int xa = (v & 0xFF) * agk::kNX;  // (an interleaved pair's union is the same box)
-    const int p0[3] = {xa, (v >> 8) & 0x7FF, (v >> 19) & 0x7FF};
-    const int p1[3] = {std::min(g.nx, xa + agk::kNX) - 1, p0[1], p0[2]};
-    for (int d = 0; d < 3; d++) {
-      i0[d] = std::min(i0[d], p0[d]);
-      i1[d] = std::max(i1[d], p1[d]);
-    }
-  }
   const int n2[3] = {g.nx / 2, g.ny / 2, g.nz / 2};
   double o[3];
   float half[3];
@@ -331,12 +320,15 @@ static std::pair<int, int> bestSplit(int ny, int nz, const int T[3], int w, int 
 // warps skip atoms: 4.49 ms per surrogate e-map on 161^3 against 4.60 ms with
 // a CTA per tile).  Otherwise a CTA is a tile and its box stays compact, which
 // the direct e-map's node sums need: they begin 9.5 half-widths from the box.
-// Writes the items (one per 8 points of a row) and at most blockCap boxes;
-// returns the number of boxes, or -1 if there are more.  Allocates nothing.
-int makeItemsInto(const ag_grid& g, const int tile[3], int warpCompact, bool dense, int* items,
+// A CTA that is a tile forms its items itself (tile_item in emap.cu); dense ones
+// read them from the list.  Writes at most blockCap boxes and, for dense CTAs,
+// the items (one per 8 points of a row; *nitemsOut of them); returns the number
+// of boxes, or -1 if there are more.  Allocates nothing.
+int makeItemsInto(const ag_grid& g, const int tile[3], int warpCompact, bool dense, int* items, int* nitemsOut,
                   agk::EmapBlock* blocks, int blockCap) {
   const int nxc = (g.nx + agk::kNX - 1) / agk::kNX;
   int nitems = 0, nblocks = 0;
+  *nitemsOut = 0;
   const int n[3] = {nxc, g.ny, g.nz}, pts[3] = {agk::kNX, 1, 1};
   int T[3] = {tile[0], tile[1], tile[2]};
   if (!dense) {
@@ -363,14 +355,8 @@ int makeItemsInto(const ag_grid& g, const int tile[3], int warpCompact, bool den
               items[nitems++] = x | (y << 8) | (z << 19) | (il ? agk::kItemInterleaved : 0);
             }
   };
-  auto addBlock = [&](int i0, int i1) {
-    if (nblocks < blockCap) {
-      agk::EmapBlock b{};
-      b.item0 = i0;
-      b.nitems = i1 - i0;
-      emapBox(g, items, b);
-      blocks[nblocks] = b;
-    }
+  auto addBlock = [&](const agk::EmapBlock& b) {
+    if (nblocks < blockCap) blocks[nblocks] = b;
     nblocks++;
   };
   const int ntx = (nxc + T[0] - 1) / T[0];
@@ -386,7 +372,24 @@ int makeItemsInto(const ag_grid& g, const int tile[3], int warpCompact, bool den
                   std::min(g.nz, kz * T[2] + T[2]));
         }
       }
-    for (int i0 = 0; i0 < nitems; i0 += 256) addBlock(i0, std::min(nitems, i0 + 256));
+    for (int item0 = 0; item0 < nitems; item0 += 256) {
+      agk::EmapBlock b{};
+      b.item0 = item0;
+      b.nitems = std::min(256, nitems - item0);
+      int i0[3] = {1 << 30, 1 << 30, 1 << 30}, i1[3] = {-1, -1, -1};
+      for (int k = item0; k < item0 + b.nitems; k++) {
+        const int v = items[k], xa = (v & 0xFF) * agk::kNX;  // (an interleaved pair's union is the same box)
+        const int p0[3] = {xa, (v >> 8) & 0x7FF, (v >> 19) & 0x7FF};
+        const int p1[3] = {std::min(g.nx, xa + agk::kNX) - 1, p0[1], p0[2]};
+        for (int d = 0; d < 3; d++) {
+          i0[d] = std::min(i0[d], p0[d]);
+          i1[d] = std::max(i1[d], p1[d]);
+        }
+      }
+      emapBox(g, i0, i1, b);
+      addBlock(b);
+    }
+    *nitemsOut = nitems;
     return nblocks <= blockCap ? nblocks : -1;
   }
   // Rows and planes are divided evenly among the tiles; a last, narrower
@@ -395,12 +398,20 @@ int makeItemsInto(const ag_grid& g, const int tile[3], int warpCompact, bool den
   for (int kz = 0; kz < ntz; kz++)
     for (int kx = 0; kx < ntx; kx++) {
       const int x0 = kx * T[0], x1 = std::min(nxc, x0 + T[0]);
+      const int z0 = g.nz * kz / ntz, z1 = g.nz * (kz + 1) / ntz;
       const int tall[3] = {x1 - x0, std::min(g.ny, T[1] * (T[0] / (x1 - x0))), T[2]};
       const int nty = bestSplit(g.ny, g.nz, tall, x1 - x0, ntz).first;
       for (int ky = 0; ky < nty; ky++) {
-        const int i0 = nitems;
-        addTile(x0, x1, g.ny * ky / nty, g.ny * (ky + 1) / nty, g.nz * kz / ntz, g.nz * (kz + 1) / ntz);
-        addBlock(i0, nitems);
+        const int y0 = g.ny * ky / nty, y1 = g.ny * (ky + 1) / nty;
+        agk::EmapBlock b{};
+        b.nitems = (x1 - x0) * (y1 - y0) * (z1 - z0);
+        b.x0 = (short)x0; b.x1 = (short)x1;
+        b.y0 = (short)y0; b.y1 = (short)y1;
+        b.z0 = (short)z0; b.z1 = (short)z1;
+        b.tileMode = !compact ? 1 : warpCompact == 2 ? 3 : 2;
+        const int i0[3] = {x0 * agk::kNX, y0, z0}, i1[3] = {std::min(g.nx, x1 * agk::kNX) - 1, y1 - 1, z1 - 1};
+        emapBox(g, i0, i1, b);
+        addBlock(b);
       }
     }
   return nblocks <= blockCap ? nblocks : -1;
@@ -408,12 +419,14 @@ int makeItemsInto(const ag_grid& g, const int tile[3], int warpCompact, bool den
 
 void makeItems(const ag_grid& g, const int tile[3], int warpCompact, bool dense, std::vector<int>& items,
                std::vector<agk::EmapBlock>& blocks) {
-  items.resize((size_t)((g.nx + agk::kNX - 1) / agk::kNX) * g.ny * g.nz);
-  blocks.resize(items.size() / 32 + 64);
-  int nb = makeItemsInto(g, tile, warpCompact, dense, items.data(), blocks.data(), (int)blocks.size());
+  const size_t all = (size_t)((g.nx + agk::kNX - 1) / agk::kNX) * g.ny * g.nz;
+  items.resize(dense ? all : 0);
+  blocks.resize(all / 32 + 64);
+  int nitems = 0;
+  int nb = makeItemsInto(g, tile, warpCompact, dense, items.data(), &nitems, blocks.data(), (int)blocks.size());
   if (nb < 0) {  // many small tiles
-    blocks.resize(items.size());
-    nb = makeItemsInto(g, tile, warpCompact, dense, items.data(), blocks.data(), (int)blocks.size());
+    blocks.resize(all);
+    nb = makeItemsInto(g, tile, warpCompact, dense, items.data(), &nitems, blocks.data(), (int)blocks.size());
   }
   blocks.resize(nb);
 }

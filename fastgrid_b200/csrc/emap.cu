@@ -95,6 +95,24 @@ __device__ __forceinline__ void unpack_item(int v, int& xc, int& y, int& z) {
   z = (v >> 19) & 0x7FF;
 }
 
+// Item k of a CTA's tile.  Warp-compact order: blocks of 4 rows x 4 planes over
+// the tile's width, x fastest; otherwise rows, then planes.  Interleaved: the
+// two items of a pair of x columns share its points alternately (a column
+// whose partner is past the tile's end keeps its own).
+__device__ __forceinline__ int tile_item(const EmapBlock& B, int k) {
+  const int w = B.x1 - B.x0, H = B.y1 - B.y0, D = B.z1 - B.z0;
+  const int by = B.tileMode >= 2 ? 4 : H, bz = B.tileMode >= 2 ? 4 : D;
+  const int zb = k / (bz * w * H);
+  k -= zb * bz * w * H;
+  const int zn = min(bz, D - zb * bz), yb = k / (by * zn * w);
+  k -= yb * by * zn * w;
+  const int yn = min(by, H - yb * by), z = k / (yn * w);
+  k -= z * yn * w;
+  const int y = k / w, x = B.x0 + k - y * w;
+  const bool il = B.tileMode == 3 && (B.x0 & 1) == 0 && (x ^ 1) < B.x1;
+  return x | ((B.y0 + yb * by + y) << 8) | ((B.z0 + zb * bz + z) << 19) | (il ? kItemInterleaved : 0);
+}
+
 // Packed FP32 pairs: Blackwell issues one instruction for two lanes of FP32
 // arithmetic (add/mul/fma .f32x2), each half rounded exactly as the scalar
 // operation, so the pair loops below halve their FP32 instruction count
@@ -442,7 +460,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
   const bool active = tid < B.nitems;
   const bool busy = warp * 32 < B.nitems;  // a warp without items only helps with the atom handling and the nodes
   int xc = 0, iy = 0, iz = 0;
-  const int item = P.items[B.item0 + (active ? tid : 0)];
+  const int item = B.tileMode ? tile_item(B, active ? tid : 0) : P.items[B.item0 + (active ? tid : 0)];
   unpack_item(item, xc, iy, iz);
   // x of point k = xb + k * xs: NX consecutive points, or every other point of
   // the 2 NX points of an interleaved column pair.

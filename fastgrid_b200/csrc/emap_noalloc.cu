@@ -52,7 +52,7 @@ namespace agc {
 void emapBinThresholdsInto(double* thr);  // fills thr[0 .. 8192]
 bool tableIsSmooth(const float* t, int n);
 int emapChunk(int nAtoms, int nblocks, int sms, int ctasPerSm);
-int makeItemsInto(const ag_grid& g, const int tile[3], int warpCompact, bool dense, int* items,
+int makeItemsInto(const ag_grid& g, const int tile[3], int warpCompact, bool dense, int* items, int* nitemsOut,
                   agk::EmapBlock* blocks, int blockCap);
 int packTableTailInto(const float* t, int n, unsigned char* raw, int cap, int& b16, int& b8, int& vec8,
                       float& kScale);  // packed tail tables of the dielectric table
@@ -194,10 +194,10 @@ int naSetup(NaDevice& d) {
 // Work items and CTA boxes of a grid, as for the ordinary entry points (a CTA
 // per 2 x 8 x 16 tile); grids that need more boxes than there is room for are
 // cut into full CTAs instead.
-int naItems(const ag_grid& g) {
+int naItems(const ag_grid& g, int& nitems) {
   static const int kTile[3] = {2, 8, 16};
-  const int nb = agc::makeItemsInto(g, kTile, 2, false, g_hItems, g_hBlocks, kNaMaxBlocks);
-  return nb >= 0 ? nb : agc::makeItemsInto(g, kTile, 2, true, g_hItems, g_hBlocks, kNaMaxBlocks);
+  const int nb = agc::makeItemsInto(g, kTile, 2, false, g_hItems, &nitems, g_hBlocks, kNaMaxBlocks);
+  return nb >= 0 ? nb : agc::makeItemsInto(g, kTile, 2, true, g_hItems, &nitems, g_hBlocks, kNaMaxBlocks);
 }
 
 }  // namespace
@@ -223,8 +223,8 @@ extern "C" int ag_emap_noalloc(const ag_grid* grid, int n_atoms, const double* d
   NaDevice& D = g_dev[dev];
   if (int e = naSetup(D)) return e;
   cudaStream_t st = (cudaStream_t)stream;
-  const int64_t nitems = (int64_t)((grid->nx + agk::kNX - 1) / agk::kNX) * grid->ny * grid->nz;
-  const int nblocks = naItems(*grid);
+  int nitems = 0;
+  const int nblocks = naItems(*grid, nitems);
   const int64_t np = (int64_t)grid->nx * grid->ny * grid->nz;
   if (n_atoms == 0) {
     if (cudaMemsetAsync(d_out, 0, sizeof(float) * np, st) != cudaSuccess ||
@@ -242,7 +242,8 @@ extern "C" int ag_emap_noalloc(const ag_grid* grid, int n_atoms, const double* d
   chunk = std::max(chunk, ((n_atoms + nsplit - 1) / nsplit + 127) / 128 * 128);
   nsplit = std::max(1, (n_atoms + chunk - 1) / chunk);
 
-  if (cudaMemcpyAsync(D.items, g_hItems, sizeof(int) * nitems, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+  if ((nitems > 0 &&
+       cudaMemcpyAsync(D.items, g_hItems, sizeof(int) * nitems, cudaMemcpyHostToDevice, st) != cudaSuccess) ||
       cudaMemcpyAsync(D.blocks, g_hBlocks, sizeof(agk::EmapBlock) * nblocks, cudaMemcpyHostToDevice, st) !=
           cudaSuccess ||
       cudaMemsetAsync(D.status, 0, sizeof(unsigned), st) != cudaSuccess ||
