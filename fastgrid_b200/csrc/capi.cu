@@ -606,7 +606,10 @@ int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const doub
 // holds; two at least where the grid gives every SM two waves of CTAs or nearly
 // (a CTA's set-up is worth about 100 atoms: 1,017 atoms on 125 x 101 x 120
 // points took 1.39 ms in quarters and 1.26 ms in halves, copies included); half
-// tiles where whole ones would not give every SM three CTAs.
+// tiles where whole ones would not give every SM three CTAs; and at most 8,192
+// or half as many, since a CTA of more runs on for a millisecond after the
+// others (20,000 atoms on 161^3 points, whole job: 15.5 ms in two splits, 14.9
+// ms in four).
 int emapChunk(int nAtoms, int nblocks, int sms, int ctasPerSm) {
   const int want = 2 * sms * ctasPerSm;
   if (nblocks >= want) return std::max(nAtoms, 1);
@@ -616,6 +619,7 @@ int emapChunk(int nAtoms, int nblocks, int sms, int ctasPerSm) {
   const int parts = (nAtoms + chunk - 1) / chunk;
   if (parts > 1 && nAtoms - (parts - 1) * chunk < chunk / 4)  // no split of a few atoms
     chunk = ((nAtoms + parts - 2) / (parts - 1) + 255) / 256 * 256;
+  if (chunk > 8192) chunk = (chunk / 2 + 255) / 256 * 256;
   return chunk;
 }
 
@@ -1418,6 +1422,19 @@ extern "C" int ag_problem_views(const ag_problem* P, ag_grid* g, ag_receptor* r,
   return AG_OK;
 }
 
+// Copy the affinity maps and the d-map to `host` on the copy stream, after the
+// context's stream.
+static int copyAffinityMaps(ag_ctx* c, float* host) {
+  const int64_t np = c->npoints();
+  const int nm = c->nMaps;
+  CK(cudaEventRecord(c->evAff, c->stream));
+  CK(cudaStreamWaitEvent(c->copyStream, c->evAff, 0));
+  if (nm) CK(cudaMemcpyAsync(host, c->maps.p, sizeof(float) * nm * np, cudaMemcpyDeviceToHost, c->copyStream));
+  CK(cudaMemcpyAsync(host + (size_t)(nm + 1) * np, c->maps.p + (size_t)(nm + 1) * np, sizeof(float) * np,
+                     cudaMemcpyDeviceToHost, c->copyStream));
+  return AG_OK;
+}
+
 extern "C" int ag_problem_compute(ag_ctx* c, ag_problem* P) {
   if (!c || !P) return fail(AG_E_INVALID, "null argument");
   ag::Problem& p = P->p;
@@ -1457,25 +1474,25 @@ extern "C" int ag_problem_compute(ag_ctx* c, ag_problem* P) {
   }
   CK(c->ensureCopyStream());
   if (conc) {
-    // Both passes at once (as ag_compute runs them): the e-map on the
-    // high-priority stream, its 17 MB copied back as soon as it is done; the
-    // affinity pass, which fills the SMs the e-map's last wave leaves free,
-    // in z-slab chunks whose rows are copied back while later chunks run, so
-    // that little of the 184 MB of affinity maps (large configuration) is
-    // copied after the last kernel.
+    // Both passes at once.  The e-map starts as soon as its inputs are there;
+    // the affinity pass, staged on the host meanwhile, runs on the high-priority
+    // stream and takes the SMs as the e-map's CTAs end, in z-slab chunks whose
+    // rows are copied back while later chunks and the rest of the e-map run: the
+    // 184 MB of affinity maps (large configuration) are on the host before the
+    // e-map is done, and only its 17 MB are copied after the last kernel.  (6,000
+    // atoms on 93^3 points, constant dielectric: 1.41 ms, against 1.73 ms with
+    // the priorities the other way round; 2,000 atoms on 61^3: 0.65 and 0.68 ms.)
     c->nMaps = nm;
     CK(c->maps.ensure(total));
     CK(cudaMemsetAsync(c->status.p, 0, sizeof(unsigned), c->stream));
     CK(c->ensureEmapStream());
     CK(cudaEventRecord(c->evFork, c->stream));
     CK(cudaStreamWaitEvent(c->emapStream, c->evFork, 0));
-    std::swap(c->stream, c->emapStream);
     int e = runEmap(c, c->maps.p + (size_t)nm * np);
-    std::swap(c->stream, c->emapStream);
     if (e) return e;
     CK(cudaMemcpyAsync(P->pinned + (size_t)nm * np, c->maps.p + (size_t)nm * np, sizeof(float) * np,
-                       cudaMemcpyDeviceToHost, c->emapStream));
-    CK(cudaEventRecord(c->evJoin, c->emapStream));
+                       cudaMemcpyDeviceToHost, c->stream));
+    std::swap(c->stream, c->emapStream);
     e = stageAffinity(c, &r, &a);
     if (!e) {
       c->haveJob = true;
@@ -1486,22 +1503,18 @@ extern "C" int ag_problem_compute(ag_ctx* c, ag_problem* P) {
         e = runAffinityChunked(c, P->pinned, chunks);
       } else {
         e = runAffinity(c, c->maps.p, c->maps.p + (size_t)(nm + 1) * np);
-        if (!e) {
-          CK(cudaEventRecord(c->evAff, c->stream));
-          CK(cudaStreamWaitEvent(c->copyStream, c->evAff, 0));
-          if (nm) CK(cudaMemcpyAsync(P->pinned, c->maps.p, sizeof(float) * nm * np, cudaMemcpyDeviceToHost,
-                                     c->copyStream));
-          CK(cudaMemcpyAsync(P->pinned + (size_t)(nm + 1) * np, c->maps.p + (size_t)(nm + 1) * np,
-                             sizeof(float) * np, cudaMemcpyDeviceToHost, c->copyStream));
-        }
+        if (!e) e = copyAffinityMaps(c, P->pinned);
       }
     }
-    // Joined on every path: no e-map work may outlive the call.
-    CK(cudaStreamWaitEvent(c->stream, c->evJoin, 0));
-    if (e) {
+    // Joined on every path: no affinity work may outlive the call.
+    const cudaError_t je = cudaEventRecord(c->evJoin, c->stream);
+    std::swap(c->stream, c->emapStream);
+    if (je == cudaSuccess) CK(cudaStreamWaitEvent(c->stream, c->evJoin, 0));
+    if (e || je != cudaSuccess) {
+      cudaStreamSynchronize(c->emapStream);
       cudaStreamSynchronize(c->stream);
       cudaStreamSynchronize(c->copyStream);
-      return e;
+      return e ? e : fail(AG_E_CUDA, "event record failed: %s", cudaGetErrorString(je));
     }
   } else {
     // Affinity, d-map and covalent maps first; their copy to the host then
@@ -1513,11 +1526,7 @@ extern "C" int ag_problem_compute(ag_ctx* c, ag_problem* P) {
                                 p.covHalfWidthSquaredInv, p.covBarrier, c->stream));
         c->launches++;
       }
-    CK(cudaEventRecord(c->evAff, c->stream));
-    CK(cudaStreamWaitEvent(c->copyStream, c->evAff, 0));
-    if (nm) CK(cudaMemcpyAsync(P->pinned, c->maps.p, sizeof(float) * nm * np, cudaMemcpyDeviceToHost, c->copyStream));
-    CK(cudaMemcpyAsync(P->pinned + (size_t)(nm + 1) * np, c->maps.p + (size_t)(nm + 1) * np, sizeof(float) * np,
-                       cudaMemcpyDeviceToHost, c->copyStream));
+    if (int e = copyAffinityMaps(c, P->pinned)) return e;
     if (int e = ag_compute(c, AG_WORK_EMAP)) return e;
     CK(cudaMemcpyAsync(P->pinned + (size_t)nm * np, c->maps.p + (size_t)nm * np, sizeof(float) * np,
                        cudaMemcpyDeviceToHost, c->stream));
