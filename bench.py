@@ -6,8 +6,9 @@ the B200 engine.
 
 A step is one map set (the e-map and the affinity pass run concurrently, as
 the library runs them; each pass is also timed alone for the rooflines).
-`value` is point-atom evaluations per second over all ranks (N_atoms x
-N_points per map set / map-set seconds), with the inputs resident in HBM; `e2e` is the same metric through the public C ABI with host
+`value` is point-atom evaluations of the defining sum per second over all ranks
+(N_atoms x N_points per map set / map-set seconds; far atoms are summed at
+interpolation nodes, and the rooflines count the terms evaluated), with the inputs resident in HBM; `e2e` is the same metric through the public C ABI with host
 buffers (ag_problem_compute: upload, compute, all maps back in host memory).  L2 is flushed (256 MiB
 write) between timed steps.
 
@@ -350,6 +351,30 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(rows)}
 
 
+def emap_work(xyz, nx, ny, nz, spacing, node_radius=24.0, half_widths=8.5):
+    """(point-atom terms, node-atom terms) that the direct e-map evaluates on a large grid: atoms
+    within node_radius (and half_widths half-widths) of a CTA's 2 x 8 x 16-item tile enter each of
+    its points, the others its 125 interpolation nodes."""
+    import numpy as np
+
+    def cuts(n, t):  # even division into tiles of at most t
+        k = -(-n // t)
+        return [(n * i // k, n * (i + 1) // k) for i in range(k)]
+
+    direct = nodes = 0
+    cols = [(8 * c, min(nx, 8 * (c + 2))) for c in range(0, -(-nx // 8), 2)]
+    for x0, x1 in cols:
+        for y0, y1 in cuts(ny, 8 if x1 - x0 > 8 else 16):
+            for z0, z1 in cuts(nz, 16):
+                lo = (np.array([x0, y0, z0]) - np.array([nx // 2, ny // 2, nz // 2])) * spacing
+                hi = (np.array([x1, y1, z1]) - 1 - np.array([nx // 2, ny // 2, nz // 2])) * spacing
+                d = np.maximum(np.maximum(lo - xyz, xyz - hi), 0.0)
+                far = (d * d).sum(1) >= max(node_radius, half_widths * float((hi - lo).max()) / 2) ** 2
+                direct += int((~far).sum()) * (x1 - x0) * (y1 - y0) * (z1 - z0)
+                nodes += int(far.sum()) * 125
+    return direct, nodes
+
+
 def max_over_ranks(value, dist, device):
     """Max of a per-rank float over all ranks (the value itself without a process group)."""
     if dist is None:
@@ -614,7 +639,10 @@ def main():
         check = float(np.abs(maps_all[nmaps]).max())
         emap_pairs_per_s = pairs / (emap_avg * 1e-3)
         aff_pairs = affinity_pairs(prob.xyzw()[:, :3], prob.grid.nx, prob.grid.ny, prob.grid.nz, prob.grid.spacing)
-        mapset_ops = 8 * pairs + (nmaps + 10) * aff_pairs
+        direct, node_terms = emap_work(prob.xyzw()[:, :3], prob.grid.nx, prob.grid.ny, prob.grid.nz,
+                                       prob.grid.spacing)
+        emap_sfu, emap_ops = direct + 2 * node_terms, 8 * direct + 14 * node_terms
+        mapset_ops = emap_ops + (nmaps + 10) * aff_pairs
         ck = clocks.summary()
 
         # ---- supplementary measurements (N=1) ----
@@ -670,20 +698,25 @@ def main():
                           "its last wave leaves free; emap_ms and affinity_ms time each pass alone in K more "
                           "steps (their sum is the map set run one pass after the other)",
                 "roofline": {"bound": "sfu", "kernel": "emap_kernel",
-                             "achieved": emap_pairs_per_s / 1e9, "peak": rsqrt_ps / 1e9, "unit": "Gpair/s",
-                             "frac": emap_pairs_per_s / rsqrt_ps, "traffic": EMAP_TRAFFIC_BYTES,
+                             "achieved": emap_sfu / (emap_avg * 1e-3) / 1e9, "peak": rsqrt_ps / 1e9, "unit": "Gop/s",
+                             "frac": emap_sfu / (emap_avg * 1e-3) / rsqrt_ps, "traffic": EMAP_TRAFFIC_BYTES,
                              "traffic_unit": "DRAM bytes per launch (ncu capture of this workload)",
-                             "note": "one SFU rsqrt per point-atom pair; peak = rsqrt/s measured by "
-                                     "ag_measure_peaks in this run (MEASURED_PEAKS.json has no SFU figure)"},
-                "roofline_fp32": {"achieved_ops": 8 * emap_pairs_per_s / 1e12, "peak": ffma_ps / 1e12,
-                                  "unit": "Tinstr/s", "frac": 8 * emap_pairs_per_s / ffma_ps,
-                                  "note": "8 algorithmic FP32-pipe ops per pair vs measured FFMA issue rate"},
+                             "point_atom_terms": direct, "node_atom_terms": node_terms,
+                             "defining_sum_pairs": pairs, "defining_sum_pairs_per_s": emap_pairs_per_s,
+                             "note": "SFU operations evaluated: one rsqrt per point-atom term (atoms near a CTA's "
+                                     "box), rsqrt and ex2 per node-atom term (far atoms enter at 125 nodes per box "
+                                     "instead of 2,048 points); peak = rsqrt/s measured by ag_measure_peaks in this "
+                                     "run (MEASURED_PEAKS.json has no SFU figure)"},
+                "roofline_fp32": {"achieved_ops": emap_ops / (emap_avg * 1e-3) / 1e12, "peak": ffma_ps / 1e12,
+                                  "unit": "Tinstr/s", "frac": emap_ops / (emap_avg * 1e-3) / ffma_ps,
+                                  "note": "8 FP32-pipe ops per point-atom term and 14 per node-atom term evaluated, "
+                                          "vs measured FFMA issue rate"},
                 "roofline_mapset_fp32": {
                     "emap_pairs": pairs, "affinity_pairs": aff_pairs, "ops": mapset_ops,
                     "achieved_ops": mapset_ops / (ms_step * 1e-3) / 1e12, "peak": ffma_ps / 1e12,
                     "unit": "Tinstr/s", "frac": mapset_ops / (ms_step * 1e-3) / ffma_ps,
-                    "note": "the whole map set (e-map + affinity maps + d-map) per map-set time: 8 FP32 ops per "
-                            "e-map pair, n_maps + 10 per in-cutoff affinity pair (geometry, bin, one add per map, "
+                    "note": "the whole map set (e-map + affinity maps + d-map) per map-set time: the e-map's ops as "
+                            "above, n_maps + 10 per in-cutoff affinity pair (geometry, bin, one add per map, "
                             "two desolvation FMAs; H-bond angular terms not counted), vs the measured FFMA rate"},
                 "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                         "ms_per_step": e2e_s * 1e3},
