@@ -621,8 +621,10 @@ def main():
         # ---- end to end through the whole-job C ABI call (ag_problem_compute):
         # the parsed job's host arrays are uploaded, every map is computed and
         # the map set is copied back to host memory, each step ----
-        h2d = n_atoms * (32 + 4 + 4 + 4 + 4 + 48) + 8192 * 4
-        h2d += prob.info.n_types * 801 * nmaps * 4
+        # x, y, z, weight; bond vectors in FP64 and FP32; info, vol, solq; the
+        # dielectric table (its packed tail not counted); pair and desolvation tables
+        h2d = n_atoms * (32 + 24 + 32 + 3 * 4) + 8192 * 4
+        h2d += (prob.info.n_types * nmaps + 1) * 801 * 4
         d2h = (nmaps + 2) * npts * 4
         for _ in range(2):
             prob.compute(ctx)

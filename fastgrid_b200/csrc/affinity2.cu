@@ -8,19 +8,20 @@
 // value lies in a guard band around the edge.  What changes is the
 // organisation, for fewer instructions per point-atom pair:
 //
-//  * each thread holds two z-neighbouring points: one shared-memory record,
-//    dx, dy and dx^2 + dy^2 of a candidate atom serve both;
-//  * a CTA covers 8 x 8 x 8 points and each warp a 4 x 4 x 4 sub-box; a warp
+//  * each thread holds two z-neighbouring points, whose geometry is packed
+//    FP32x2: one shared-memory record and one guard test per candidate serve both;
+//  * a block covers 8 x 8 x 8 points and each warp a 4 x 4 x 4 sub-box; a warp
 //    walks only the candidates within 8 A of its own sub-box;
-//  * candidates are gathered from a type-major cell list ((cell, type)
-//    segments, file order inside each), so a batch arrives sorted by receptor
-//    type without a sort, and each type's table rows are loaded once per batch
-//    (one TMA bulk copy);
-//  * the plain map sums add whole table rows with packed FP32x2 adds (types
-//    without an H-bond term) or FMAs with a per-type 0/1 mask; the mask removes
-//    the maps whose H-bond term applies to that type (the "slots", at most four
-//    per pass), which read their table entry separately; a spare column of the
-//    row carries the desolvation value;
+//  * a block is two CTAs that add into zeroed slot maps: PLAIN sums whole table
+//    rows, SLOTS the maps whose H-bond term applies to a type (at most four per
+//    pass).  Apart they need 80 registers instead of 128 and share an SM;
+//  * candidates are gathered from a type-major cell list (a type's cells of one
+//    row along x are one run, file order inside each cell), so a batch arrives
+//    sorted by receptor type without a sort, and each type's table is loaded
+//    once per batch (one TMA bulk copy);
+//  * the plain sums add whole table rows with packed FP32x2 adds; a slot map's
+//    column is zero there, maps whose columns agree for every type share one, and
+//    the last column carries the desolvation value;
 //  * a point beyond 8 A of the atom reads an all-zero extra table row, so the
 //    plain sums need no branch;
 //  * the nearest H donor of each point (the reference's kd-tree query,
@@ -53,8 +54,8 @@ constexpr float kBias = 8388608.f;   // 2^23
 constexpr int kPlaneRows = kA2PlaneRows;
 static_assert(kPlaneRows >= kAffRows && kPlaneRows * sizeof(float) % 16 == 0, "plane rows");
 
-// The pass is two kernels over the same CTA blocks: PLAIN forms the whole-row
-// map sums of every type, SLOTS the H-bond slots, from the types they apply to.
+// The two CTAs of a block: PLAIN forms the whole-row map sums of every type,
+// SLOTS the H-bond slots, from the types they apply to.
 enum { PART_PLAIN = 0, PART_SLOTS = 1 };
 
 // Candidate data only one of the parts needs.

@@ -101,7 +101,7 @@ struct AffParams {
   const float* solq;              // solpar + solparQ * |q|
   const float4* rv8;              // per atom: rvector, 0, rvector2, 0 (FP32)
   const double* rv64;             // rvector, 3 per atom (FP64, for exact sign decisions)
-  // cell list (8 A cells)
+  // cell list (two-point kernel: type-major keys over 4 A cells; one-point: 8 A cells)
   const int* cellStart;           // ncell + 1
   const int* cellAtoms;
   double cellLo[3];

@@ -100,10 +100,10 @@ int64_t ag_ctx_launch_count(const ag_ctx* ctx);
 #define AG_TUNE_SURROGATE_TCGEN05 6   /* 0/1: surrogate corrector convolutions on tcgen05 (1, default) or mma.sync (0) */
 #define AG_TUNE_AFFINITY_KERNEL 9     /* affinity pass: 2 two grid points per thread, type-major candidates,
                                          nearest donor found in the kernel (default); 1 one point per thread
-                                         with a separate nearest-donor kernel (also used for passes with more
-                                         than 4 H-bond maps) */
-#define AG_TUNE_CONCURRENT_PASSES 10 /* 0/1: a map set's e-map and affinity pass run concurrently, the e-map on a
-                                         high-priority stream (1, default), or one after the other (0) */
+                                         with a separate nearest-donor kernel */
+#define AG_TUNE_CONCURRENT_PASSES 10 /* 0/1: a map set's e-map and affinity pass run concurrently, one of them on
+                                         a high-priority stream (the e-map; the affinity pass in
+                                         ag_problem_compute) (1, default), or one after the other (0) */
 #define AG_TUNE_EMAP_NODE_RADIUS 11   /* A, >= 24 (default 24): atoms this far from a CTA box (further for boxes wider
                                          than 5.6 A) are summed at the box's 125 interpolation nodes; 0: point by point */
 /* Failure-detection test hooks (default 0 = off).  IDLE_WAIT: 1..64 polls of an
