@@ -351,17 +351,18 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(rows)}
 
 
-def emap_work(xyz, nx, ny, nz, spacing, node_radius=24.0, half_widths=8.5):
-    """(point-atom terms, node-atom terms) that the direct e-map evaluates on a large grid: atoms
-    within node_radius (and half_widths half-widths) of a CTA's 2 x 8 x 16-item tile enter each of
-    its points, the others its 125 interpolation nodes."""
+def emap_work(xyz, nx, ny, nz, spacing, node_radius=24.0, half_widths=8.5, far_radius=57.0, far_half_widths=17.5):
+    """(point-atom terms, node-atom terms, far-node-atom terms) that the direct e-map evaluates on a
+    large grid: atoms within node_radius (and half_widths half-widths) of a CTA's 2 x 8 x 16-item
+    tile enter each of its points, the others its 125 interpolation nodes or, from far_radius (and
+    far_half_widths) on, 64 nodes."""
     import numpy as np
 
     def cuts(n, t):  # even division into tiles of at most t
         k = -(-n // t)
         return [(n * i // k, n * (i + 1) // k) for i in range(k)]
 
-    direct = nodes = 0
+    direct = nodes = far_nodes = 0
     cols = [(8 * c, min(nx, 8 * (c + 2))) for c in range(0, -(-nx // 8), 2)]
     for x0, x1 in cols:
         for y0, y1 in cuts(ny, 8 if x1 - x0 > 8 else 16):
@@ -369,10 +370,13 @@ def emap_work(xyz, nx, ny, nz, spacing, node_radius=24.0, half_widths=8.5):
                 lo = (np.array([x0, y0, z0]) - np.array([nx // 2, ny // 2, nz // 2])) * spacing
                 hi = (np.array([x1, y1, z1]) - 1 - np.array([nx // 2, ny // 2, nz // 2])) * spacing
                 d = np.maximum(np.maximum(lo - xyz, xyz - hi), 0.0)
-                far = (d * d).sum(1) >= max(node_radius, half_widths * float((hi - lo).max()) / 2) ** 2
+                d2, half = (d * d).sum(1), float((hi - lo).max()) / 2
+                far = d2 >= max(node_radius, half_widths * half) ** 2
+                far4 = d2 >= max(far_radius, far_half_widths * half) ** 2
                 direct += int((~far).sum()) * (x1 - x0) * (y1 - y0) * (z1 - z0)
-                nodes += int(far.sum()) * 125
-    return direct, nodes
+                nodes += int((far & ~far4).sum()) * 125
+                far_nodes += int(far4.sum()) * 64
+    return direct, nodes, far_nodes
 
 
 def max_over_ranks(value, dist, device):
@@ -641,9 +645,10 @@ def main():
         check = float(np.abs(maps_all[nmaps]).max())
         emap_pairs_per_s = pairs / (emap_avg * 1e-3)
         aff_pairs = affinity_pairs(prob.xyzw()[:, :3], prob.grid.nx, prob.grid.ny, prob.grid.nz, prob.grid.spacing)
-        direct, node_terms = emap_work(prob.xyzw()[:, :3], prob.grid.nx, prob.grid.ny, prob.grid.nz,
-                                       prob.grid.spacing)
-        emap_sfu, emap_ops = direct + 2 * node_terms, 8 * direct + 14 * node_terms
+        direct, node_terms, far_terms = emap_work(prob.xyzw()[:, :3], prob.grid.nx, prob.grid.ny, prob.grid.nz,
+                                                  prob.grid.spacing)
+        emap_sfu = direct + 2 * node_terms + far_terms
+        emap_ops = 8 * direct + 14 * node_terms + 6 * far_terms
         mapset_ops = emap_ops + (nmaps + 10) * aff_pairs
         ck = clocks.summary()
 
@@ -704,15 +709,16 @@ def main():
                              "frac": emap_sfu / (emap_avg * 1e-3) / rsqrt_ps, "traffic": EMAP_TRAFFIC_BYTES,
                              "traffic_unit": "DRAM bytes per launch (ncu capture of this workload)",
                              "point_atom_terms": direct, "node_atom_terms": node_terms,
+                             "far_node_atom_terms": far_terms,
                              "defining_sum_pairs": pairs, "defining_sum_pairs_per_s": emap_pairs_per_s,
                              "note": "SFU operations evaluated: one rsqrt per point-atom term (atoms near a CTA's "
                                      "box), rsqrt and ex2 per node-atom term (far atoms enter at 125 nodes per box "
-                                     "instead of 2,048 points); peak = rsqrt/s measured by ag_measure_peaks in this "
+                                     "instead of 2,048 points), one rsqrt per far-node term (64 nodes); peak = rsqrt/s measured by ag_measure_peaks in this "
                                      "run (MEASURED_PEAKS.json has no SFU figure)"},
                 "roofline_fp32": {"achieved_ops": emap_ops / (emap_avg * 1e-3) / 1e12, "peak": ffma_ps / 1e12,
                                   "unit": "Tinstr/s", "frac": emap_ops / (emap_avg * 1e-3) / ffma_ps,
-                                  "note": "8 FP32-pipe ops per point-atom term and 14 per node-atom term evaluated, "
-                                          "vs measured FFMA issue rate"},
+                                  "note": "8 FP32-pipe ops per point-atom term, 14 per node-atom and 6 per far-node term "
+                                          "evaluated, vs measured FFMA issue rate"},
                 "roofline_mapset_fp32": {
                     "emap_pairs": pairs, "affinity_pairs": aff_pairs, "ops": mapset_ops,
                     "achieved_ops": mapset_ops / (ms_step * 1e-3) / 1e12, "peak": ffma_ps / 1e12,

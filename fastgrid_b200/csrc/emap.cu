@@ -67,15 +67,29 @@ enum { kClsNode = 0, kClsNear = 1, kClsMid = 2, kClsMid16 = 3, kClsMid8 = 4, kCl
 constexpr int kNodes1 = 5;                             // interpolation nodes per axis
 constexpr int kNodes = kNodes1 * kNodes1 * kNodes1;    // per CTA box
 constexpr int kNodeGroups = 4;                         // thread groups that share a tile's node atoms
+// Atoms at least this far from the box (0.01 A, and half extents) need only
+// 4 x 4 x 4 nodes and the saturated dielectric: 8.63 exp(-0.3154 r), the
+// largest part of a term left out, is 1.4e-7 at 57 A, and interpolation from 4
+// nodes errs by at most 2.1e-6 of a term (rms 6e-7) at 17.5 half extents, no
+// more than from 5 nodes at 8.5.  A quarter of the SFU operations per atom:
+// 60,000 atoms on 255^3 points 59.3 -> 49.3 ms, 40,000 on 201^3 26.0 -> 23.5,
+// 20,000 on 161^3 10.6 -> 10.4, and 2.15 ms either way for 8,000 on 125 x 97 x 83.
+constexpr float kFarNodeRadius = 5700.f, kFarNodeHalfWidths = 17.5f;
+constexpr int kFarNodes1 = 4;
+constexpr int kFarNodes = kFarNodes1 * kFarNodes1 * kFarNodes1;
+static_assert(kFarNodes == 2 * 32, "a warp holds two far nodes per lane");
 
 struct EmapSmem {
   float tab[kTabLen];             // 32 KB
   double4 ring[2][kTile];         // 16 KB, TMA destination
+  // Packed table tail; the last 4 KB hold the far nodes' sums (farAcc) where the
+  // box's mid atoms do not read that far.
   __align__(16) unsigned char packed[kEmapPackedBytes];
   // This tile's atoms grouped by class: local scaled x, y, z and 100*w
   // (near, mid), 100*w*g*2^-16 (packed mid) or 100*w*g (far).  The node atoms
-  // come first, two atoms in two entries: (x0, x1, y0, y1), (z0, z1, w0, w1).
-  float4 list[kTile + 2];
+  // come first, two atoms in two entries: (x0, x1, y0, y1), (z0, z1, w0, w1);
+  // far-node atoms, where the box has such, are the last class in the same form.
+  float4 list[kTile + 4];
   float4 nodeAcc[kThreads];       // per thread: Kahan sum and compensation of its two nodes
   short nearIdx[kTile + 2];       // tile slot of each near atom (for FP64 lookups)
   // Near atom: bit w set if it lies within rNear of warp w's points, bit 8 + w
@@ -84,10 +98,17 @@ struct EmapSmem {
   float4 wlo[kThreads / 32], whi[kThreads / 32];  // each warp's box (local, scaled), widened by 0.01 A
   int cnt[kNumCls][kThreads / 32];
   double wpart[kThreads / 32];
+  float rnode2, rfn2;             // squared radii of the box's node and far-node atoms
   int unit;                       // persistent batch kernel: the unit being processed
   uint64_t bar[2];
   uint64_t barIdle;               // never arrived on (target of the expiry test hook)
+
+  // Per thread: Kahan sum and compensation of its two far nodes.
+  __device__ __forceinline__ float4* farAcc() {
+    return reinterpret_cast<float4*>(packed + kEmapPackedBytes) - kThreads;
+  }
 };
+constexpr int kFarAccVecs = (kEmapPackedBytes - kThreads * (int)sizeof(float4)) / 16;  // tail vectors that leave room
 
 __device__ __forceinline__ void unpack_item(int v, int& xc, int& y, int& z) {
   xc = v & 0xFF;
@@ -339,6 +360,73 @@ __device__ __forceinline__ void node_atoms(EmapSmem& S, const int npairs, const 
   S.nodeAcc[threadIdx.x] = a;
 }
 
+// Far node k of [-1, 1]: cos((2 k + 1) pi / 8).
+__device__ __forceinline__ float far_node(int k) {
+  const float v = (k == 0 || k == 3) ? 0.92387953f : 0.38268343f;
+  return k > 1 ? -v : v;
+}
+
+// Lagrange weights of the four far nodes at t; 1 / prod_{m != j} (c_j - c_m) is
+// 2 (-1)^j sin((2 j + 1) pi / 8).
+__device__ __forceinline__ void far_weights(float t, float (&w)[kFarNodes1]) {
+  const float inv[kFarNodes1] = {0.76536686f, -1.84775907f, 1.84775907f, -0.76536686f};
+#pragma unroll
+  for (int j = 0; j < kFarNodes1; j++) {
+    float p = inv[j];
+#pragma unroll
+    for (int m = 0; m < kFarNodes1; m++)
+      if (m != j) p *= t - far_node(m);
+    w[j] = p;
+  }
+}
+
+// Sum of a tile's far-node atoms (pairs from list) at this lane's two far
+// nodes, neighbours along x, so one dy and dz serve both; the warps take the
+// pairs in turn.  Saturated dielectric: one rsqrt per term.
+__device__ __forceinline__ void far_node_atoms(EmapSmem& S, const float4* list, const int npairs, const float hx,
+                                               const float hy, const float hz) {
+  int n = 2 * (threadIdx.x & 31);
+  asm volatile("" : "+r"(n));  // keeps the node positions out of the caller's loops
+  const float2 nx0 = dup2(-far_node(n & 3) * hx), nx1 = dup2(-far_node((n & 3) + 1) * hx);
+  const float2 ny = dup2(-far_node((n >> 2) & 3) * hy), nz = dup2(-far_node(n >> 4) * hz);
+  float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+#pragma unroll 4
+  for (int p = threadIdx.x >> 5; p < npairs; p += kThreads / 32) {
+    const float4 xy = list[2 * p], zw = list[2 * p + 1];
+    const float2 dy = __fadd2_rn(make_float2(xy.z, xy.w), ny), dz = __fadd2_rn(make_float2(zw.x, zw.y), nz);
+    const float2 yz = __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)), w = make_float2(zw.z, zw.w);
+    const float2 x0 = __fadd2_rn(make_float2(xy.x, xy.y), nx0), x1 = __fadd2_rn(make_float2(xy.x, xy.y), nx1);
+    s0 = __ffma2_rn(w, rsqrt2(__ffma2_rn(x0, x0, yz)), s0);
+    s1 = __ffma2_rn(w, rsqrt2(__ffma2_rn(x1, x1, yz)), s1);
+  }
+  float4 a = S.farAcc()[threadIdx.x];
+  const float y0 = (s0.x + s0.y) - a.y, t0 = a.x + y0;
+  const float y1 = (s1.x + s1.y) - a.w, t1 = a.z + y1;
+  a.y = (t0 - a.x) - y0;
+  a.x = t0;
+  a.w = (t1 - a.z) - y1;
+  a.z = t1;
+  S.farAcc()[threadIdx.x] = a;
+}
+
+// The far nodes' field (sums F4, x fastest) at near node n: exact, a cubic's
+// values at the five nodes per axis stand for the cubic itself.
+__device__ __forceinline__ double far_field(const double* F4, int n) {
+  float wx[kFarNodes1], wy[kFarNodes1], wz[kFarNodes1];
+  asm volatile("" : "+r"(n));  // keeps the weights out of the caller's loops
+  far_weights(cheb_node(n % kNodes1), wx);
+  far_weights(cheb_node((n / kNodes1) % kNodes1), wy);
+  far_weights(cheb_node(n / (kNodes1 * kNodes1)), wz);
+  double f = 0.0;
+#pragma unroll
+  for (int k = 0; k < kFarNodes1 * kFarNodes1; k++) {
+    const double* r = F4 + kFarNodes1 * k;
+    const double w = (double)(wz[k >> 2] * wy[k & 3]);
+    f += w * ((double)wx[0] * r[0] + (double)wx[1] * r[1] + (double)wx[2] * r[2] + (double)wx[3] * r[3]);
+  }
+  return f;
+}
+
 // The node atoms' field at this thread's points, from the node sums F (in
 // shared memory, x fastest): the y and z weights first, then x per point.
 __device__ __forceinline__ void node_field(const float* F, const float2 (&gxn)[kNX / 2], float gy, float gz, float hx,
@@ -481,9 +569,26 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
   // Atoms this far (0.01 A) from the box are summed at its nodes.
   const float rnode = NODES ? fmaxf(P.rnodeHalfWidths * B.rnode, P.rnodeMin) : __int_as_float(0x7F800000);
   // Mid-list bins may pass the table's end (not if the node atoms begin before).
-  const bool clampMid = B.clampMid && !(rnode + 2.f * sqrtf(B.hx * B.hx + B.hy * B.hy + B.hz * B.hz) < 8100.f);
-  int nodeTotal = 0;  // node atoms seen so far (uniform)
-  if (NODES) S.nodeAcc[tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float midEndR = rnode + 2.f * sqrtf(B.hx * B.hx + B.hy * B.hy + B.hz * B.hz);
+  const bool clampMid = B.clampMid && !(midEndR < 8100.f);
+  int nodeSeen = 0;  // uniform; bit 0: node atoms, bit 1: far-node atoms
+  // The part of the packed tail that this box's mid atoms read: 16-bit entries
+  // up to the farthest bin only, if the node atoms begin before the 8-bit ones.
+  const int tailVecs = NODES && DDD && midEndR < 8100.f && rnode * rnode <= P.r8sq
+                           ? min(P.packedVecs, max(0, (int)midEndR + 3 - P.b16) / 8 + 1)
+                           : P.packedVecs;
+  // Far nodes: where the node atoms begin before the saturated point sums, so
+  // that kClsFar holds far-node atoms or none (else kClsFar is summed at the points).
+  const bool farNodes = NODES && DDD && rnode * rnode <= B.rfar2 && tailVecs <= kFarAccVecs;
+  const float rfn = fmaxf(kFarNodeHalfWidths * B.rnode, fmaxf(kFarNodeRadius, rnode));
+  if (NODES) {
+    if (tid == 0) {
+      S.rnode2 = rnode * rnode;
+      S.rfn2 = farNodes ? rfn * rfn : __int_as_float(0x7F800000);
+    }
+    S.nodeAcc[tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (farNodes) S.farAcc()[tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
 
   // Packed tail tables for this box: only when no bin can pass the table's end.
   const bool pk = DDD && P.packed != nullptr && !clampMid;
@@ -493,7 +598,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
     for (int i = tid; i < kTabLen / 4; i += kThreads) dst[i] = src[i];
     if (pk) {
       uint4* pdst = reinterpret_cast<uint4*>(S.packed);
-      for (int i = tid; i < P.packedVecs; i += kThreads) pdst[i] = P.packed[i];
+      for (int i = tid; i < tailVecs; i += kThreads) pdst[i] = P.packed[i];
     }
   }
   // This warp's box: the extent of its active lanes' points (an empty box,
@@ -579,8 +684,8 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
       const float dx = fmaxf(fabsf(loc.x) - B.hx, 0.f), dy = fmaxf(fabsf(loc.y) - B.hy, 0.f),
                   dz = fmaxf(fabsf(loc.z) - B.hz, 0.f);
       const float d2 = dx * dx + dy * dy + dz * dz;
-      if (NODES && d2 >= rnode * rnode) {
-        cls = kClsNode;
+      if (NODES && d2 >= S.rnode2) {
+        cls = DDD && d2 >= S.rfn2 ? kClsFar : kClsNode;
         loc.w *= gFar;
       } else if (d2 < P.rnear2) {
         cls = kClsNear;
@@ -618,9 +723,13 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
     __syncthreads();
     // Start of each class in the list, and of this warp's atoms within it.
     int base[kNumCls];
-    int run = 0, myPos = 0, nodeCnt = 0;
+    int run = 0, myPos = 0, nodeCnt = 0, midEnd = 0;
 #pragma unroll
     for (int c = NODES ? kClsNode : kClsNear; c < kNumCls; c++) {
+      if (c == kClsFar) {
+        midEnd = run;
+        if (NODES && DDD) run = (run + 1) & ~1;
+      }
       base[c] = run;
       int off = 0;
 #pragma unroll
@@ -636,7 +745,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
       }
     }
     const int nNode = NODES ? base[kClsNear] : 0;
-    if (NODES && cls == kClsNode) {
+    if (NODES && (cls == kClsNode || (farNodes && cls == kClsFar))) {
       float* pr = reinterpret_cast<float*>(S.list) + 8 * (myPos >> 1) + (myPos & 1);
       pr[0] = loc.x;
       pr[2] = loc.y;
@@ -649,18 +758,22 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
         S.nearMask[myPos] = (unsigned short)nearBits;
       }
     }
-    if (NODES && tid == 0 && (nodeCnt & 1)) {
+    if (NODES && ((tid == 0 && (nodeCnt & 1)) || (farNodes && tid == 1 && (run & 1)))) {
       // An odd last pair is completed by an atom of no weight far away.
-      float* pr = reinterpret_cast<float*>(S.list) + 8 * (nodeCnt >> 1) + 1;
+      float* pr = reinterpret_cast<float*>(S.list) + 8 * ((tid == 0 ? nodeCnt : run) >> 1) + 1;
       pr[0] = 1.0e7f;
       pr[2] = 0.f;
       pr[4] = 0.f;
       pr[6] = 0.f;
     }
     __syncthreads();
+    if (farNodes && run > base[kClsFar]) {
+      far_node_atoms(S, S.list + base[kClsFar], (run - base[kClsFar] + 1) >> 1, B.hx, B.hy, B.hz);
+      nodeSeen |= 2;
+    }
     if (NODES && nNode > 0) {
       node_atoms<DDD>(S, nNode >> 1, B.hx, B.hy, B.hz);
-      nodeTotal += nNode;
+      nodeSeen |= 1;
     }
 
     // Mid atoms: table read, or a packed tail table.
@@ -676,13 +789,13 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
         const uint32_t p8 = smem_u32(S.packed) + 16u * (uint32_t)P.vec8 - (0x4B000000u + (uint32_t)P.b8);
         mid_packed_atoms<MODE, 2>(S.list + base[kClsMid16], p16, base[kClsMid8] - base[kClsMid16], gxn, gy, gz, sum,
                                   cmp, P.kScale);
-        mid_packed_atoms<MODE, 1>(S.list + base[kClsMid8], p8, base[kClsFar] - base[kClsMid8], gxn, gy, gz, sum,
+        mid_packed_atoms<MODE, 1>(S.list + base[kClsMid8], p8, midEnd - base[kClsMid8], gxn, gy, gz, sum,
                                   cmp, P.kScale);
       }
     }
 
     // Far atoms: saturated dielectric (or the constant dielectric), no table.
-    const int nFar = busy ? run - base[kClsFar] : 0;
+    const int nFar = busy && !farNodes ? run - base[kClsFar] : 0;
     const float4* farA = S.list + base[kClsFar];
 #pragma unroll 1
     for (int j0 = 0; j0 < nFar; j0 += kChunk) {
@@ -761,10 +874,23 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
 
   // The node atoms' part: their sums at the nodes, interpolated to the points.
   float fld[kNX] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (NODES && nodeTotal > 0) {
+  if (NODES && nodeSeen) {
     float* F = reinterpret_cast<float*>(S.list);
+    double* F4 = reinterpret_cast<double*>(S.list + 64);  // far nodes' sums
+    if (nodeSeen & 2) {
+      if (tid < kFarNodes) {
+        double f = 0.0;
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; w++) {
+          const float4 a = S.farAcc()[32 * w + (tid >> 1)];
+          f += (tid & 1) ? (double)a.z - (double)a.w : (double)a.x - (double)a.y;
+        }
+        F4[tid] = f;
+      }
+      __syncthreads();
+    }
     if (tid < kNodes) {
-      double f = 0.0;
+      double f = (nodeSeen & 2) ? far_field(F4, tid) : 0.0;
 #pragma unroll
       for (int grp = 0; grp < kNodeGroups; grp++) {
         const float4 a = S.nodeAcc[64 * grp + (tid >> 1)];

@@ -68,6 +68,38 @@ def test_smooth_dielectric_is_the_table_between_its_steps():
     assert 0.5 * step[0] < 7.3e-6 and 0.5 * step[300] < 2.9e-6
 
 
+FAR_NODES = np.cos((2 * np.arange(4) + 1) * np.pi / 8)
+
+
+@pytest.mark.parametrize("half", [(2.81, 1.31, 2.81), (2.81, 2.81, 2.81), (0.4, 2.9, 2.9), (4.5, 2.1, 4.5)])
+def test_far_node_error_at_the_least_distance(half):
+    """From 57 A and 17.5 half-widths on: four nodes per axis and the saturated dielectric, within
+    2.2e-6 (interpolation) and 1.4e-7 (the dielectric's part left out) of a term."""
+    rng = np.random.default_rng(2)
+    R = max(17.5 * max(half), 57.0)
+    axis = np.linspace(-1, 1, 9)
+    W = np.ones((9, 4))
+    for j in range(4):
+        for m in range(4):
+            if m != j:
+                W[:, j] *= (axis - FAR_NODES[m]) / (FAR_NODES[j] - FAR_NODES[m])
+    for _ in range(150):
+        d = rng.standard_normal(3) * (rng.random(3) > 0.3)
+        if not d.any():
+            continue
+        d /= np.linalg.norm(d)
+        a = np.where(d == 0, rng.uniform(-1, 1, 3), np.sign(d)) * half + R * d
+
+        def r(x, y, z):
+            return np.sqrt((x[:, None, None] - a[0]) ** 2 + (y[:, None] - a[1]) ** 2 + (z - a[2]) ** 2)
+
+        got = np.einsum("xi,yj,zk,ijk->xyz", W, W, W, 1 / r(*(FAR_NODES * h for h in half)))
+        want = r(*(axis * h for h in half))
+        E = np.exp(-LAMBDA * (want - 0.005))
+        assert (np.abs(got * want - 1) < 2.2e-6).all()
+        assert (E * ((A + C) + C * (A + C) * E) < 1.4e-7).all()
+
+
 def _atoms(rng, n, spread):
     """Atoms around the grid and on shells out to 120 A, some far outside."""
     inner = rng.normal(0, spread, (n, 3))
@@ -105,6 +137,42 @@ def test_node_sums_match_point_sums_and_oracle(nx, ny, nz, h, n):
                 got = ctx.emap(g, xyzw, eps)
                 assert (np.abs(got - point.astype(np.float64)) <= tol * mag + 1e-7).all()
                 assert np.abs(got - ref).max() <= E_TOL
+    finally:
+        ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,nz,h", [(33, 45, 29, 0.375), (41, 9, 17, 0.375), (129, 1, 1, 0.375),
+                                        (24, 23, 22, 0.6), (24, 23, 22, 0.7), (45, 37, 31, 1.0)])
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 257, 1100])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_far_nodes_match_point_sums_and_oracle(nx, ny, nz, h, n, mixed):
+    """Atoms beyond 57 A of every box alone (odd and even counts around a tile), and in one list with
+    nearer ones of every class.  Alone, a term may differ by its interpolation error (2.2e-6 far;
+    4e-6 where wide boxes keep five nodes), the dielectric left out and FP32 rounding (1e-6);
+    mixed, by the node sums' own 12.3e-6."""
+    rng = np.random.default_rng(nx + n)
+    ends = np.array([nx, ny, nz]) * h / 2
+    d = rng.standard_normal((n, 3))
+    d /= np.abs(d).max(axis=1, keepdims=True)
+    xyz = d * (ends.max() + rng.uniform(58, 140, (n, 1)))  # one coordinate past the grid by that much
+    xyzw = np.concatenate([xyz, rng.normal(0, 0.03, (n, 1))], axis=1)
+    if mixed:
+        xyzw = np.concatenate([xyzw, _atoms(rng, 150, 9.0)])
+        xyzw = xyzw[rng.permutation(len(xyzw))]
+    g = fg.Grid(nx, ny, nz, h)
+    eps = fg.ddd_table()
+    ref = oracle.emap(g, xyzw, eps)
+    mag = oracle.emap(g, np.abs(xyzw) * [0, 0, 0, 1] + xyzw * [1, 1, 1, 0], eps)
+    ctx = fg.Context(0)
+    try:
+        ctx.tune(fg.AG_TUNE_EMAP_NODE_RADIUS, 0)
+        point = ctx.emap(g, xyzw, eps)
+        ctx.tune(fg.AG_TUNE_EMAP_NODE_RADIUS, 24)
+        got = ctx.emap(g, xyzw, eps)
+        tol = 12.3e-6 if mixed else 5.2e-6
+        assert (np.abs(got - point.astype(np.float64)) <= tol * mag + 1e-7).all()
+        assert np.abs(got - ref).max() <= E_TOL
     finally:
         ctx.close()
 
