@@ -167,6 +167,8 @@ struct ag_ctx {
   float nearRadius() const { return rNear > 0.f ? rNear : ddd && !itemsDense ? 11.75f : 11.0f; }
   static constexpr float kNodeRadius = 24.0f, kNodeHalfWidths = 8.5f, kNodeHalfWidthsConst = 9.5f;
   float rNode = kNodeRadius;        // AG_TUNE_EMAP_NODE_RADIUS (0: no node sums)
+  bool rNodeSet = false;            // ... set by the caller
+  bool batchJob = false;            // a batch's job: its CTAs run beside other jobs'
   bool smoothTail = false;          // the staged dielectric table is AutoGrid's function
   float delta = 2.0e-3f;
   int packedTable = 1;              // AG_TUNE_EMAP_PACKED_TABLE

@@ -185,6 +185,7 @@ extern "C" int ag_ctx_tune(ag_ctx* c, int knob, double v) {
     case AG_TUNE_EMAP_NODE_RADIUS:
       if (!(v == 0.0 || (v >= 24.0 && v <= 1.0e6))) return fail(AG_E_INVALID, "node radius must be 0 or at least 24 A");
       c->rNode = (float)v;
+      c->rNodeSet = true;
       return AG_OK;
     case AG_TUNE_EMAP_PACKED_TABLE:
       if (!(v == 0.0 || v == 1.0)) return fail(AG_E_INVALID, "packed-table switch must be 0 or 1");
@@ -432,8 +433,8 @@ void makeItems(const ag_grid& g, const int tile[3], int warpCompact, bool dense,
 }
 
 // Whether the direct e-map's CTAs are cut densely and no node sums are formed:
-// where they could not take a fair share of the atoms, that is where no atom is 1.7 (default) node
-// radii from a grid point along any axis (2,000 atoms on 61^3 points: 0.334 ms dense,
+// for few pairs, and where they could not take a fair share of the atoms, that is where no atom is
+// 1.7 (default) node radii from a grid point along any axis (2,000 atoms on 61^3 points: 0.334 ms dense,
 // 0.367 ms with a CTA per tile; 1,017 atoms on 150^3: 1.23 and 1.00 ms).
 bool denseItems(const ag_ctx* c) {
   if (c->ddd && !c->smoothTail) return true;  // no node sums
@@ -442,6 +443,12 @@ bool denseItems(const ag_ctx* c) {
   const double radius = std::max<double>(
       std::max(c->rNear > 0.f ? c->rNear : 11.f, c->ddd ? ag_ctx::kNodeRadius : 0.f),
       (c->ddd ? ag_ctx::kNodeHalfWidths : ag_ctx::kNodeHalfWidthsConst) * 7.5 * g.spacing);
+  // Few pairs: the tiles' own cost (tables, classes, half-empty CTAs) outweighs
+  // what the nodes save.  1,227 atoms on 56 x 147 x 49 points (4.9e8): 0.329 ms
+  // dense, 0.375 ms with tiles; 3,000 on 45 x 111 x 45 (6.7e8): 0.396 and 0.419;
+  // 5,000 on 45 x 111 x 45 (1.1e9): 0.541 and 0.515.  Not for a batch's jobs,
+  // which share the GPU, nor where the caller has set the node radius.
+  if (c->ddd && !c->rNodeSet && !c->batchJob && (double)c->nAtoms * (double)c->npoints() < 1.0e9) return true;
   for (int d = 0; d < 3; d++) {
     const double lo = -(n[d] / 2) * g.spacing, hi = (n[d] - 1 - n[d] / 2) * g.spacing;
     if (std::max(c->atomHi[d] - lo, hi - c->atomLo[d]) >= 1.7 * radius) return false;
@@ -1693,6 +1700,7 @@ extern "C" int ag_batch_create(ag_ctx* ctx, ag_problem* const* problems, int n, 
     ag_ctx* c = nullptr;
     if (int e = ag_ctx_create(ctx->device, &c)) { ag_batch_free(b); return e; }
     c->affKernel = ctx->affKernel;
+    c->batchJob = true;
     b->sub.push_back(c);
     b->probs.push_back(problems[i]);
     ag_grid g;

@@ -222,3 +222,30 @@ def test_other_tables_are_summed_point_by_point():
             ctx.tune(fg.AG_TUNE_EMAP_NODE_RADIUS, 10)
     finally:
         ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [970, 971])
+def test_both_sides_of_the_few_pairs_rule(n):
+    """970 and 971 atoms on 101^3 points lie on either side of 1e9 pairs, below which no node sums are
+    formed: both match the oracle, and a node radius set by hand (node sums on either side) within
+    the node sums' 12.3e-6 of the terms' magnitudes."""
+    rng = np.random.default_rng(3)
+    xyzw = _atoms(rng, 485, 9.0)[:n]
+    if len(xyzw) < n:
+        xyzw = np.concatenate([xyzw, _atoms(rng, 1, 9.0)[:n - len(xyzw)]])
+    g = fg.Grid(101, 101, 101, 0.375)
+    idx = np.unique(rng.integers(0, 101 ** 3, 3000))
+    eps = fg.ddd_table()
+    want = oracle.emap_points(g, xyzw, eps, idx)
+    mag = oracle.emap_points(g, np.abs(xyzw) * [0, 0, 0, 1] + xyzw * [1, 1, 1, 0], eps, idx)
+    ctx = fg.Context(0)
+    try:
+        default = ctx.emap(g, xyzw, eps).ravel()[idx].astype(np.float64)
+        ctx.tune(fg.AG_TUNE_EMAP_NODE_RADIUS, 24)
+        nodes = ctx.emap(g, xyzw, eps).ravel()[idx]
+    finally:
+        ctx.close()
+    assert len(xyzw) == n
+    assert np.abs(default - want).max() <= E_TOL
+    assert (np.abs(nodes - default) <= 12.3e-6 * mag + 1e-7).all()
