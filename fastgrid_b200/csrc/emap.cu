@@ -555,11 +555,13 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
   const bool il = (item & kItemInterleaved) != 0;
   const int xb = il ? (xc >> 1) * (2 * kNX) + (xc & 1) : xc * kNX;
   const int xs = il ? 2 : 1;
+  // A point past the grid's end stands on the last one (and is not written): the
+  // box holds every point that is evaluated, on which the table reads' clamps rely.
   const double h = P.h;
   float gx[kNX];
 #pragma unroll
   for (int k = 0; k < kNX; k++)
-    gx[k] = (float)(((double)(xb + k * xs - P.n2x) * h - B.ox) * 100.0);
+    gx[k] = (float)(((double)(min(xb + k * xs, P.nx - 1) - P.n2x) * h - B.ox) * 100.0);
   const float gy = (float)(((double)(iy - P.n2y) * h - B.oy) * 100.0);
   const float gz = (float)(((double)(iz - P.n2z) * h - B.oz) * 100.0);
   float2 gxn[kNX / 2];
@@ -830,8 +832,7 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
       if (DDD && !((S.nearMask[j] >> warp) & 1u)) {
         // At least rNear from every point of this warp (uniform): the mid-list
         // arithmetic (no cap, round-down bin), each term compensated.  The
-        // clamp keeps the bin inside the table for any box size, and for the
-        // lanes without an item, whose stand-in points can lie anywhere.
+        // clamp keeps the bin inside the table for any box size.
         const uint32_t tabB = smem_u32(S.tab) - 0x2C000000u;
 #pragma unroll
         for (int k = 0; k < kNX / 2; k++) {
