@@ -316,8 +316,8 @@ static std::pair<int, int> bestSplit(int ny, int nz, const int T[3], int w, int 
 // one shared-memory bank.  A column whose partner is past the grid edge keeps
 // its own NX consecutive points.
 // dense: the tiles' items, in boustrophedon tile order, are cut into CTAs of
-// 256 whatever the tiles, so that every CTA but the last is full and a box may
-// span two tiles (the surrogate's near field, whose cost is per CTA and whose
+// 256 (255 where a pair would be split) whatever the tiles, so that every CTA but
+// the last is full and a box may span two tiles (the surrogate's near field, whose cost is per CTA and whose
 // warps skip atoms: 4.49 ms per surrogate e-map on 161^3 against 4.60 ms with
 // a CTA per tile).  Otherwise a CTA is a tile and its box stays compact, which
 // the direct e-map's node sums need: they begin 9.5 half-widths from the box.
@@ -373,10 +373,16 @@ int makeItemsInto(const ag_grid& g, const int tile[3], int warpCompact, bool den
                   std::min(g.nz, kz * T[2] + T[2]));
         }
       }
-    for (int item0 = 0; item0 < nitems; item0 += 256) {
+    for (int item0 = 0, n = 0; item0 < nitems; item0 += n) {
       agk::EmapBlock b{};
+      n = std::min(256, nitems - item0);
+      // A pair of interleaved columns stays in one CTA: each has points of both.
+      // (Pairs start with the even column; after a tile of an odd number of
+      // unpaired items they no longer start at even places of the list.)
+      const int last = items[item0 + n - 1];
+      if ((last & agk::kItemInterleaved) && !(last & 1)) n--;
       b.item0 = item0;
-      b.nitems = std::min(256, nitems - item0);
+      b.nitems = n;
       int i0[3] = {1 << 30, 1 << 30, 1 << 30}, i1[3] = {-1, -1, -1};
       for (int k = item0; k < item0 + b.nitems; k++) {
         const int v = items[k], xa = (v & 0xFF) * agk::kNX;  // (an interleaved pair's union is the same box)

@@ -37,6 +37,15 @@ def _check(nx, ny, nz, h, order):
     assert (np.abs(got - want) <= tol * mag + 1e-7).all()
 
 
+@pytest.mark.parametrize("nx,ny,nz", [(49, 53, 27), (33, 45, 33), (21, 45, 55), (37, 53, 25)])
+@pytest.mark.parametrize("h", [0.375, 0.7])
+@pytest.mark.parametrize("order", [0, 1, 2])
+def test_interleaved_columns_stay_in_one_box(nx, ny, nz, h, order):
+    """Odd row and plane counts of the last, unpaired column leave the pairs after it at odd places
+    of the item list."""
+    _check(nx, ny, nz, h, order)
+
+
 @pytest.mark.parametrize("nx,ny,nz", [(1, 1, 1), (1, 3, 2), (9, 2, 1), (10, 5, 5), (23, 4, 4)])
 @pytest.mark.parametrize("h", [2.0, 8.0, 27.0, 400.0])
 def test_points_past_the_end_of_widely_spaced_rows(nx, ny, nz, h):
