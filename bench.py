@@ -351,11 +351,13 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(rows)}
 
 
-def emap_work(xyz, nx, ny, nz, spacing, node_radius=24.0, half_widths=8.5, far_radius=57.0, far_half_widths=17.5):
+def emap_work(xyzw, nx, ny, nz, spacing, node_radius=24.0, half_widths=8.5, far_radius=57.0, far_half_widths=20.0,
+              near_radius=11.75):
     """(point-atom terms, node-atom terms, far-node-atom terms) that the direct e-map evaluates on a
     large grid: atoms within node_radius (and half_widths half-widths) of a CTA's 2 x 8 x 16-item
     tile enter each of its points, the others its 125 interpolation nodes or, from far_radius (and
-    far_half_widths) on, 64 nodes."""
+    far_half_widths) on, 64 nodes.  The node radius grows by up to half, until the density of squared
+    weights about near_radius is three times that beyond it, weighted by exp(-2 lambda r)."""
     import numpy as np
 
     def cuts(n, t):  # even division into tiles of at most t
@@ -363,16 +365,33 @@ def emap_work(xyz, nx, ny, nz, spacing, node_radius=24.0, half_widths=8.5, far_r
         return [(n * i // k, n * (i + 1) // k) for i in range(k)]
 
     direct = nodes = far_nodes = 0
+    w2 = xyzw[:, 3] ** 2
     cols = [(8 * c, min(nx, 8 * (c + 2))) for c in range(0, -(-nx // 8), 2)]
     for x0, x1 in cols:
         for y0, y1 in cuts(ny, 8 if x1 - x0 > 8 else 16):
             for z0, z1 in cuts(nz, 16):
                 lo = (np.array([x0, y0, z0]) - np.array([nx // 2, ny // 2, nz // 2])) * spacing
                 hi = (np.array([x1, y1, z1]) - 1 - np.array([nx // 2, ny // 2, nz // 2])) * spacing
-                d = np.maximum(np.maximum(lo - xyz, xyz - hi), 0.0)
-                d2, half = (d * d).sum(1), float((hi - lo).max()) / 2
-                far = d2 >= max(node_radius, half_widths * half) ** 2
-                far4 = d2 >= max(far_radius, far_half_widths * half) ** 2
+                d = np.maximum(np.maximum(lo - xyzw[:, :3], xyzw[:, :3] - hi), 0.0)
+                d, half = np.sqrt((d * d).sum(1)), float((hi - lo).max()) / 2
+                r = max(node_radius, half_widths * half)
+                a, b, c = (hi - lo)
+                near = w2[np.abs(d - near_radius) < 3.5].sum() / (
+                    2 * (a * b + b * c + c * a) * 7 + np.pi * (a + b + c) * 7 * 2 * near_radius +
+                    4 * np.pi / 3 * ((near_radius + 3.5) ** 3 - (near_radius - 3.5) ** 3))
+                e = w2 * np.exp(-2 * 0.3153767175 * (d - r)) * (d < 1.5 * r)
+                depth = 1 / (2 * 0.3153767175)
+                vol = depth * (2 * (a * b + b * c + c * a) + 2 * np.pi * (a + b + c) * (r + depth) +
+                               4 * np.pi * (r + depth) ** 2)
+                v = [3 * e[d >= r * (1 + k / 6)].sum() / vol for k in range(3)] + [0.0]
+                k = next(k for k in range(4) if k == 3 or near >= v[k])
+                t = k
+                if k > 0 and near > 0:
+                    fall = min(np.log(v[k - 1] / v[k]) if v[k] > 0 else np.inf, r / 6 / depth)
+                    t = k - 1 + min(1.0, np.log(v[k - 1] / near) / fall)
+                r *= 1 + t / 6
+                far = d >= r
+                far4 = d >= max(far_radius, far_half_widths * half, r)
                 direct += int((~far).sum()) * (x1 - x0) * (y1 - y0) * (z1 - z0)
                 nodes += int((far & ~far4).sum()) * 125
                 far_nodes += int(far4.sum()) * 64
@@ -645,7 +664,7 @@ def main():
         check = float(np.abs(maps_all[nmaps]).max())
         emap_pairs_per_s = pairs / (emap_avg * 1e-3)
         aff_pairs = affinity_pairs(prob.xyzw()[:, :3], prob.grid.nx, prob.grid.ny, prob.grid.nz, prob.grid.spacing)
-        direct, node_terms, far_terms = emap_work(prob.xyzw()[:, :3], prob.grid.nx, prob.grid.ny, prob.grid.nz,
+        direct, node_terms, far_terms = emap_work(prob.xyzw(), prob.grid.nx, prob.grid.ny, prob.grid.nz,
                                                   prob.grid.spacing)
         emap_sfu = direct + 2 * node_terms + far_terms
         emap_ops = 8 * direct + 14 * node_terms + 6 * far_terms

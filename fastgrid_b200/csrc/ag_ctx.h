@@ -106,6 +106,7 @@ struct ag_ctx {
   agc::DevBuf<double> thr;
   agc::DevBuf<int> items;
   agc::DevBuf<agk::EmapBlock> blocks;
+  agc::DevBuf<float2> radius;         // per CTA box: node and far-node radii
   agc::DevBuf<double> partial;
   agc::DevBuf<float> maps;
   agc::DevBuf<unsigned> status;

@@ -50,9 +50,12 @@ struct EmapParams {
   int b16, b8;
   float r16sq, r8sq;              // (b16 + 2)^2, (b8 + 2)^2: mid atoms at least that far (0.01 A units) from the box
   float kScale;                   // 2^(e + 126) / g, g = table[8191] = 2^e * m: turns 100 w g 2^-16 into 100 w ulp(g) 2^133
-  // Atoms at least max(rnodeMin, rnodeHalfWidths * EmapBlock::rnode) from the box (0.01 A) are summed at its nodes.
+  // Atoms at least max(rnodeMin, rnodeHalfWidths * EmapBlock::rnode) from the box (0.01 A) are summed at its nodes;
+  // with the distance-dependent dielectric, from the radius on that emap_launch finds for each box, of which that
+  // is the least.
   float rnodeMin;                 // +inf: none
   float rnodeHalfWidths;
+  float2* radius;                 // nblocks: node and far-node radii, filled by the launch (null: constant dielectric, or no node sums)
   int testIdleWait;               // test hook: > 0 adds a wait of that many polls on a barrier nothing arrives on
   float* out;
   double* partial;                // nsplit * npoints, when nsplit > 1

@@ -154,6 +154,7 @@ extern "C" int ag_ctx_destroy(ag_ctx* c) {
   c->atoms.release();
   c->thr.release();
   c->partial.release();
+  c->radius.release();
   c->thrA.release();
   c->checksum.release();
   agc::surrFree(c->surr);
@@ -664,6 +665,10 @@ int buildEmapParams(ag_ctx* c, float* dOut, bool allowSplit, agk::EmapParams& P)
   P.rnodeMin = (c->rNode > 0.f && (!c->ddd || c->smoothTail) && !c->itemsDense)
                    ? 100.f * std::max(c->nearRadius(), c->ddd ? c->rNode : 0.f)
                    : INFINITY;
+  if (c->ddd && P.rnodeMin < INFINITY) {
+    CK(c->radius.ensure(P.nblocks));
+    P.radius = c->radius.p;
+  }
   if (c->ddd && c->packedTable && c->pkVecs > 0) {
     P.packed = c->epsPacked.p;
     P.packedVecs = c->pkVecs;
@@ -704,7 +709,7 @@ int runEmap(ag_ctx* c, float* dOut) {
   P.checksum = c->checksum.p;
   c->checksumSplits = nsplit;
   CK(agk::emap_launch(P, c->ddd, c->emapMode, P.nblocks * nsplit, c->stream));
-  c->launches += nsplit > 1 ? 2 : 1;
+  c->launches += 1 + (P.radius ? 1 : 0) + (nsplit > 1 ? 1 : 0);
   return AG_OK;
 }
 

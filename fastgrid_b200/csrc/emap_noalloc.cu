@@ -73,6 +73,7 @@ constexpr int kNaCtasPerSm = 8;                  // as AG_TUNE_EMAP_CTAS_PER_SM'
 static __device__ __align__(256) double g_naPartial[kNaMaxPartial];
 static __device__ __align__(256) int g_naItems[kNaMaxItems];
 static __device__ __align__(256) agk::EmapBlock g_naBlocks[kNaMaxBlocks];
+static __device__ __align__(256) float2 g_naRadius[kNaMaxBlocks];
 static __device__ __align__(256) double g_naThr[kNaThr];
 static __device__ __align__(256) unsigned g_naStatus[64];
 static __device__ __align__(256) double g_naChecksum[kNaMaxSplit];
@@ -85,6 +86,7 @@ struct NaDevice {
   double* partial = nullptr;
   int* items = nullptr;
   agk::EmapBlock* blocks = nullptr;
+  float2* radius = nullptr;       // per CTA box
   double* thr = nullptr;
   unsigned* status = nullptr;
   double* checksum = nullptr;
@@ -174,6 +176,7 @@ int naSetup(NaDevice& d) {
   if (cudaGetSymbolAddress((void**)&d.partial, g_naPartial) != cudaSuccess ||
       cudaGetSymbolAddress((void**)&d.items, g_naItems) != cudaSuccess ||
       cudaGetSymbolAddress((void**)&d.blocks, g_naBlocks) != cudaSuccess ||
+      cudaGetSymbolAddress((void**)&d.radius, g_naRadius) != cudaSuccess ||
       cudaGetSymbolAddress((void**)&d.thr, g_naThr) != cudaSuccess ||
       cudaGetSymbolAddress((void**)&d.status, g_naStatus) != cudaSuccess ||
       cudaGetSymbolAddress((void**)&d.checksum, g_naChecksum) != cudaSuccess ||
@@ -292,6 +295,7 @@ extern "C" int ag_emap_noalloc(const ag_grid* grid, int n_atoms, const double* d
   P.rnear2 = (100.f * kNaNear) * (100.f * kNaNear);
   P.delta = 2.0e-3f;
   P.rnodeHalfWidths = 9.5f;
+  P.radius = smooth && d_inv_eps ? D.radius : nullptr;
   P.rnodeMin = smooth ? 100.f * (d_inv_eps ? kNaNode : kNaNear) : INFINITY;
   P.out = d_out;
   P.status = D.status;

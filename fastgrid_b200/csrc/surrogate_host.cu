@@ -573,6 +573,7 @@ int runEmapSurrogate(ag_ctx* c, float* dOut) {
     agk::EmapParams P;
     if (int e = buildEmapParams(c, dOut, false, P)) return e;
     P.checksum = nullptr;
+    P.rnodeMin = INFINITY;  // point by point
     P.items = S.dItems.p;
     P.blocks = S.dBlocks.p;
     P.nblocks = nb;

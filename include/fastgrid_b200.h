@@ -105,7 +105,8 @@ int64_t ag_ctx_launch_count(const ag_ctx* ctx);
                                          a high-priority stream (the e-map; the affinity pass in
                                          ag_problem_compute) (1, default), or one after the other (0) */
 #define AG_TUNE_EMAP_NODE_RADIUS 11   /* A, >= 24 (default 24): atoms this far from a CTA box (further for boxes wider
-                                         than 5.6 A) are summed at the box's 125 interpolation nodes (64 from 57 A on), on small
+                                         than 5.6 A, and up to half as far again for boxes beside the receptor) are summed
+                                         at the box's 125 interpolation nodes (64 from 57 A on), on small
                                          jobs only when set; 0: point by point */
 /* Failure-detection test hooks (default 0 = off).  IDLE_WAIT: 1..64 polls of an
  * extra wait, after each direct e-map CTA's first atom tile has landed, on a
