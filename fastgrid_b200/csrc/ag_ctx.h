@@ -165,7 +165,15 @@ struct ag_ctx {
   float rNear = 0.f;                // AG_TUNE_EMAP_RNEAR (0: the default, which nearRadius() gives)
   // 11.75 A where atoms beyond the node radius are taken without the table's
   // steps: the exact bins' larger share then keeps the map's error what it was.
-  float nearRadius() const { return rNear > 0.f ? rNear : ddd && !itemsDense ? 11.75f : 11.0f; }
+  // Also where the caller has turned the node sums off, so that the other terms
+  // are the same with and without them.
+  float nearRadius() const {
+    const bool off = rNode == 0.f && smoothTail && emapMode == agk::kEmapKahan;
+    return rNear > 0.f ? rNear : ddd && (nodeSums() || off) ? 11.75f : 11.0f;
+  }
+  // Whether atoms far from a CTA box are summed at its nodes: with CTAs that are tiles.
+  bool nodeSums() const { return nodesPossible() && !itemsDense; }
+  bool nodesPossible() const { return rNode > 0.f && (!ddd || smoothTail) && emapMode == agk::kEmapKahan; }
   static constexpr float kNodeRadius = 24.0f, kNodeHalfWidths = 8.5f, kNodeHalfWidthsConst = 9.5f;
   float rNode = kNodeRadius;        // AG_TUNE_EMAP_NODE_RADIUS (0: no node sums)
   bool rNodeSet = false;            // ... set by the caller

@@ -440,11 +440,18 @@ void makeItems(const ag_grid& g, const int tile[3], int warpCompact, bool dense,
 }
 
 // Whether the direct e-map's CTAs are cut densely and no node sums are formed:
-// for few pairs, and where they could not take a fair share of the atoms, that is where no atom is
-// 1.7 (default) node radii from a grid point along any axis (2,000 atoms on 61^3 points: 0.334 ms dense,
-// 0.367 ms with a CTA per tile; 1,017 atoms on 150^3: 1.23 and 1.00 ms).
+// where there are none to form, for few pairs, and where they could not take a
+// fair share of the atoms, that is where no atom is 1.7 times the least node
+// radius from a grid point along any axis (2,000 atoms on 61^3 points: 0.334 ms dense,
+// 0.367 ms with a CTA per tile; 1,017 atoms on 150^3: 1.23 and 1.00 ms; without
+// node sums 20,000 atoms on 161^3: 25.2 and 28.8 ms).
 bool denseItems(const ag_ctx* c) {
-  if (c->ddd && !c->smoothTail) return true;  // no node sums
+  const bool few = (double)c->nAtoms * (double)c->npoints() < 1.0e9;
+  // A small job whose node radius is set by hand is cut the same for 0 as for any
+  // radius, so that the two compare box by box (left alone it has no node sums).
+  const bool byHand = c->rNodeSet && few && !c->batchJob && (!c->ddd || c->smoothTail) &&
+                      c->emapMode == agk::kEmapKahan;
+  if (!c->nodesPossible() && !byHand) return true;
   const ag_grid& g = c->grid;
   const int n[3] = {g.nx, g.ny, g.nz};
   const double radius = std::max<double>(
@@ -455,7 +462,7 @@ bool denseItems(const ag_ctx* c) {
   // dense, 0.375 ms with tiles; 3,000 on 45 x 111 x 45 (6.7e8): 0.396 and 0.419;
   // 5,000 on 45 x 111 x 45 (1.1e9): 0.541 and 0.515.  Not for a batch's jobs,
   // which share the GPU, nor where the caller has set the node radius.
-  if (c->ddd && !c->rNodeSet && !c->batchJob && (double)c->nAtoms * (double)c->npoints() < 1.0e9) return true;
+  if (c->ddd && few && !c->rNodeSet && !c->batchJob) return true;
   for (int d = 0; d < 3; d++) {
     const double lo = -(n[d] / 2) * g.spacing, hi = (n[d] - 1 - n[d] / 2) * g.spacing;
     if (std::max(c->atomHi[d] - lo, hi - c->atomLo[d]) >= 1.7 * radius) return false;
@@ -554,6 +561,21 @@ bool tableIsSmooth(const float* t, int n) {
   return true;
 }
 
+// Put the work items and CTA boxes, which depend on the grid and the cut only, on the device.
+int stageItems(ag_ctx* c) {
+  buildItems(c);
+  if (c->itemsOnDevice) return AG_OK;
+  CK(c->items.ensure(c->hItems.size()));
+  CK(c->blocks.ensure(c->hBlocks.size()));
+  CK(cudaMemcpyAsync(c->items.p, c->hItems.data(), sizeof(int) * c->hItems.size(), cudaMemcpyHostToDevice,
+                     c->stream));
+  CK(cudaMemcpyAsync(c->blocks.p, c->hBlocks.data(), sizeof(agk::EmapBlock) * c->hBlocks.size(),
+                     cudaMemcpyHostToDevice, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  c->itemsOnDevice = true;
+  return AG_OK;
+}
+
 int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const double* inv_eps, bool deviceInputs) {
   if (int r = checkGrid(g)) return r;
   if (n < 0 || (n > 0 && !xyzw)) return fail(AG_E_INVALID, "bad atom array");
@@ -599,18 +621,7 @@ int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const doub
     c->epsPacked.p = reinterpret_cast<uint4*>(c->epsBuf.p + 8192);
     CK(c->epsStage.copy(c->epsBuf.p, tabBytes + pkBytes, c->stream));
   }
-  buildItems(c);
-  if (!c->itemsOnDevice) {  // the work items and CTA boxes depend on the grid only
-    CK(c->items.ensure(c->hItems.size()));
-    CK(c->blocks.ensure(c->hBlocks.size()));
-    CK(cudaMemcpyAsync(c->items.p, c->hItems.data(), sizeof(int) * c->hItems.size(), cudaMemcpyHostToDevice,
-                       c->stream));
-    CK(cudaMemcpyAsync(c->blocks.p, c->hBlocks.data(), sizeof(agk::EmapBlock) * c->hBlocks.size(),
-                       cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    c->itemsOnDevice = true;
-  }
-  return AG_OK;
+  return stageItems(c);
 }
 
 // Atoms per CTA when the grid alone does not give every SM enough waves of
@@ -662,7 +673,7 @@ int buildEmapParams(ag_ctx* c, float* dOut, bool allowSplit, agk::EmapParams& P)
   // has no steps and takes the interpolation's own error lower instead.  Near atoms
   // (the cap of 1/r, compensated terms) are never summed at the nodes.
   P.rnodeHalfWidths = c->ddd ? ag_ctx::kNodeHalfWidths : ag_ctx::kNodeHalfWidthsConst;
-  P.rnodeMin = (c->rNode > 0.f && (!c->ddd || c->smoothTail) && !c->itemsDense)
+  P.rnodeMin = c->nodeSums()
                    ? 100.f * std::max(c->nearRadius(), c->ddd ? c->rNode : 0.f)
                    : INFINITY;
   if (c->ddd && P.rnodeMin < INFINITY) {
@@ -698,6 +709,8 @@ int buildEmapParams(ag_ctx* c, float* dOut, bool allowSplit, agk::EmapParams& P)
 
 int runEmap(ag_ctx* c, float* dOut) {
   const int64_t np = c->npoints();
+  if (denseItems(c) != c->itemsDense)  // the node radius was set after staging
+    if (int e = stageItems(c)) return e;
   agk::EmapParams P;
   if (int e = buildEmapParams(c, dOut, true, P)) return e;
   const int nsplit = P.nsplit;
@@ -1325,10 +1338,10 @@ extern "C" int ag_emap_mode(ag_ctx* c, const ag_grid* g, int n, const double* xy
   c->haveJob = false;
   c->haveAff = false;
   c->nMaps = 0;
-  if (int e = stageEmap(c, g, n, xyzw, inv_eps, false)) return e;
-  CK(c->maps.ensure((size_t)2 * c->npoints()));
   c->emapMode = mode;
-  int e = runEmap(c, c->maps.p);
+  int e = stageEmap(c, g, n, xyzw, inv_eps, false);
+  if (!e && c->maps.ensure((size_t)2 * c->npoints()) != cudaSuccess) e = fail(AG_E_CUDA, "cannot allocate the map");
+  if (!e) e = runEmap(c, c->maps.p);
   c->emapMode = agk::kEmapKahan;
   if (e) return e;
   CK(cudaMemcpyAsync(out, c->maps.p, sizeof(float) * c->npoints(), cudaMemcpyDeviceToHost, c->stream));

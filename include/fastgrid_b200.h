@@ -91,7 +91,8 @@ int64_t ag_ctx_launch_count(const ag_ctx* ctx);
  * --cuda-* switches played this role for its kernels).  Results stay within
  * the stated tolerances for every allowed value. */
 #define AG_TUNE_EMAP_RNEAR 1          /* A, >= 8: atoms nearer the CTA box take the exact-bin path (default 11,
-                                         11.75 where far atoms are summed at interpolation nodes) */
+                                         11.75 where far atoms are summed at interpolation nodes and
+                                         where AG_TUNE_EMAP_NODE_RADIUS 0 has turned that off) */
 #define AG_TUNE_EMAP_PACKED_TABLE 2   /* 0/1: mid atoms in the table's saturating tail (from about 22 A) read 16- and 8-bit copies of it (1, default) or the FP32 table (0) */
 #define AG_TUNE_EMAP_CTAS_PER_SM 3    /* 1..8: half the CTAs per SM the atom split aims for on small grids (default 8) */
 #define AG_TUNE_EMAP_WARP_COMPACT 4   /* e-map item order: 0 rows, 1 each warp's items form a compact box, 2 as 1 with
