@@ -1724,6 +1724,9 @@ extern "C" int ag_batch_create(ag_ctx* ctx, ag_problem* const* problems, int n, 
     ag_ctx* c = nullptr;
     if (int e = ag_ctx_create(ctx->device, &c)) { ag_batch_free(b); return e; }
     c->affKernel = ctx->affKernel;
+    c->rNear = ctx->rNear;
+    c->rNode = ctx->rNode;
+    c->packedTable = ctx->packedTable;
     c->batchJob = true;
     b->sub.push_back(c);
     b->probs.push_back(problems[i]);

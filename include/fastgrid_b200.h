@@ -203,7 +203,8 @@ int ag_problem_write(ag_problem* p);
 /* ag_batch_compute captures the whole batch in a CUDA graph and later calls*/
 /* replay it.  No counterpart in the reference (one job per process).       */
 /* Problems must outlive the batch; all use the distance-dependent          */
-/* dielectric.                                                               */
+/* dielectric.  A job takes the context's e-map radii, packed-table switch   */
+/* and affinity kernel as they are set when the batch is created.            */
 /* ------------------------------------------------------------------------ */
 typedef struct ag_batch ag_batch;
 int ag_batch_create(ag_ctx* ctx, ag_problem* const* problems, int n, ag_batch** out);
