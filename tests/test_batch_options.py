@@ -69,3 +69,22 @@ def test_batch_takes_the_contexts_emap_options(tmp_path, knob, value):
     assert not np.array_equal(default, tuned)
     want = oracle.emap(p.grid, p.xyzw(), p.inv_eps())
     assert np.abs(tuned - want).max() <= E_TOL and np.abs(default - want).max() <= E_TOL
+
+
+def test_batch_keeps_no_staged_inputs(tmp_path):
+    """A job's staged inputs (about 400 KB) are not kept once it is on the device: the process grows by
+    less than half of that per job (the host copies of the table and the boxes take some 80 KB)."""
+    probs = _problems(tmp_path, [(2000, 31, "A C HD N OA SA")])
+
+    def resident():
+        return int(next(l for l in open("/proc/self/status") if l.startswith("VmRSS")).split()[1]) * 1024
+
+    grown = []
+    for _ in range(2):  # the first also loads code
+        ctx = fg.Context(0)
+        before = resident()
+        b = fg.Batch(ctx, probs * 48)
+        grown.append(resident() - before)
+        b.close()
+        ctx.close()
+    assert grown[1] < 48 * 200e3
