@@ -624,27 +624,33 @@ int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const doub
   return stageItems(c);
 }
 
-// Atoms per CTA when the grid alone does not give every SM enough waves of
-// resident CTAs to even out their unequal costs (with CTAs for 16 per SM 8,000
-// atoms on 101^3 points took 2.45 ms, with 6 per SM 2.63 ms).  Whole 256-atom
-// tiles, since a tile costs its barriers and its latency however few atoms it
-// holds; two at least where the grid gives every SM two waves of CTAs or nearly
-// (a CTA's set-up is worth about 100 atoms: 1,017 atoms on 125 x 101 x 120
-// points took 1.39 ms in quarters and 1.26 ms in halves, copies included); half
-// tiles where whole ones would not give every SM three CTAs; and at most 8,192
-// or half as many, since a CTA of more runs on for a millisecond after the
-// others (20,000 atoms on 161^3 points, whole job: 15.5 ms in two splits, 14.9
-// ms in four).
+// Atoms per CTA.  Where the grid alone does not give every SM enough waves of
+// resident CTAs to even out their unequal costs, atoms are split (with CTAs for
+// 16 per SM 8,000 atoms on 101^3 points took 2.45 ms, with 6 per SM 2.63 ms):
+// whole 256-atom tiles, since a tile costs its barriers and its latency however
+// few atoms it holds; two at least where the grid gives every SM two waves of
+// CTAs or nearly (a CTA's set-up is worth about 100 atoms: 1,017 atoms on
+// 125 x 101 x 120 points took 1.39 ms in quarters and 1.26 ms in halves, copies
+// included); half tiles where whole ones would not give every SM three CTAs.
+// Up to 4.5 times that many CTAs (175 MB of partial sums), also on larger grids, as
+// long as a CTA has more than kMost atoms, since it then runs on long after the
+// others: 20,000 atoms on 161^3 points take 11.7 ms in one part and 11.2 in four;
+// 40,000 17.7 and 16.8, 60,000 20.2 and 19.5; 40,000 on 201^3 27.3 ms and 26.8 in
+// two; 30,000 on 121^3 7.3 ms in four and 7.1 in six.
 int emapChunk(int nAtoms, int nblocks, int sms, int ctasPerSm) {
+  constexpr int kMost = 5120;
   const int want = 2 * sms * ctasPerSm;
-  if (nblocks >= want) return std::max(nAtoms, 1);
   if ((int64_t)nblocks * ((nAtoms + 255) / 256) < 3 * sms) return 128;
-  const int ns = (want + nblocks - 1) / nblocks;
-  int chunk = std::max(nblocks >= 5 * sms ? 512 : 256, nAtoms / ns / 256 * 256);
-  const int parts = (nAtoms + chunk - 1) / chunk;
-  if (parts > 1 && nAtoms - (parts - 1) * chunk < chunk / 4)  // no split of a few atoms
-    chunk = ((nAtoms + parts - 2) / (parts - 1) + 255) / 256 * 256;
-  if (chunk > 8192) chunk = (chunk / 2 + 255) / 256 * 256;
+  int chunk = std::max(nAtoms, 1);
+  if (nblocks < want) {
+    const int ns = (want + nblocks - 1) / nblocks;
+    chunk = std::max(nblocks >= 5 * sms ? 512 : 256, nAtoms / ns / 256 * 256);
+    const int parts = (nAtoms + chunk - 1) / chunk;
+    if (parts > 1 && nAtoms - (parts - 1) * chunk < chunk / 4)  // no split of a few atoms
+      chunk = ((nAtoms + parts - 2) / (parts - 1) + 255) / 256 * 256;
+  }
+  const int parts = std::min((nAtoms + kMost - 1) / kMost, 9 * want / 2 / nblocks);
+  if (parts > 1) chunk = std::min(chunk, ((nAtoms + parts - 1) / parts + 255) / 256 * 256);
   return chunk;
 }
 
