@@ -357,7 +357,8 @@ def emap_work(xyzw, nx, ny, nz, spacing, node_radius=24.0, half_widths=8.5, far_
     large grid: atoms within node_radius (and half_widths half-widths) of a CTA's 2 x 8 x 16-item
     tile enter each of its points, the others its 125 interpolation nodes or, from far_radius (and
     far_half_widths) on, 64 nodes.  The node radius grows by up to half, until the density of squared
-    weights about near_radius is three times that beyond it, weighted by exp(-2 lambda r)."""
+    weights about near_radius is that beyond it, weighted by exp(-2 lambda r), or three times that
+    where those about near_radius lie to one side of the tile."""
     import numpy as np
 
     def cuts(n, t):  # even division into tiles of at most t
@@ -372,18 +373,21 @@ def emap_work(xyzw, nx, ny, nz, spacing, node_radius=24.0, half_widths=8.5, far_
             for z0, z1 in cuts(nz, 16):
                 lo = (np.array([x0, y0, z0]) - np.array([nx // 2, ny // 2, nz // 2])) * spacing
                 hi = (np.array([x1, y1, z1]) - 1 - np.array([nx // 2, ny // 2, nz // 2])) * spacing
-                d = np.maximum(np.maximum(lo - xyzw[:, :3], xyzw[:, :3] - hi), 0.0)
-                d, half = np.sqrt((d * d).sum(1)), float((hi - lo).max()) / 2
+                u = np.maximum(xyzw[:, :3] - hi, 0.0) - np.maximum(lo - xyzw[:, :3], 0.0)
+                d, half = np.sqrt((u * u).sum(1)), float((hi - lo).max()) / 2
                 r = max(node_radius, half_widths * half)
                 a, b, c = (hi - lo)
-                near = w2[np.abs(d - near_radius) < 3.5].sum() / (
+                shell = np.abs(d - near_radius) < 3.5
+                lean = np.linalg.norm((w2[shell] / d[shell]) @ u[shell])
+                margin = 1 if lean < 0.35 * w2[shell].sum() else 3
+                near = w2[shell].sum() / (
                     2 * (a * b + b * c + c * a) * 7 + np.pi * (a + b + c) * 7 * 2 * near_radius +
                     4 * np.pi / 3 * ((near_radius + 3.5) ** 3 - (near_radius - 3.5) ** 3))
                 e = w2 * np.exp(-2 * 0.3153767175 * (d - r)) * (d < 1.5 * r)
                 depth = 1 / (2 * 0.3153767175)
                 vol = depth * (2 * (a * b + b * c + c * a) + 2 * np.pi * (a + b + c) * (r + depth) +
                                4 * np.pi * (r + depth) ** 2)
-                v = [3 * e[d >= r * (1 + k / 6)].sum() / vol for k in range(3)] + [0.0]
+                v = [margin * e[d >= r * (1 + k / 6)].sum() / vol for k in range(3)] + [0.0]
                 k = next(k for k in range(4) if k == 3 or near >= v[k])
                 t = k
                 if k > 0 and near > 0:

@@ -83,7 +83,7 @@ static_assert(kFarNodes == 2 * 32, "a warp holds two far nodes per lane");
 // Node radii of a box (box_radii): from the least one to three steps outwards.
 constexpr int kRadiusSteps = 3;
 constexpr float kRadiusStep = 1.f / 6.f;               // of the least radius: 24 to 28, 32 and 36 A
-constexpr float kRadiusMargin = 3.f;
+constexpr float kRadiusMargin = 3.f, kRadiusLean = 0.35f;
 constexpr int kRadiusBoxes = 4;                        // boxes per CTA
 
 struct EmapSmem {
@@ -1028,20 +1028,23 @@ __device__ __forceinline__ float area_at(const float3 h, float d) {
 // receptor, the second is 1.8 times the first for R = 24 A.  Beside a receptor
 // few atoms are near and many far.  So R is the least radius from 24 A on for
 // which the density of squared weights within 3.5 A of the exact radius is at
-// least kRadiusMargin times that of the node atoms', weighted by their energy:
-// the energy left out is then a fifth of the one removed, also for those points
-// of a box that have fewer near atoms than the box.  Past 36 A the steps are
-// below FP32 rounding.
+// least that of the node atoms', weighted by their energy.  Where the near weights
+// lie to one side of the box (their mean unit vector is longer than kRadiusLean;
+// half a shell has 0.5), some of its points have far fewer near atoms than the
+// box, and the density must be kRadiusMargin times as large: the energy left out is
+// then a fifth of the one removed.  Past 36 A the steps are below FP32 rounding.
 //
 // Errors against FP64 (relative 2-norm), 20,000 atoms (43 A) and 41^3 points 0,
 // 50, 55, 63 and 75 A from the middle, over those without node sums and with
-// exact bins to 11 A: 0.88, 0.95, 0.93, 0.96 and 0.82; with R = 24 A everywhere
-// 0.94, 1.10, 1.23, 2.2 and 0.92; with a margin of 1: 0.94, 1.05, 1.03, 1.00 and
-// 0.82.  Time for 20,000 atoms on 161^3 points 11.7 ms, with R = 24 A 11.2, margin 1
-// 11.2; 60,000 on 255^3 53.2, 50.5 and 50.7; 8,000 on 125 x 97 x 83 2.54, 2.48, 2.49.
+// exact bins to 11 A: 0.91, 0.90, 0.93, 0.95 and 0.82; with R = 24 A everywhere
+// 0.91, 1.04, 1.24, 2.19 and 0.92.  Time for 20,000 atoms on 161^3 points 10.9 ms,
+// with R = 24 A 10.7, with the margin everywhere 11.2; 60,000 on 255^3 51.6, 50.5
+// and 53.3; 8,000 on 125 x 97 x 83 2.53, 2.48 and 2.54.
 template <int NB>
 __device__ __forceinline__ void box_radii(const EmapParams& P, const int blk0) {
-  constexpr int kSums = kRadiusSteps + 1;  // energies from each radius on, then the near squared weights
+  // Energies from each radius on, the near squared weights, and those times
+  // their unit vectors from the box.
+  constexpr int kSums = kRadiusSteps + 4;
   __shared__ float part[kThreads / 32][NB][kSums];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float rn = sqrtf(P.rnear2), n0 = rn - 350.f, n1 = rn + 350.f;
@@ -1067,7 +1070,13 @@ __device__ __forceinline__ void box_radii(const EmapParams& P, const int blk0) {
       const float dx = fmaxf(fabsf(x - o[b].x) - h[b].x, 0.f), dy = fmaxf(fabsf(y - o[b].y) - h[b].y, 0.f),
                   dz = fmaxf(fabsf(z - o[b].z) - h[b].z, 0.f);
       const float d = sqrtf(dx * dx + dy * dy + dz * dz), u = d - inner[b], step = kRadiusStep * inner[b];
-      if (d >= n0 && d < n1) s[b][kRadiusSteps] = fmaf(w, w, s[b][kRadiusSteps]);
+      if (d >= n0 && d < n1) {
+        const float w2 = w * w, wd = __fdividef(w2, d);
+        s[b][kRadiusSteps] += w2;
+        s[b][kRadiusSteps + 1] += copysignf(dx, x - o[b].x) * wd;
+        s[b][kRadiusSteps + 2] += copysignf(dy, y - o[b].y) * wd;
+        s[b][kRadiusSteps + 3] += copysignf(dz, z - o[b].z) * wd;
+      }
       const float e = w * w * ex2_approx(nl2 * u);
 #pragma unroll
       for (int k = 0; k < kRadiusSteps; k++)
@@ -1092,7 +1101,9 @@ __device__ __forceinline__ void box_radii(const EmapParams& P, const int blk0) {
       for (int k = 0; k < kSums; k++) v[k] += part[w][tid][k];
     const float r0 = fmaxf(P.rnodeHalfWidths * B.rnode, P.rnodeMin);
     const float nearVol = volume_within(hb, n1) - volume_within(hb, n0), farVol = depth * area_at(hb, r0 + depth);
-    const float limit = v[kRadiusSteps] * farVol, scale = kRadiusMargin * nearVol;
+    const float vx = v[kRadiusSteps + 1], vy = v[kRadiusSteps + 2], vz = v[kRadiusSteps + 3], vn = v[kRadiusSteps];
+    const bool inside = vx * vx + vy * vy + vz * vz < kRadiusLean * kRadiusLean * vn * vn;
+    const float limit = vn * farVol, scale = (inside ? 1.f : kRadiusMargin) * nearVol;
     int k = 0;
     while (k < kRadiusSteps && limit < scale * v[k]) k++;
     float t = (float)k;
