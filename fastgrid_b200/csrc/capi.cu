@@ -1606,6 +1606,7 @@ struct ag_batch {
   DevBuf<double> checks;                 // per job: net-charge checksum of its e-map (FP64 weight sum)
   std::vector<double> hChecks;
   int ne = 0, na = 0, na2 = 0, nmPadMax = 4, nmapsMax = 0;  // na2: two-point jobs
+  int64_t launches = 0;                  // kernels in the graph
   bool anySlots = false;                 // some two-point pass has H-bond slots
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -1787,8 +1788,13 @@ extern "C" int ag_batch_compute(ag_batch* b) {
       err = fail(AG_E_CUDA, "batch e-map launch failed");
     if (!err && conc && cudaEventRecord(bc->evJoin, est) != cudaSuccess)
       err = fail(AG_E_CUDA, "batch graph join failed");
-    for (ag_ctx* c : b->sub)
+    b->launches = 2;  // the e-map's node radii and the e-map
+    for (ag_ctx* c : b->sub) {
+      const int64_t before = c->launches;
       if (!err) err = prepAffinity(c, st);
+      b->launches += c->launches - before;
+    }
+    b->launches += b->twoPoint && b->anySlots ? 2 : 1;
     if (!err) {
       const cudaError_t ae =
           b->twoPoint ? agk::aff2_batch_launch(b->a2jobs.p, b->na2, b->aunits.p, b->na, b->counters.p + 1,
@@ -1816,7 +1822,7 @@ extern "C" int ag_batch_compute(ag_batch* b) {
   CK(cudaEventRecord(b->ev[0], st));
   CK(cudaGraphLaunch(b->exec, st));
   CK(cudaEventRecord(b->ev[1], st));
-  b->ctx->launches += 2 + (int64_t)b->sub.size();
+  b->ctx->launches += b->launches;
   CK(cudaStreamSynchronize(st));
   {
     float ms = 0.f;

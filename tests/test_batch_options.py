@@ -88,3 +88,20 @@ def test_batch_keeps_no_staged_inputs(tmp_path):
         b.close()
         ctx.close()
     assert grown[1] < 48 * 200e3
+
+
+def test_batch_counts_its_kernels(tmp_path):
+    """Node radii, e-map, cell list, slot maps' zeroing and affinity pass; a receptor of more than 8,192
+    atoms takes four kernels for its cell list."""
+    probs = _problems(tmp_path, [(1000, 25, "C HD"), (9000, 25, "C HD"), (1000, 25, "C")])
+    ctx = fg.Context(0)
+    count = []
+    for p in probs:
+        b = fg.Batch(ctx, [p])
+        for _ in range(2):
+            before = ctx.launches
+            b.compute()
+            count.append(ctx.launches - before)
+        b.close()
+    ctx.close()
+    assert count == [5, 5, 8, 8, 4, 4]
