@@ -848,7 +848,7 @@ __device__ __forceinline__ bool aff2_unit(const Aff2Params& P, const int cta, un
 
 // CTAs per SM: three (80 registers, 76 KB of shared memory), so that the plain
 // parts' table reads, which fill the shared-memory pipe, overlap the slot
-// parts' arithmetic; rows of 16 columns (51 KB tables) leave room for two.
+// parts' arithmetic; rows of 16 columns (64 KB tables) leave room for two.
 template <int NMAX>
 constexpr int aff2_ctas_per_sm() {
   return NMAX <= 12 ? 3 : 2;

@@ -246,7 +246,7 @@ int checkGrid(const ag_grid* g);
 void makeItems(const ag_grid& g, const int tile[3], int warpCompact, bool dense, std::vector<int>& items,
                std::vector<agk::EmapBlock>& blocks);
 // Stage the e-map inputs of a job (atoms, dielectric table, CTA boxes).
-int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const double* inv_eps, bool deviceInputs);
+int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const double* inv_eps);
 // Launch parameters of the direct e-map of the staged job.
 int buildEmapParams(ag_ctx* c, float* dOut, bool allowSplit, agk::EmapParams& P);
 int runEmap(ag_ctx* c, float* dOut);

@@ -321,7 +321,8 @@ static std::pair<int, int> bestSplit(int ny, int nz, const int T[3], int w, int 
 // the last is full and a box may span two tiles (the surrogate's near field, whose cost is per CTA and whose
 // warps skip atoms: 4.49 ms per surrogate e-map on 161^3 against 4.60 ms with
 // a CTA per tile).  Otherwise a CTA is a tile and its box stays compact, which
-// the direct e-map's node sums need: they begin 9.5 half-widths from the box.
+// the direct e-map's node sums need: they begin 8.5 half-widths from the box (9.5
+// for the constant dielectric).
 // A CTA that is a tile forms its items itself (tile_item in emap.cu); dense ones
 // read them from the list.  Writes at most blockCap boxes and, for dense CTAs,
 // the items (one per 8 points of a row; *nitemsOut of them); returns the number
@@ -576,34 +577,32 @@ int stageItems(ag_ctx* c) {
   return AG_OK;
 }
 
-int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const double* inv_eps, bool deviceInputs) {
+int stageEmap(ag_ctx* c, const ag_grid* g, int n, const double* xyzw, const double* inv_eps) {
   if (int r = checkGrid(g)) return r;
   if (n < 0 || (n > 0 && !xyzw)) return fail(AG_E_INVALID, "bad atom array");
   c->grid = *g;
   c->nAtoms = n;
   c->ddd = inv_eps != nullptr;
   CK(cudaSetDevice(c->device));
-  if (!deviceInputs) {
-    for (int64_t i = 0; i < 4 * (int64_t)n; i++)
-      if (!std::isfinite(xyzw[i])) return fail(AG_E_INVALID, "non-finite atom coordinate or weight at atom %lld", (long long)(i / 4));
-    c->wSum = 0;
-    c->wAbsSum = 0;
-    for (int d = 0; d < 3; d++) {
-      c->atomLo[d] = DBL_MAX;
-      c->atomHi[d] = -DBL_MAX;
-    }
-    for (int i = 0; i < n; i++) {
-      c->wSum += xyzw[4 * (size_t)i + 3];
-      c->wAbsSum += std::fabs(xyzw[4 * (size_t)i + 3]);
-      for (int d = 0; d < 3; d++) {
-        c->atomLo[d] = std::min(c->atomLo[d], xyzw[4 * (size_t)i + d]);
-        c->atomHi[d] = std::max(c->atomHi[d], xyzw[4 * (size_t)i + d]);
-      }
-    }
-    CK(c->atoms.ensure(n));
-    if (n) CK(cudaMemcpyAsync(c->atoms.p, xyzw, sizeof(double) * 4 * n, cudaMemcpyHostToDevice, c->stream));
-    c->atomsVersion++;  // the surrogate reads the staged atoms back when it needs a host copy
+  for (int64_t i = 0; i < 4 * (int64_t)n; i++)
+    if (!std::isfinite(xyzw[i])) return fail(AG_E_INVALID, "non-finite atom coordinate or weight at atom %lld", (long long)(i / 4));
+  c->wSum = 0;
+  c->wAbsSum = 0;
+  for (int d = 0; d < 3; d++) {
+    c->atomLo[d] = DBL_MAX;
+    c->atomHi[d] = -DBL_MAX;
   }
+  for (int i = 0; i < n; i++) {
+    c->wSum += xyzw[4 * (size_t)i + 3];
+    c->wAbsSum += std::fabs(xyzw[4 * (size_t)i + 3]);
+    for (int d = 0; d < 3; d++) {
+      c->atomLo[d] = std::min(c->atomLo[d], xyzw[4 * (size_t)i + d]);
+      c->atomHi[d] = std::max(c->atomHi[d], xyzw[4 * (size_t)i + d]);
+    }
+  }
+  CK(c->atoms.ensure(n));
+  if (n) CK(cudaMemcpyAsync(c->atoms.p, xyzw, sizeof(double) * 4 * n, cudaMemcpyHostToDevice, c->stream));
+  c->atomsVersion++;  // the surrogate reads the staged atoms back when it needs a host copy
   c->epsHost.clear();
   if (c->ddd) {
     c->epsHost.assign(inv_eps, inv_eps + 8192);
@@ -1284,7 +1283,7 @@ extern "C" int ag_upload(ag_ctx* c, const ag_grid* g, const ag_receptor* r, cons
   if (!c || !r) return fail(AG_E_INVALID, "null argument");
   c->haveJob = false;
   c->haveAff = false;
-  if (int e = stageEmap(c, g, r->n_atoms, r->xyzw, inv_eps, false)) return e;
+  if (int e = stageEmap(c, g, r->n_atoms, r->xyzw, inv_eps)) return e;
   c->nMaps = 0;
   if (p)
     if (int e = stageAffinity(c, r, p)) return e;
@@ -1345,7 +1344,7 @@ extern "C" int ag_emap_mode(ag_ctx* c, const ag_grid* g, int n, const double* xy
   c->haveAff = false;
   c->nMaps = 0;
   c->emapMode = mode;
-  int e = stageEmap(c, g, n, xyzw, inv_eps, false);
+  int e = stageEmap(c, g, n, xyzw, inv_eps);
   if (!e && c->maps.ensure((size_t)2 * c->npoints()) != cudaSuccess) e = fail(AG_E_CUDA, "cannot allocate the map");
   if (!e) e = runEmap(c, c->maps.p);
   c->emapMode = agk::kEmapKahan;
@@ -1496,7 +1495,7 @@ extern "C" int ag_problem_compute(ag_ctx* c, ag_problem* P) {
   if (conc) {
     c->haveJob = false;
     c->haveAff = false;
-    if (int e = stageEmap(c, &g, r.n_atoms, r.xyzw, eps, false)) return e;
+    if (int e = stageEmap(c, &g, r.n_atoms, r.xyzw, eps)) return e;
   } else if (int e = ag_upload(c, &g, &r, &a, eps)) {
     return e;
   }

@@ -582,9 +582,9 @@ __device__ __forceinline__ void emap_unit(const EmapParams& P, const int blk, co
   const float2 radius = NODES && DDD && P.radius ? P.radius[blk] : make_float2(0.f, 0.f);
   const float rnode = !NODES ? __int_as_float(0x7F800000)
                       : DDD && P.radius ? radius.x : fmaxf(P.rnodeHalfWidths * B.rnode, P.rnodeMin);
-  // Mid-list bins may pass the table's end (not if the node atoms begin before).
+  const bool clampMid = B.clampMid;  // mid-list bins may pass the table's end
+  // No mid atom is this far from a point of the box.
   const float midEndR = rnode + 2.f * sqrtf(B.hx * B.hx + B.hy * B.hy + B.hz * B.hz);
-  const bool clampMid = B.clampMid && !(midEndR < 8100.f);
   int nodeSeen = 0;  // uniform; bit 0: node atoms, bit 1: far-node atoms
   // The part of the packed tail that this box's mid atoms read: 16-bit entries
   // up to the farthest bin only, if the node atoms begin before the 8-bit ones.

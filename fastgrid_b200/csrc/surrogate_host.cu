@@ -692,7 +692,7 @@ extern "C" int ag_emap_surrogate(ag_ctx* c, const ag_grid* g, int n, const doubl
   c->haveJob = false;
   c->haveAff = false;
   c->nMaps = 0;
-  if (int e = stageEmap(c, g, n, xyzw, inv_eps, false)) return e;
+  if (int e = stageEmap(c, g, n, xyzw, inv_eps)) return e;
   CK(c->maps.ensure((size_t)2 * c->npoints()));
   if (int e = runEmapSurrogate(c, c->maps.p)) return e;
   CK(cudaMemcpyAsync(out, c->maps.p, sizeof(float) * c->npoints(), cudaMemcpyDeviceToHost, c->stream));
@@ -727,7 +727,7 @@ extern "C" int ag_surrogate_features(ag_ctx* c, const ag_grid* g, int n, const d
   c->haveJob = false;
   c->haveAff = false;
   c->nMaps = 0;
-  if (int e = stageEmap(c, g, n, xyzw, inv_eps, false)) return e;
+  if (int e = stageEmap(c, g, n, xyzw, inv_eps)) return e;
   SurrState& S = surrOf(c);
   const int64_t np = c->npoints();
   CK(c->maps.ensure((size_t)2 * np));
@@ -845,7 +845,7 @@ extern "C" int ag_surrogate_train(ag_ctx* c, const ag_surrogate_train_params* tp
     c->haveJob = false;
     c->haveAff = false;
     c->nMaps = 0;
-    int e = stageEmap(c, &grid, natoms[i], recs[i].data(), eps.data(), false);
+    int e = stageEmap(c, &grid, natoms[i], recs[i].data(), eps.data());
     if (!e) e = runEmap(c, direct.p);
     if (!e) e = surrBase(c, S, c->maps.p, featAll.p + (size_t)i * np, 1.f);
     if (!e && agk::surr_residual_launch(direct.p, c->maps.p, yAll.p + (size_t)i * np, featAll.p + (size_t)i * np, np,

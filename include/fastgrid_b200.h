@@ -204,7 +204,10 @@ int ag_problem_write(ag_problem* p);
 /* replay it.  No counterpart in the reference (one job per process).       */
 /* Problems must outlive the batch; all use the distance-dependent          */
 /* dielectric.  A job takes the context's e-map radii, packed-table switch   */
-/* and affinity kernel as they are set when the batch is created.            */
+/* and affinity kernel as they are set when the batch is created.  Its e-map */
+/* may differ in the last bits from the same job's alone (both are within    */
+/* tolerance): fewer than 1e9 point-atom pairs are summed point by point     */
+/* alone, and with node sums in a batch, whose CTAs share the GPU.           */
 /* ------------------------------------------------------------------------ */
 typedef struct ag_batch ag_batch;
 int ag_batch_create(ag_ctx* ctx, ag_problem* const* problems, int n, ag_batch** out);
