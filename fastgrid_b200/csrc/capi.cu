@@ -1011,6 +1011,16 @@ double twoPointCells(const ag_ctx* c, double lo[3], int ncell[3]) {
   return 8.0;
 }
 
+// Cell keys are 32-bit: a grid of too wide a spacing has more of them.
+static int checkCells(const ag_grid& g, double edge, int types) {
+  const double h = g.spacing;
+  double keys = types;
+  for (int n : {g.nx, g.ny, g.nz}) keys *= std::max(1.0, std::ceil(((n - 1) * h + 16.0) / edge));
+  if (keys < 2147000000.0) return AG_OK;
+  return fail(AG_E_INVALID, "a grid of %d x %d x %d points at %g A has too many %g A cells for the affinity pass", g.nx,
+              g.ny, g.nz, h, edge);
+}
+
 // Whether every affinity pass of the staged job runs on the two-point kernel.
 bool useTwoPoint(const ag_ctx* c) {
   if (c->affKernel != 2) return false;
@@ -1034,6 +1044,7 @@ int prepAffinity(ag_ctx* c, cudaStream_t st) {
   int launched = 0;
   if (useTwoPoint(c)) {
     C.edge = twoPointCells(c, lo, ncell);
+    if (int e = checkCells(g, C.edge, c->nTypes)) return e;
     const size_t nkeys = (size_t)ncell[0] * ncell[1] * ncell[2] * c->nTypes;
     for (int d = 0; d < 3; d++) { C.lo[d] = lo[d]; C.ncell[d] = ncell[d]; }
     CK(c->ctStart.ensure(nkeys + 1)); CK(c->count.ensure(2 * (nkeys + 1)));
@@ -1047,6 +1058,7 @@ int prepAffinity(ag_ctx* c, cudaStream_t st) {
     return AG_OK;
   }
   C.edge = 8.0;
+  if (int e = checkCells(g, C.edge, 1)) return e;
   cellGrid(g, C.edge, lo, ncell);
   const int ncellT = ncell[0] * ncell[1] * ncell[2];
   for (int d = 0; d < 3; d++) { C.lo[d] = lo[d]; C.ncell[d] = ncell[d]; }
