@@ -461,8 +461,11 @@ bool denseItems(const ag_ctx* c) {
   // Few pairs: the tiles' own cost (tables, classes, half-empty CTAs) outweighs
   // what the nodes save.  1,227 atoms on 56 x 147 x 49 points (4.9e8): 0.329 ms
   // dense, 0.375 ms with tiles; 3,000 on 45 x 111 x 45 (6.7e8): 0.396 and 0.419;
-  // 5,000 on 45 x 111 x 45 (1.1e9): 0.541 and 0.515.  Not for a batch's jobs,
-  // which share the GPU, nor where the caller has set the node radius.
+  // 5,000 on 45 x 111 x 45 (1.1e9): 0.541 and 0.515; on cubes the two are close
+  // (whole ag_emap calls: 10,000 on 45^3, 9.1e8, 0.597 and 0.618 ms; 4,000 on 61^3,
+  // 9.1e8, 0.628 both; 950 on 101^3, 9.8e8, 0.902 and 0.886; 20,000 on 31^3, 6.0e8,
+  // 0.474 and 0.450).  Not for a batch's jobs, which share the GPU, nor where the
+  // caller has set the node radius.
   if (c->ddd && few && !c->rNodeSet && !c->batchJob) return true;
   for (int d = 0; d < 3; d++) {
     const double lo = -(n[d] / 2) * g.spacing, hi = (n[d] - 1 - n[d] / 2) * g.spacing;
