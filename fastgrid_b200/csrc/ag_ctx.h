@@ -173,6 +173,7 @@ struct ag_ctx {
   };
   std::vector<Pass> passes;
   int typeHbond[agk::kMaxTypes] = {0};
+  unsigned char typeOrder[agk::kMaxTypes] = {0};  // receptor types as the two-point kernel sums them
   // job
   bool haveJob = false, haveAff = false, ddd = true;
   ag_grid grid{};
